@@ -87,7 +87,7 @@ struct mdt_ctx {
     int *rptraj = nullptr;     // trajectories of the packs
     int rnpack = 0, rblock = 0;
     bool rfull = false;         // the plan packs every trajectory of the batch (not a re-pack)
-    double *lcoef = nullptr;    // constant-friction Langevin coefficients of the thread-per-atom kernel
+    double *lcoef = nullptr;    // constant-friction Langevin coefficients, 8 per atom
     RadialNN RG{};              // tensor-core network tables of a generic model (own descriptor order)
     double *tc_G = nullptr;     // its pass buffers: raw descriptors, atomic energies [ba][maxsf], [ba]
     double *tc_eat = nullptr;
@@ -230,7 +230,28 @@ PropParams to_dev(const mdt_ctx *c, const mdt_prop_params *p) {
     P.zeta = c->rnd[1];
     P.andersen_v = c->rnd[2];
     P.andersen_u = c->rnd[3];
+    P.lcoef = c->lcoef;
     return P;
+}
+
+// Constant-friction Langevin coefficients for the parameters of a propagation: they depend on
+// (gamma, dt, T) and the batch's masses, bead counts and propagators (fixed by mdt_batch_define),
+// so they are formed once per parameter set.
+int ensure_lcoef(mdt_ctx *c, const mdt_prop_params *p) {
+    bool need = false;
+    for (int t = 0; t < c->ntypes; ++t) need |= c->B.algo[t] == kPropLangevinConst;
+    const double key[4] = {p->gamma_const, p->step, p->Tsurf, p->Tproj};
+    if (!need || (c->lcoef && c->lc_valid && std::memcmp(key, c->lc_key, sizeof(key)) == 0)) return MDT_OK;
+    cudaError_t e = cudaSuccess;
+    if (!c->lcoef) c->lcoef = dalloc<double>(c, 8 * (size_t)c->total_atoms, e);
+    if (!c->lcoef) return fail(c, MDT_ERR_NOMEM, "Langevin coefficient buffer");
+    c->lc_valid = false;
+    e = launch_lcoef(c->stream, c->B, to_dev(c, p), c->ba_traj, c->total_ba, c->lcoef);
+    c->launches++;
+    if (e != cudaSuccess) return cuda_fail(c, e, "Langevin coefficients");
+    std::memcpy(c->lc_key, key, sizeof(key));
+    c->lc_valid = true;
+    return MDT_OK;
 }
 
 int check_ready(mdt_ctx *c, bool need_emt) {
@@ -804,22 +825,6 @@ int run_radial(mdt_ctx *c, const PropParams &P, int nsteps, int mode, bool surr,
     R.surrogate = surr ? 1 : 0;
     R.fscal = c->F.scal;
     R.fdscal = c->F.dscal;
-    if (mode == 2) {
-        // constant-friction coefficients depend on (gamma, dt, T) and the batch's masses and
-        // propagators (fixed by mdt_batch_define): formed once per parameter set
-        const double key[4] = {P.gamma_const, P.step, P.Tsurf, P.Tproj};
-        if (!c->lcoef || !c->lc_valid || std::memcmp(key, c->lc_key, sizeof(key)) != 0) {
-            cudaError_t e = cudaSuccess;
-            if (!c->lcoef) c->lcoef = dalloc<double>(c, 8 * (size_t)c->total_ba, e);
-            if (!c->lcoef) return fail(c, MDT_ERR_NOMEM, "Langevin coefficient buffer");
-            e = launch_nnr_lcoef(c->stream, c->B, P, c->ba_traj, c->total_ba, c->lcoef);
-            c->launches++;
-            if (e != cudaSuccess) return cuda_fail(c, e, "Langevin coefficients");
-            std::memcpy(c->lc_key, key, sizeof(key));
-            c->lc_valid = true;
-        }
-    }
-    c->X.lcoef = c->lcoef;
     const cudaError_t e = launch_nnr(LaunchCfg{c->stream, grid, c->order, c->counter}, c->B, R, c->E, c->X, P,
                                      c->rpacks, c->rptraj, c->rnpack, nsteps, mode);
     c->launches++;
@@ -1038,6 +1043,12 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
         if (idx[a] < 1 || idx[a] > ntypes) return fail(c, MDT_ERR_ARG, "atom type index out of range");
 
     // host-side derived arrays
+    std::vector<double> imass(at), comfac(ntraj);
+    for (int a = 0; a < at; ++a) imass[a] = 1.0 / mass[a];
+    for (int t = 0; t < ntraj; ++t) {
+        const double n = natoms[t];
+        comfac[t] = n * (1.0 - std::pow(1.0 - 1.0 / n, 1000.0));
+    }
     std::vector<int8_t> type(at);
     for (int a = 0; a < at; ++a) type[a] = (int8_t)(idx[a] - 1);
     c->h_type.assign(type.begin(), type.end());
@@ -1089,7 +1100,7 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
     } while (0)
     int *d_natoms, *d_nbeads, *d_atom_off, *d_bead_off, *d_cjk_off, *d_status, *d_steps;
     int64_t *d_ba_off, *d_pair_off;
-    double *d_mass, *d_box, *d_ibox, *d_cjk;
+    double *d_mass, *d_imass, *d_comfac, *d_box, *d_ibox, *d_cjk;
     int8_t *d_type;
     uint8_t *d_fixed;
     ALLOC(d_natoms, int, ntraj);
@@ -1106,6 +1117,8 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
     ALLOC(d_ba_off, int64_t, ntraj);
     ALLOC(d_pair_off, int64_t, ntraj);
     ALLOC(d_mass, double, at);
+    ALLOC(d_imass, double, at);
+    ALLOC(d_comfac, double, ntraj);
     ALLOC(d_box, double, 9 * (size_t)ntraj);
     ALLOC(d_ibox, double, 9 * (size_t)ntraj);
     ALLOC(d_cjk, double, cjk_host.size());
@@ -1132,6 +1145,8 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
     up(d_ba_off, c->ba_off.data(), sizeof(int64_t) * ntraj);
     up(d_pair_off, pair_off.data(), sizeof(int64_t) * ntraj);
     up(d_mass, mass, sizeof(double) * at);
+    up(d_imass, imass.data(), sizeof(double) * at);
+    up(d_comfac, comfac.data(), sizeof(double) * ntraj);
     up(d_box, simbox, sizeof(double) * 9 * ntraj);
     up(d_ibox, ibox.data(), sizeof(double) * 9 * ntraj);
     up(d_cjk, cjk_host.data(), sizeof(double) * cjk_host.size());
@@ -1160,6 +1175,8 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
     B.ax = arr[6]; B.ay = arr[7]; B.az = arr[8];
     B.fx = arr[9]; B.fy = arr[10]; B.fz = arr[11];
     B.mass = d_mass;
+    B.imass = d_imass;
+    B.comfac = d_comfac;
     B.type = d_type;
     B.fixed = d_fixed;
     B.box = d_box;
@@ -1366,7 +1383,7 @@ int32_t mdt_calc_force(mdt_ctx *c, int32_t flag, int32_t precision, const mdt_pr
 int32_t mdt_propagate_1(mdt_ctx *c, const mdt_prop_params *p) {
     int rc = check_ready(c, false);
     if (rc) return rc;
-    if ((rc = check_params(c, p))) return rc;
+    if ((rc = check_params(c, p)) || (rc = ensure_lcoef(c, p))) return rc;
     const PropParams P = to_dev(c, p);
     cudaError_t e = launch_phase(cfg(c, 0), c->B, c->E, P, kPhaseProp1, 0);
     c->launches++;
@@ -1376,7 +1393,7 @@ int32_t mdt_propagate_1(mdt_ctx *c, const mdt_prop_params *p) {
 int32_t mdt_propagate_2(mdt_ctx *c, const mdt_prop_params *p) {
     int rc = check_ready(c, false);
     if (rc) return rc;
-    if ((rc = check_params(c, p))) return rc;
+    if ((rc = check_params(c, p)) || (rc = ensure_lcoef(c, p))) return rc;
     const PropParams P = to_dev(c, p);
     cudaError_t e = launch_phase(cfg(c, 0), c->B, c->E, P, kPhaseProp2, 0);
     c->launches++;
@@ -1391,6 +1408,7 @@ int32_t mdt_md_steps(mdt_ctx *c, int32_t nsteps, int32_t precision, const mdt_pr
     if (tc_mode(precision) && c->pes_kind == MDT_PES_EMT) return fail(c, MDT_ERR_UNSUPPORTED, kBf16Scope);
     if ((rc = check_params(c, p))) return rc;
     if (p->rng_mode == 1 && nsteps > 1) return fail(c, MDT_ERR_ARG, "rng_mode 1 supports one step per call");
+    if (nsteps > 0 && (rc = ensure_lcoef(c, p))) return rc;
     if (c->pes_kind != MDT_PES_EMT) {
         if ((rc = check_nn_ready(c))) return rc;
         if (c->pes_kind == MDT_PES_SURROGATE && (rc = ensure_scratch(c, MDT_PREC_FP64))) return rc;
@@ -1832,6 +1850,10 @@ int32_t mdt_autotune(mdt_ctx *c, int32_t precision, int32_t nsteps, const mdt_pr
     e = copy_all(true);
     const int keep_block = c->rmaxblock;
     const double keep_skin = c->skin_ang;
+    if (e == cudaSuccess && (rc = ensure_lcoef(c, p))) {
+        cudaFree(snap);
+        return rc;
+    }
     const PropParams P = to_dev(c, p);
     const bool surr = c->pes_kind == MDT_PES_SURROGATE;
     const int tc = tc_mode(precision);

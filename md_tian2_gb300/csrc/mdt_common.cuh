@@ -49,6 +49,7 @@ constexpr int kStatusErrNonFinite = -11;
 struct EmtConst {
     int nspecies;                 // 1 or 2
     int slot_of_type[kMaxTypes];  // universe type (0-based) -> species slot, -1 = not EMT
+    int type_of_slot[2];
     uint32_t pair_mask;           // bit ti*kMaxTypes+tj set when pes(ti,tj) == emt
     int hh_quirk;                 // 2 species: slot-0/slot-0 derivative uses eta2 of slot 1
     double cut2;                  // (1.5*rcut)^2
@@ -58,6 +59,7 @@ struct EmtConst {
     double igamma1[2], g2v0[2];   // 1/gamma1, v0/gamma2
     double n0[2], e0[2], lambda[2], kappa[2], v0[2], dens_exp[2];
     double chi[2][2];             // density at a from neighbour b scaled by chi[a][b]
+    double ibe[2], e0l2[2], v6[2], v6k[2];  // 1/betaeta2, e0 lambda^2, 6 v0, 6 v0 kappa
 };
 
 // Everything a kernel needs to address the batch.  Passed by value.
@@ -73,6 +75,8 @@ struct Batch {
     double *dens;              // per bead-atom
     double *epot;              // per bead
     const double *mass;        // per atom
+    const double *imass;       // per atom, 1/mass
+    const double *comfac;      // per trajectory: N (1 - (1 - 1/N)^1000) (remove_com)
     const int8_t *type;        // per atom, 0-based universe type
     const uint8_t *fixed;      // per bead-atom, bit d set when dimension d is frozen
     const double *box, *ibox;  // per trajectory, 9 doubles column major
@@ -114,6 +118,7 @@ struct PropParams {
     const double *zeta;       // rng_mode 1: PILE deviates
     const double *andersen_v; // rng_mode 1: Andersen unit deviates
     const double *andersen_u; // rng_mode 1: Andersen uniforms (per ba)
+    const double *lcoef;      // constant-friction Langevin coefficients, kLcN per atom
 };
 
 // ---------------------------------------------------------------------------
@@ -145,12 +150,17 @@ __device__ __forceinline__ double u01_53(uint32_t a, uint32_t b) {
 // (useful_things.f90:121-173: sqrt(-2 ln u1) cos(2 pi u2)), evaluated in FP32: on this
 // GPU FP64 runs at 1/64 of FP32, and the thermostat noise needs no more than 24-bit
 // uniforms (u1 in (0, 1]: tails end at sqrt(2 ln 2^24) = 5.77 sigma).
-__device__ __forceinline__ double normal_deviate(uint64_t seed, uint32_t traj, uint32_t step,
-                                                 uint32_t slot, uint32_t stream) {
+__device__ __forceinline__ float normal_deviate_f(uint64_t seed, uint32_t traj, uint32_t step,
+                                                  uint32_t slot, uint32_t stream) {
     U4 r = philox4x32_10(U4{step, slot, stream, traj}, (uint32_t)seed, (uint32_t)(seed >> 32));
     const float u1 = (float)((r.x >> 8) + 1u) * (1.0f / 16777216.0f);
     const float u2 = (float)(r.z >> 8) * (1.0f / 16777216.0f);
-    return (double)(sqrtf(-2.0f * logf(u1)) * cospif(2.0f * u2));
+    return sqrtf(-2.0f * logf(u1)) * cospif(2.0f * u2);
+}
+
+__device__ __forceinline__ double normal_deviate(uint64_t seed, uint32_t traj, uint32_t step,
+                                                 uint32_t slot, uint32_t stream) {
+    return (double)normal_deviate_f(seed, traj, step, slot, stream);
 }
 
 __device__ __forceinline__ double uniform_deviate(uint64_t seed, uint32_t traj, uint32_t step,

@@ -28,6 +28,10 @@ cudaError_t launch_pack_state(cudaStream_t s, const Batch &B, double *dr, double
                               int64_t total_ba, const int *ba_traj);
 cudaError_t launch_pack_scalar(cudaStream_t s, const Batch &B, double *dst, const double *x, int64_t total_ba,
                                const int *ba_traj);
+// the constant-friction Langevin coefficients of every atom (kLcN each) for the parameters P: the
+// propagators read them instead of forming them (FP64 exp, sqrt and divisions) every half-step
+cudaError_t launch_lcoef(cudaStream_t s, const Batch &B, const PropParams &P, const int *ba_traj, int64_t total_ba,
+                         double *lcoef);
 cudaError_t launch_summary(cudaStream_t s, const Batch &B, const PropParams &P, double *out5);
 int max_resident_ctas(int max_atoms, int max_beads, int precision);
 
@@ -67,11 +71,6 @@ int nnr_resident_ctas(const RadialNN &R);
 cudaError_t launch_nn_tc(cudaStream_t s, int grid, const Batch &B, const RadialNN &R, const double *G,
                          const int *ba_traj, int64_t total_ba, float *dg, double *eat, int *err, int do_forces);
 size_t nn_tc_smem(int nin, int nh, int tc);
-// the constant-friction Langevin coefficients of every single-bead slot (8 per slot) for
-// the propagation parameters P: the thread-per-atom kernel reads them instead of forming
-// them (FP64 exp, sqrt and divisions) for every pack of every launch
-cudaError_t launch_nnr_lcoef(cudaStream_t s, const Batch &B, const PropParams &P, const int *ba_traj,
-                             int64_t total_ba, double *lcoef);
 cudaError_t launch_nnr(const LaunchCfg &c, const Batch &B, const RadialNN &R, const EmtConst &E, const NNScratch &X,
                        const PropParams &P, const int2 *packs, const int *ptraj, int npack, int nsteps, int mode);
 

@@ -30,27 +30,18 @@ template <typename R>
 __device__ void calc_force(const Batch &B, const EmtConst &E, const PropParams &P, const SmemEmt<R> &S,
                            const TrajView &T, bool do_forces) {
     const int tot = T.N * T.nb;
-    for (int s = threadIdx.x; s < tot; s += blockDim.x) {
-        const int64_t k = T.base + s;
-        B.fx[k] = 0.0; B.fy[k] = 0.0; B.fz[k] = 0.0;
-        B.ax[k] = 0.0; B.ay[k] = 0.0; B.az[k] = 0.0;
-    }
+    const bool single = T.nb == 1 && do_forces;  // no spring forces: the bead's forces are stored, not added
+    if (!single)
+        for (int s = threadIdx.x; s < tot; s += blockDim.x) {
+            const int64_t k = T.base + s;
+            B.fx[k] = 0.0; B.fy[k] = 0.0; B.fz[k] = 0.0;
+            B.ax[k] = 0.0; B.ay[k] = 0.0; B.az[k] = 0.0;
+        }
     for (int b = threadIdx.x; b < T.nb; b += blockDim.x) B.epot[B.bead_off[T.t] + b] = 0.0;
     __syncthreads();
     if (T.nb > 1) ring_polymer_step(B, P, T, S.cjk);
-    for (int b = 0; b < T.nb; ++b) emt_bead<R>(B, E, S, T.t, b, do_forces);
-    if (do_forces) {
-        // set_acceleration, force.f90:89-98
-        for (int s = threadIdx.x; s < tot; s += blockDim.x) {
-            const int64_t k = T.base + s;
-            const int i = s % T.N;
-            const double m = B.mass[T.aoff + i];
-            const uint8_t fx = B.fixed[k];
-            if (!(fx & 1)) B.ax[k] = B.fx[k] / m;
-            if (!(fx & 2)) B.ay[k] = B.fy[k] / m;
-            if (!(fx & 4)) B.az[k] = B.fz[k] / m;
-        }
-    }
+    for (int b = 0; b < T.nb; ++b) emt_bead<R>(B, E, S, T.t, b, do_forces, single);
+    if (do_forces) set_acceleration(B, T);
     __syncthreads();
 }
 
@@ -383,6 +374,22 @@ __global__ void summary_kernel(Batch B, PropParams P, double *out) {
         }
         __syncthreads();
     }
+}
+
+__global__ void lcoef_kernel(Batch B, PropParams P, const int *ba_traj, int64_t total_ba, double *lcoef) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total_ba; k += (int64_t)gridDim.x * blockDim.x) {
+        const TrajView T = traj_view(B, ba_traj[k]);
+        const int64_t i = k - T.base;
+        if (i < T.N && B.algo[B.type[T.aoff + i]] == kPropLangevinConst)
+            lc_setup(B, P, T, (int)i, lcoef + kLcN * (T.aoff + i));
+    }
+}
+
+cudaError_t launch_lcoef(cudaStream_t s, const Batch &B, const PropParams &P, const int *ba_traj, int64_t total_ba,
+                         double *lcoef) {
+    const int grid = (int)std::min<int64_t>((total_ba + 255) / 256, 4096);
+    lcoef_kernel<<<std::max(grid, 1), 256, 0, s>>>(B, P, ba_traj, total_ba, lcoef);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_summary(cudaStream_t s, const Batch &B, const PropParams &P, double *out5) {

@@ -52,7 +52,7 @@ struct SmemR {
     float4 *ph, *pl;                     // [slot] unwrapped positions (bohr), FP32 hi/lo split (x, y, z, 0)
     float *f3;                           // [3][bs] neighbour force accumulators (Ha/bohr)
     double *ea;                          // [slot] atomic energies (Ha)
-    double *lc;                          // [8][slot] Langevin coefficients of the atom (see LcR)
+    double *lc;                          // [8][slot] Langevin coefficients of the atom (mdt_prop.cuh)
     double *im;                          // [slot] 1 / mass
     int8_t *elem;                        // [slot]
     float *hb;                           // [hbw][bs] per-thread network buffer
@@ -988,33 +988,9 @@ __device__ __forceinline__ float nnr_network_tc(const RadialNN &R, const SmemR &
     return out;
 }
 
-// Propagators of the fused step for single-bead atoms.  The constant-friction Langevin
-// coefficients (langevin_coef of md_algo.f90:165-198 / 253-285: exp, sqrt and divisions in
-// FP64, the slowest pipe of the GPU) depend only on the atom, so they are formed once per
-// pack by the same FP64 expressions as langevin_1 / langevin_2 and the per-step updates
-// apply them exactly as those functions do.
-enum { kLcC0, kLcC1, kLcC2S, kLcC1mC2, kLcSr, kLcSvr, kLcC2, kLcSv2, kLcN };
-
-__device__ __forceinline__ void lc_setup(const Batch &B, const PropParams &P, const TrajView &T, int i, double *lc,
-                                         int stride) {
-    const int ty = B.type[T.aoff + i];
-    const double temp = kBoltz * T.nb * temp_of(B, P, ty) / B.mass[T.aoff + i];
-    const bool all_big = all_xidt_big(B, P, T, i, kPropLangevinConst);
-    LangCoef a, b;
-    langevin_coef(P.gamma_const, P.step, temp, all_big, false, a);
-    langevin_coef(P.gamma_const, P.step, temp, all_big, true, b);
-    lc[kLcC0 * stride] = a.c0;
-    lc[kLcC1 * stride] = a.c1;
-    lc[kLcC2S * stride] = a.c2 * P.step;
-    lc[kLcC1mC2 * stride] = a.c1 - a.c2;
-    lc[kLcSr * stride] = a.sigma_r;
-    lc[kLcSvr * stride] = a.sigma_v * a.c_rv;
-    lc[kLcC2 * stride] = b.c2;
-    lc[kLcSv2 * stride] = b.sigma_v * sqrt(1 - b.c_rv * b.c_rv);
-}
-
-// langevin_1 (md_algo.f90:146-232) for one single-bead atom with its coefficients
-__device__ __forceinline__ void lc_half1(const Batch &B, const PropParams &P, const TrajView &T, int i, int step,
+// langevin_1 (md_algo.f90:146-232) for one single-bead atom, its coefficients (mdt_prop.cuh) in
+// shared memory
+__device__ __forceinline__ void lc_half1_s(const Batch &B, const PropParams &P, const TrajView &T, int i, int step,
                                          const double *lc, int stride) {
     const int64_t k = T.base + i;
     const uint8_t fx = B.fixed[k];
@@ -1033,8 +1009,8 @@ __device__ __forceinline__ void lc_half1(const Batch &B, const PropParams &P, co
     }
 }
 
-// langevin_2 (md_algo.f90:236-300) for one single-bead atom with its coefficients
-__device__ __forceinline__ void lc_half2(const Batch &B, const PropParams &P, const TrajView &T, int i, int step,
+// langevin_2 (md_algo.f90:236-300) likewise
+__device__ __forceinline__ void lc_half2_s(const Batch &B, const PropParams &P, const TrajView &T, int i, int step,
                                          const double *lc, int stride) {
     const int64_t k = T.base + i;
     const uint8_t fx = B.fixed[k];
@@ -1145,7 +1121,7 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
             A.algo = B.algo[ty];
             S.im[tid] = 1.0 / B.mass[T.aoff + A.i];
             if (mode == 2 && A.algo == kPropLangevinConst) {
-                const double *src = X.lcoef + kLcN * (A.base + A.i);
+                const double *src = P.lcoef + kLcN * (T.aoff + A.i);
 #pragma unroll
                 for (int q = 0; q < kLcN; ++q) S.lc[q * bs + tid] = src[q];
             }
@@ -1173,8 +1149,8 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
             // ---- first half-step, positions, exit decision ------------------------------
             if (active) {
                 if (mode == 2) {
-                    if (A.algo == kPropVerlet) verlet_half(B, P, T, A.i, true);
-                    else lc_half1(B, P, T, A.i, step, S.lc + tid, bs);
+                    if (A.algo == kPropVerlet) verlet_half3(B, P, T, A.i, true);
+                    else lc_half1_s(B, P, T, A.i, step, S.lc + tid, bs);
                 }
                 const int64_t k = A.base + A.i;
                 const double rx = B.rx[k], ry = B.ry[k], rz = B.rz[k];
@@ -1339,8 +1315,8 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
             }
             // ---- second half-step ------------------------------------------------------------
             if (active && mode == 2) {
-                if (A.algo == kPropVerlet) verlet_half(B, P, T, A.i, false);
-                else lc_half2(B, P, T, A.i, step, S.lc + tid, bs);
+                if (A.algo == kPropVerlet) verlet_half3(B, P, T, A.i, false);
+                else lc_half2_s(B, P, T, A.i, step, S.lc + tid, bs);
                 // trajectory observables by the projectile's thread; the closest approach is
                 // the nearest entry of its skin list (every image within the cutoff + skin)
                 if (A.i == 0) {
@@ -1558,22 +1534,6 @@ cudaError_t launch_nn_tc(cudaStream_t s, int grid, const Batch &B, const RadialN
     MDT_NNTC(24, 2) MDT_NNTC(24, 1) MDT_NNTC(48, 2) MDT_NNTC(48, 1)
 #undef MDT_NNTC
     return cudaErrorInvalidValue;
-}
-
-__global__ void lcoef_kernel(Batch B, PropParams P, const int *ba_traj, int64_t total_ba, double *lcoef) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total_ba; k += (int64_t)gridDim.x * blockDim.x) {
-        const int t = ba_traj[k];
-        const TrajView T = traj_view(B, t);
-        const int i = (int)(k - T.base);
-        if (T.nb == 1 && B.algo[B.type[T.aoff + i]] == kPropLangevinConst) lc_setup(B, P, T, i, lcoef + kLcN * k, 1);
-    }
-}
-
-cudaError_t launch_nnr_lcoef(cudaStream_t s, const Batch &B, const PropParams &P, const int *ba_traj,
-                             int64_t total_ba, double *lcoef) {
-    const int grid = (int)std::min<int64_t>((total_ba + 255) / 256, 4096);
-    lcoef_kernel<<<std::max(grid, 1), 256, 0, s>>>(B, P, ba_traj, total_ba, lcoef);
-    return cudaGetLastError();
 }
 
 // The tensor-core network's wait, exercised alone: every thread waits (max_polls tries, as a

@@ -86,6 +86,11 @@ int emt_derive_constants(int32_t ntypes, const double *eta2, const double *n0, c
         E.igamma1[s] = 1.0 / g1;
         E.g2v0[s] = (1.0 / g2) * E.v0[s];
         E.dens_exp[s] = 0.5 / kBohr2Ang - E.betaeta2[s];
+        E.type_of_slot[s] = slots[s];
+        E.ibe[s] = 1.0 / E.betaeta2[s];
+        E.e0l2[s] = E.e0[s] * E.lambda[s] * E.lambda[s];
+        E.v6[s] = 6.0 * E.v0[s];
+        E.v6k[s] = E.v6[s] * E.kappa[s];
     }
     E.chi[0][0] = E.chi[1][1] = 1.0;
     E.chi[0][1] = E.chi[1][0] = 1.0;

@@ -28,7 +28,11 @@ static __device__ __forceinline__ double temp_of(const Batch &B, const PropParam
 static __device__ __forceinline__ double rand_normal(const PropParams &P, const TrajView &T, int step, int b, int i,
                                               int d, uint32_t stream, const double *injected) {
     if (P.rng_mode == 1) return injected[(T.base + (int64_t)i * T.nb + b) * 3 + d];
-    return normal_deviate(P.seed, (uint32_t)T.t, (uint32_t)step, (uint32_t)((b * T.N + i) * 3 + d), stream);
+    return f64_of(normal_deviate_f(P.seed, (uint32_t)T.t, (uint32_t)step, (uint32_t)((b * T.N + i) * 3 + d), stream));
+}
+
+static __device__ __forceinline__ double *comp_ptr(double *x, double *y, double *z, int d) {
+    return d == 0 ? x : (d == 1 ? y : z);
 }
 
 static __device__ __forceinline__ double &comp(double *x, double *y, double *z, int d, int64_t k) {
@@ -72,8 +76,8 @@ static __device__ void observe_core(const Batch &B, const PropParams &P, int t, 
     if (force) s[kObsInter] += 1;  // check_for_proj_surf_interaction (:140-148)
     // check_for_bounce (:152-241): unit vectors, dot products in the slot of this step
     if (near >= 0) {
-        const double ir = 1.0 / sqrt(rx * rx + ry * ry + rz * rz), iv = 1.0 / sqrt(vx * vx + vy * vy + vz * vz),
-                     iff = 1.0 / sqrt(fx * fx + fy * fy + fz * fz);
+        const double ir = rsqrt_nr(rx * rx + ry * ry + rz * rz), iv = rsqrt_nr(vx * vx + vy * vy + vz * vz),
+                     iff = rsqrt_nr(fx * fx + fy * fy + fz * fz);
         const double rv1 = (rx * vx + ry * vy + rz * vz) * (ir * iv);
         const double rf1 = (rx * fx + ry * fy + rz * fz) * (ir * iff);
         const double vf1 = (vx * fx + vy * fy + vz * fz) * (iv * iff);
@@ -125,74 +129,144 @@ static __device__ void observe_step(const Batch &B, const PropParams &P, const T
 // Closest approach of the projectile (atom 0) after a step: the minimum image of the
 // centroids of atom 0 and atom i over i >= 1 (trajectory_info.f90:92-105), CTA-wide; every
 // thread gets the distance, *near the nearest atom (first index on ties) and r the vector
-// from the projectile to it (`cell` and `red` are shared-memory scratch).
+// from the projectile to it (`cell` and `red` are shared-memory scratch).  FP32 distances with
+// a bound on their error pick the candidates; only those (one atom, as a rule) are evaluated in
+// FP64, where each atom cost about 30 instructions of the slowest pipe.
 static __device__ double closest_approach_step(const Batch &B, const TrajView &T, Cell *cell, double *red, int *near,
                                                double *r) {
-    __syncthreads();
-    if (threadIdx.x == 0) load_cell(B, T.t, *cell);
-    __syncthreads();
-    double c0x = 0.0, c0y = 0.0, c0z = 0.0;
-    for (int b = 0; b < T.nb; ++b) {
-        const int64_t k = T.base + (int64_t)b * T.N;
-        c0x += B.rx[k];
-        c0y += B.ry[k];
-        c0z += B.rz[k];
-    }
-    c0x /= T.nb;
-    c0y /= T.nb;
-    c0z /= T.nb;
-    double dmin = kDefaultReal;
-    int imin = T.N;
-    for (int i = 1 + threadIdx.x; i < T.N; i += blockDim.x) {
-        double cx = 0.0, cy = 0.0, cz = 0.0;
+    auto centroid = [&](int i, double &x, double &y, double &z) {
+        x = y = z = 0.0;
         for (int b = 0; b < T.nb; ++b) {
             const int64_t k = T.base + (int64_t)b * T.N + i;
-            cx += B.rx[k];
-            cy += B.ry[k];
-            cz += B.rz[k];
+            x += B.rx[k];
+            y += B.ry[k];
+            z += B.rz[k];
         }
-        double dx, dy, dz;
-        min_image(*cell, c0x - cx / T.nb, c0y - cy / T.nb, c0z - cz / T.nb, dx, dy, dz);
+        if (T.nb > 1) {
+            x /= T.nb;
+            y /= T.nb;
+            z /= T.nb;
+        }
+    };
+    auto centroid_f = [&](int i, float &x, float &y, float &z, float &m) {
+        x = y = z = m = 0.f;
+        for (int b = 0; b < T.nb; ++b) {
+            const int64_t k = T.base + (int64_t)b * T.N + i;
+            const float a = f32_of(B.rx[k]), c = f32_of(B.ry[k]), d = f32_of(B.rz[k]);
+            x += a;
+            y += c;
+            z += d;
+            m += fabsf(a) + fabsf(c) + fabsf(d);
+        }
+        const float s = 1.f / T.nb;
+        x *= s;
+        y *= s;
+        z *= s;
+        m *= s;
+    };
+    __syncthreads();
+    load_cell(B, T.t, *cell);
+    unsigned *best_up = (unsigned *)red;                          // smallest upper bound (FP32 bits)
+    unsigned long long *best_d = (unsigned long long *)(red + 1);  // smallest distance (FP64 bits)
+    int *best_i = (int *)(red + 2);
+    if (threadIdx.x == 0) {
+        *best_up = 0x7f800000u;
+        *best_d = 0x7fefffffffffffffull;  // kDefaultReal
+        *best_i = T.N;
+    }
+    __syncthreads();
+    float x0, y0, z0, m0;
+    centroid_f(0, x0, y0, z0, m0);
+    // lower and upper bound of atom i's distance; a fractional coordinate near a tie of the
+    // image choice gives (0, infinity)
+    auto bounds = [&](int i, float &lo, float &up) {
+        float x, y, z, m;
+        centroid_f(i, x, y, z, m);
+        const float ex = x0 - x, ey = y0 - y, ez = z0 - z;
+        float n[3];
+        bool tie = false;
+        // relative rounding 2^-24 of each bead position, of its sum over up to 32 beads and of
+        // the differences: 64 ulps cover them
+        const float err = 4e-6f * (m + m0) + 1e-6f;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const float w = cell->hif[q] * ex + cell->hif[q + 3] * ey + cell->hif[q + 6] * ez;
+            n[q] = rintf(w);
+            const float dw = 1e-4f + err * (fabsf(cell->hif[q]) + fabsf(cell->hif[q + 3]) + fabsf(cell->hif[q + 6]));
+            tie = tie || !(fabsf(fabsf(w - n[q]) - 0.5f) > dw);
+        }
+        const float dx = ex - (cell->hf[0] * n[0] + cell->hf[3] * n[1] + cell->hf[6] * n[2]);
+        const float dy = ey - (cell->hf[1] * n[0] + cell->hf[4] * n[1] + cell->hf[7] * n[2]);
+        const float dz = ez - (cell->hf[2] * n[0] + cell->hf[5] * n[1] + cell->hf[8] * n[2]);
+        const float d = sqrtf(dx * dx + dy * dy + dz * dz), e = err + 1e-6f * (d + fabsf(ex) + fabsf(ey) + fabsf(ez));
+        lo = tie ? 0.f : d - e;
+        up = tie ? INFINITY : d + e;
+        if (!(up >= 0.f)) {  // not a number: left to the FP64 evaluation
+            lo = 0.f;
+            up = INFINITY;
+        }
+    };
+    float up_min = INFINITY, lo, up;
+    for (int i = 1 + threadIdx.x; i < T.N; i += blockDim.x) {
+        bounds(i, lo, up);
+        up_min = fminf(up_min, up);
+    }
+    const unsigned wmin = __reduce_min_sync(0xffffffffu, __float_as_uint(up_min));
+    if ((threadIdx.x & 31) == 0) atomicMin(best_up, wmin);
+    __syncthreads();
+    up_min = __uint_as_float(*best_up);
+    double c0x, c0y, c0z, d_own = kDefaultReal;
+    int i_own = T.N;
+    bool have0 = false;
+    for (int i = 1 + threadIdx.x; i < T.N; i += blockDim.x) {
+        bounds(i, lo, up);
+        if (!(lo <= up_min)) continue;
+        double cx, cy, cz, dx, dy, dz;
+        if (!have0) centroid(0, c0x, c0y, c0z);
+        have0 = true;
+        centroid(i, cx, cy, cz);
+        min_image(*cell, c0x - cx, c0y - cy, c0z - cz, dx, dy, dz);
         const double d = sqrt(dx * dx + dy * dy + dz * dz);
-        if (d < dmin) {
-            dmin = d;
-            imin = i;
+        if (d < d_own) {
+            d_own = d;
+            i_own = i;
         }
     }
-    const double best = block_min(dmin, red);
-    const int ib = (int)block_min(dmin == best ? (double)imin : (double)T.N, red);
+    if (i_own < T.N) atomicMin(best_d, (unsigned long long)__double_as_longlong(d_own));
+    __syncthreads();
+    const double best = __longlong_as_double((long long)*best_d);
+    if (i_own < T.N && d_own == best) atomicMin(best_i, i_own);
+    __syncthreads();
+    const int ib = *best_i;
     *near = ib < T.N ? ib : -1;
     r[0] = r[1] = r[2] = 0.0;
-    if (ib < T.N) {
-        double cx = 0.0, cy = 0.0, cz = 0.0;
-        for (int b = 0; b < T.nb; ++b) {
-            const int64_t k = T.base + (int64_t)b * T.N + ib;
-            cx += B.rx[k];
-            cy += B.ry[k];
-            cz += B.rz[k];
-        }
-        min_image(*cell, cx / T.nb - c0x, cy / T.nb - c0y, cz / T.nb - c0z, r[0], r[1], r[2]);
+    if (ib < T.N && threadIdx.x == 0) {
+        double cx, cy, cz;
+        if (!have0) centroid(0, c0x, c0y, c0z);
+        centroid(ib, cx, cy, cz);
+        min_image(*cell, cx - c0x, cy - c0y, cz - c0z, r[0], r[1], r[2]);
     }
     return best;
 }
 
-// verlet_1 / verlet_2, md_algo.f90:110-142
-static __device__ void verlet_half(const Batch &B, const PropParams &P, const TrajView &T, int i, bool move_r) {
+// verlet_1 / verlet_2, md_algo.f90:110-142, for one dimension of an atom
+static __device__ __forceinline__ void verlet_half(const Batch &B, const PropParams &P, const TrajView &T, int i, int d,
+                                                   bool move_r) {
+    double *v = comp_ptr(B.vx, B.vy, B.vz, d) + T.base + i;
+    const double *a = comp_ptr(B.ax, B.ay, B.az, d) + T.base + i;
+    const uint8_t *fx = B.fixed + T.base + i;
     for (int b = 0; b < T.nb; ++b) {
-        const int64_t k = T.base + (int64_t)b * T.N + i;
-        const uint8_t fx = B.fixed[k];
-        for (int d = 0; d < 3; ++d) {
-            double &v = comp(B.vx, B.vy, B.vz, d, k);
-            if (!(fx >> d & 1)) v = v + 0.5 * P.step * comp(B.ax, B.ay, B.az, d, k);
-            else v = 0.0;
-        }
+        const int64_t k = (int64_t)b * T.N;
+        if (!(fx[k] >> d & 1)) v[k] = v[k] + 0.5 * P.step * a[k];
+        else v[k] = 0.0;
     }
-    if (move_r && T.nb == 1) {
-        const int64_t k = T.base + i;
-        const uint8_t fx = B.fixed[k];
-        for (int d = 0; d < 3; ++d)
-            if (!(fx >> d & 1)) comp(B.rx, B.ry, B.rz, d, k) += P.step * comp(B.vx, B.vy, B.vz, d, k);
-    }
+    if (move_r && T.nb == 1 && !(*fx >> d & 1)) comp_ptr(B.rx, B.ry, B.rz, d)[T.base + i] += P.step * *v;
+}
+
+// all three dimensions of an atom
+static __device__ __forceinline__ void verlet_half3(const Batch &B, const PropParams &P, const TrajView &T, int i,
+                                                    bool move_r) {
+    for (int d = 0; d < 3; ++d) verlet_half(B, P, T, i, d, move_r);
 }
 
 struct LangCoef { double c0, c1, c2, sigma_r, sigma_v, c_rv; };
@@ -226,6 +300,67 @@ static __device__ bool all_xidt_big(const Batch &B, const PropParams &P, const T
     for (int b = 0; b < T.nb; ++b)
         if (!(friction(B, P, algo, T.base + (int64_t)b * T.N + i) * P.step > (double)1e-2f)) all_big = false;
     return all_big;
+}
+
+// Constant-friction Langevin coefficients of an atom (langevin_coef of md_algo.f90:165-198 /
+// 253-285: exp, sqrt and divisions in FP64, the slowest pipe of the GPU).  They depend on the
+// atom's mass and type, the bead count and the run's parameters only, so they are formed once per
+// parameter set (lcoef_kernel) by the same FP64 expressions as langevin_1 / langevin_2, and the
+// per-step updates apply them exactly as those functions do.
+enum { kLcC0, kLcC1, kLcC2S, kLcC1mC2, kLcSr, kLcSvr, kLcC2, kLcSv2, kLcN };
+
+static __device__ __forceinline__ void lc_setup(const Batch &B, const PropParams &P, const TrajView &T, int i,
+                                                double *lc) {
+    const int ty = B.type[T.aoff + i];
+    const double temp = kBoltz * T.nb * temp_of(B, P, ty) / B.mass[T.aoff + i];
+    const bool all_big = all_xidt_big(B, P, T, i, kPropLangevinConst);
+    LangCoef a, b;
+    langevin_coef(P.gamma_const, P.step, temp, all_big, false, a);
+    langevin_coef(P.gamma_const, P.step, temp, all_big, true, b);
+    lc[kLcC0] = a.c0;
+    lc[kLcC1] = a.c1;
+    lc[kLcC2S] = a.c2 * P.step;
+    lc[kLcC1mC2] = a.c1 - a.c2;
+    lc[kLcSr] = a.sigma_r;
+    lc[kLcSvr] = a.sigma_v * a.c_rv;
+    lc[kLcC2] = b.c2;
+    lc[kLcSv2] = b.sigma_v * sqrt(1 - b.c_rv * b.c_rv);
+}
+
+// langevin_1 / langevin_2 with constant friction for one dimension of an atom
+static __device__ __forceinline__ void lc_half1(const Batch &B, const PropParams &P, const TrajView &T, int i, int d,
+                                                int step) {
+    const double *lc = P.lcoef + kLcN * (int64_t)(T.aoff + i);
+    const double c0 = lc[kLcC0], c1 = lc[kLcC1], c2s = lc[kLcC2S], c1mc2 = lc[kLcC1mC2], sr = lc[kLcSr],
+                 svr = lc[kLcSvr];
+    for (int b = 0; b < T.nb; ++b) {
+        const int64_t k = T.base + (int64_t)b * T.N + i;
+        double &v = comp(B.vx, B.vy, B.vz, d, k);
+        if (!(B.fixed[k] >> d & 1)) {
+            const double rnd = rand_normal(P, T, step, b, i, d, kStreamLangevin, P.randy);
+            const double a = comp(B.ax, B.ay, B.az, d, k);
+            comp(B.rx, B.ry, B.rz, d, k) += c1 * v + c2s * a + sr * rnd;
+            v = c0 * v + c1mc2 * a + svr * rnd;
+        } else {
+            v = 0.0;
+        }
+    }
+}
+
+static __device__ __forceinline__ void lc_half2(const Batch &B, const PropParams &P, const TrajView &T, int i, int d,
+                                                int step) {
+    const double *lc = P.lcoef + kLcN * (int64_t)(T.aoff + i);
+    const double c2 = lc[kLcC2], sv = lc[kLcSv2];
+    for (int b = 0; b < T.nb; ++b) {
+        const int64_t k = T.base + (int64_t)b * T.N + i;
+        double &v = comp(B.vx, B.vy, B.vz, d, k);
+        if (!(B.fixed[k] >> d & 1)) {
+            const double rnd = rand_normal(P, T, step, b, i, d, kStreamLangevin, P.randy);
+            v = v + c2 * comp(B.ax, B.ay, B.az, d, k) + sv * rnd;
+        } else {
+            v = 0.0;
+        }
+    }
 }
 
 // langevin_1, md_algo.f90:146-232
@@ -307,7 +442,7 @@ static __device__ void langevin_2(const Batch &B, const PropParams &P, const Tra
 }
 
 // andersen, md_algo.f90:402-432
-static __device__ void andersen(const Batch &B, const PropParams &P, const TrajView &T, int i, int step) {
+static __device__ void andersen(const Batch &B, const PropParams &P, const TrajView &T, int i, int d, int step) {
     const int ty = B.type[T.aoff + i];
     const double ibetaN = T.nb * kBoltz * temp_of(B, P, ty);
     const double sd = sqrt(ibetaN / B.mass[T.aoff + i]);
@@ -318,13 +453,8 @@ static __device__ void andersen(const Batch &B, const PropParams &P, const TrajV
         const double u = P.rng_mode == 1 ? P.andersen_u[T.base + (int64_t)i * T.nb + b]
                                          : uniform_deviate(P.seed, (uint32_t)T.t, (uint32_t)step, (uint32_t)slot,
                                                            kStreamAndersenU);
-        if (u < thr) {
-            const uint8_t fx = B.fixed[k];
-            for (int d = 0; d < 3; ++d)
-                if (!(fx >> d & 1))
-                    comp(B.vx, B.vy, B.vz, d, k) =
-                        rand_normal(P, T, step, b, i, d, kStreamAndersenV, P.andersen_v) * sd;
-        }
+        if (u < thr && !(B.fixed[k] >> d & 1))
+            comp(B.vx, B.vy, B.vz, d, k) = rand_normal(P, T, step, b, i, d, kStreamAndersenV, P.andersen_v) * sd;
     }
 }
 
@@ -420,35 +550,49 @@ static __device__ __forceinline__ void nm_back(const double *cjk, int nb, const 
     x[nb - 1] = c;
 }
 
-// pile_thermostat, md_algo.f90:440-502 (one thread per atom, all three dimensions; the
-// per-type, per-mode damping from pile_tables)
-static __device__ void pile(const Batch &B, const PropParams &P, const TrajView &T, double *cjk, int i, int step) {
+// pile_thermostat, md_algo.f90:440-502, for one dimension of an atom (the per-type, per-mode
+// damping from pile_tables)
+static __device__ void pile(const Batch &B, const PropParams &P, const TrajView &T, double *cjk, int i, int d,
+                            int step) {
     const int nb = T.nb;
     const int ty = B.type[T.aoff + i];
     const double m = B.mass[T.aoff + i];
     const double betaN = 1.0 / (kBoltz * temp_of(B, P, ty) * nb);
     const double sq = sqrt(m / betaN);
     const double *c1t = rp_table(cjk, nb, kRpC1) + ty * nb, *c2t = rp_table(cjk, nb, kRpC2) + ty * nb;
-    for (int d = 0; d < 3; ++d) {
-        double newP[32], atomP[32];
-        for (int b = 0; b < nb; ++b) atomP[b] = m * comp(B.vx, B.vy, B.vz, d, T.base + (int64_t)b * T.N + i);
-        nm_forward(cjk, nb, atomP, newP);
-        for (int kk = 0; kk < nb; ++kk) {
-            const double z = rand_normal(P, T, step, kk, i, d, kStreamPile, P.zeta);
-            newP[kk] = c1t[kk] * newP[kk] + sq * c2t[kk] * z;
-        }
-        nm_back(cjk, nb, newP, atomP);
-        for (int b = 0; b < nb; ++b) {
-            const int64_t k = T.base + (int64_t)b * T.N + i;
-            comp(B.vx, B.vy, B.vz, d, k) = (B.fixed[k] >> d & 1) ? 0.0 : atomP[b] / m;
-        }
+    const double im = B.imass[T.aoff + i];
+    double newP[32], atomP[32];
+    for (int b = 0; b < nb; ++b) atomP[b] = m * comp(B.vx, B.vy, B.vz, d, T.base + (int64_t)b * T.N + i);
+    nm_forward(cjk, nb, atomP, newP);
+    for (int kk = 0; kk < nb; ++kk) {
+        const double z = rand_normal(P, T, step, kk, i, d, kStreamPile, P.zeta);
+        newP[kk] = c1t[kk] * newP[kk] + sq * c2t[kk] * z;
+    }
+    nm_back(cjk, nb, newP, atomP);
+    for (int b = 0; b < nb; ++b) {
+        const int64_t k = T.base + (int64_t)b * T.N + i;
+        comp(B.vx, B.vy, B.vz, d, k) = (B.fixed[k] >> d & 1) ? 0.0 : div_by(atomP[b], m, im);
+    }
+}
+
+// set_acceleration, force.f90:89-98
+static __device__ __forceinline__ void set_acceleration(const Batch &B, const TrajView &T) {
+    const int tot = T.N * T.nb;
+    for (int s = threadIdx.x; s < tot; s += blockDim.x) {
+        const int64_t k = T.base + s;
+        const int i = s % T.N;
+        const double m = B.mass[T.aoff + i], im = B.imass[T.aoff + i];
+        const uint8_t fx = B.fixed[k];
+        B.ax[k] = fx & 1 ? 0.0 : div_by(B.fx[k], m, im);
+        B.ay[k] = fx & 2 ? 0.0 : div_by(B.fy[k], m, im);
+        B.az[k] = fx & 4 ? 0.0 : div_by(B.fz[k], m, im);
     }
 }
 
 // remove_com_velocity, universe_mod.f90:222-241.  Its 1000 subtraction sweeps have the
 // closed form v -= v_cm0 * N * (1 - (1 - 1/N)^1000), applied to every bead-atom.
 static __device__ void remove_com(const Batch &B, const TrajView &T, double *red) {
-    double sx = 0, sy = 0, sz = 0, ms = 0;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
     for (int i = threadIdx.x; i < T.N; i += blockDim.x) {
         const double m = B.mass[T.aoff + i];
         double ax = 0, ay = 0, az = 0;
@@ -458,18 +602,14 @@ static __device__ void remove_com(const Batch &B, const TrajView &T, double *red
             ay += B.vy[k];
             az += B.vz[k];
         }
-        sx += ax * m;
-        sy += ay * m;
-        sz += az * m;
-        ms += m;
+        v[0] += ax * m;
+        v[1] += ay * m;
+        v[2] += az * m;
+        v[3] += m;
     }
-    sx = block_sum(sx, red);
-    sy = block_sum(sy, red);
-    sz = block_sum(sz, red);
-    ms = block_sum(ms, red);
-    const double n = (double)T.N;
-    const double fac = n * (1.0 - pow(1.0 - 1.0 / n, 1000.0));
-    const double cx = sx / ms / T.nb / n * fac, cy = sy / ms / T.nb / n * fac, cz = sz / ms / T.nb / n * fac;
+    block_sum4(v, red);
+    const double n = (double)T.N, ms = v[3], fac = B.comfac[T.t];
+    const double cx = v[0] / ms / T.nb / n * fac, cy = v[1] / ms / T.nb / n * fac, cz = v[2] / ms / T.nb / n * fac;
     const int tot = T.N * T.nb;
     for (int s = threadIdx.x; s < tot; s += blockDim.x) {
         const int64_t k = T.base + s;
@@ -490,23 +630,28 @@ static __device__ bool traj_has_algo(const Batch &B, int id) {
 static __device__ void propagate_1(const Batch &B, const PropParams &P, const TrajView &T, double *cjk, int step,
                             double *red) {
     if (traj_has_algo(B, kPropPile)) pile_tables(B, P, T, cjk);
-    for (int i = threadIdx.x; i < T.N; i += blockDim.x) {
+    // work items (dimension, atom): three times the threads of a loop over atoms, so that a small
+    // trajectory's FP64 work spreads over the CTA's warps
+    for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
+        const int d = w / T.N, i = w - d * T.N;
         const int algo = B.algo[B.type[T.aoff + i]];
         switch (algo) {
-            case kPropVerlet: verlet_half(B, P, T, i, true); break;
+            case kPropVerlet: verlet_half(B, P, T, i, d, true); break;
             case kPropAndersen:
-                verlet_half(B, P, T, i, true);
-                andersen(B, P, T, i, step);
+                verlet_half(B, P, T, i, d, true);
+                andersen(B, P, T, i, d, step);
                 break;
             case kPropPile:
-                pile(B, P, T, cjk, i, step);
-                verlet_half(B, P, T, i, true);
+                pile(B, P, T, cjk, i, d, step);
+                verlet_half(B, P, T, i, d, true);
                 break;
-            case kPropLangevin:
-            case kPropLangevinConst: langevin_1(B, P, T, i, step, algo); break;
+            case kPropLangevinConst: lc_half1(B, P, T, i, d, step); break;
             default: break;
         }
     }
+    if (traj_has_algo(B, kPropLangevin))  // LDFA: an atom's coefficients serve its three dimensions
+        for (int i = threadIdx.x; i < T.N; i += blockDim.x)
+            if (B.algo[B.type[T.aoff + i]] == kPropLangevin) langevin_1(B, P, T, i, step, kPropLangevin);
     __syncthreads();
     if (traj_has_algo(B, kPropAndersen) || traj_has_algo(B, kPropPile)) remove_com(B, T, red);
 }
@@ -514,17 +659,18 @@ static __device__ void propagate_1(const Batch &B, const PropParams &P, const Tr
 // propagate_2, md_algo.f90:80-106
 static __device__ void propagate_2(const Batch &B, const PropParams &P, const TrajView &T, int step) {
     bool bad = false;
-    for (int i = threadIdx.x; i < T.N; i += blockDim.x) {
+    for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
+        const int d = w / T.N, i = w - d * T.N;
         const int algo = B.algo[B.type[T.aoff + i]];
-        if (algo == kPropLangevin) {
-            if (!ldfa(B, T, i)) bad = true;
-            langevin_2(B, P, T, i, step, algo);
-        } else if (algo == kPropLangevinConst) {
-            langevin_2(B, P, T, i, step, algo);
-        } else {
-            verlet_half(B, P, T, i, false);
-        }
+        if (algo == kPropLangevinConst) lc_half2(B, P, T, i, d, step);
+        else if (algo != kPropLangevin) verlet_half(B, P, T, i, d, false);
     }
+    if (traj_has_algo(B, kPropLangevin))
+        for (int i = threadIdx.x; i < T.N; i += blockDim.x)
+            if (B.algo[B.type[T.aoff + i]] == kPropLangevin) {
+                if (!ldfa(B, T, i)) bad = true;
+                langevin_2(B, P, T, i, step, kPropLangevin);
+            }
     if (bad) B.status[T.t] = kStatusErrDensity;
     __syncthreads();
 }
@@ -556,7 +702,7 @@ static __device__ void ring_polymer_step(const Batch &B, const PropParams &P, co
     for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
         const int i = w / 3, d = w - 3 * (w / 3);
         const int ty = B.type[T.aoff + i];
-        const double m = B.mass[T.aoff + i];
+        const double m = B.mass[T.aoff + i], im = B.imass[T.aoff + i];
         double p[32], q[32], np[32], nq[32];
         for (int b = 0; b < nb; ++b) {
             const int64_t k = T.base + (int64_t)b * T.N + i;
@@ -587,7 +733,7 @@ static __device__ void ring_polymer_step(const Batch &B, const PropParams &P, co
                 const int64_t k = T.base + (int64_t)b * T.N + i;
                 if (B.fixed[k] >> d & 1) continue;
                 comp(B.rx, B.ry, B.rz, d, k) = q[b];
-                comp(B.vx, B.vy, B.vz, d, k) = p[b] / m;
+                comp(B.vx, B.vy, B.vz, d, k) = div_by(p[b], m, im);
             }
         }
         if (revert) {
@@ -615,8 +761,8 @@ static __device__ void end_of_step(const Batch &B, const PropParams &P, const Tr
     const int tot = T.N * T.nb;
     for (int s = threadIdx.x; s < tot; s += blockDim.x) {
         const int64_t k = T.base + s;
-        const double a = (B.rx[k] + B.ry[k]) + (B.rz[k] + B.vx[k]) + (B.vy[k] + B.vz[k]);
-        bad |= isfinite(a) ? 0 : 1;
+        bad |= not_finite(B.rx[k]) || not_finite(B.ry[k]) || not_finite(B.rz[k]) || not_finite(B.vx[k]) ||
+               not_finite(B.vy[k]) || not_finite(B.vz[k]);
     }
     bad = __syncthreads_or(bad);
     if (threadIdx.x == 0) {
