@@ -156,49 +156,53 @@ static __device__ __forceinline__ void acsf_wrap_one(double xa, double ya, doubl
     }
 }
 
+// the oracle's cutoff test of one image in FP64, in its operation order (no fused multiply-add)
+static __device__ __noinline__ bool acsf_inside(double xi, double yi, double zi, double xj, double yj, double zj,
+                                                double d1n, double d2n, double d3n, const double *L, double cut2) {
+    const double xt = __dadd_rn(__dadd_rn(__dadd_rn(xj, __dmul_rn(d1n, L[0])), __dmul_rn(d2n, L[3])),
+                                __dmul_rn(d3n, L[6]));
+    const double yt = __dadd_rn(__dadd_rn(__dadd_rn(yj, __dmul_rn(d1n, L[1])), __dmul_rn(d2n, L[4])),
+                                __dmul_rn(d3n, L[7]));
+    const double zt = __dadd_rn(__dadd_rn(__dadd_rn(zj, __dmul_rn(d1n, L[2])), __dmul_rn(d2n, L[5])),
+                                __dmul_rn(d3n, L[8]));
+    const double e1 = __dsub_rn(xt, xi), e2 = __dsub_rn(yt, yi), e3 = __dsub_rn(zt, zi);
+    return __dadd_rn(__dadd_rn(__dmul_rn(e1, e1), __dmul_rn(e2, e2)), __dmul_rn(e3, e3)) <= cut2;
+}
+
 // neighbour list of atom i in RuNNer's order (neighbor_para_short.f90:117-163).
-// Returns the count (may exceed maxnb: the caller flags the overflow).
+// Returns the count (may exceed maxnb: the caller flags the overflow).  An FP32 screen, the exact
+// FP64 test only within 1e-4 (relative) of the cutoff.  Three FP64 subtractions per atom j; formed
+// per image, with the cell's conversions, the screen was 15 FP64-pipe instructions for each of
+// an atom's 27 and more images: most of the generic FP32 kernel's FP64 work.
 static __device__ int acsf_neighbors_one(const NNDev &M, int i, int N, const double *px, const double *py,
                                          const double *pz, const double *L, int na, int nbi, int nc, int *out) {
     const double cut2 = __dmul_rn(M.maxcut, M.maxcut);
-    const float cut2f_hi = (float)cut2 * 1.0001f, cut2f_lo = (float)cut2 * 0.9999f;
+    const float c2 = f32_of(cut2), cut2f_hi = c2 * 1.0001f, cut2f_lo = c2 * 0.9999f;
+    float Lf[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Lf[k] = f32_of(L[k]);
     int cnt = 0;
     const double xi = px[i], yi = py[i], zi = pz[i];
     for (int j = 0; j < N; ++j) {
         const double xj = px[j], yj = py[j], zj = pz[j];
+        const float dx = f32_of(xj - xi), dy = f32_of(yj - yi), dz = f32_of(zj - zi);
         for (int n1 = -na; n1 <= na; ++n1)
-            for (int n2 = -nbi; n2 <= nbi; ++n2)
+            for (int n2 = -nbi; n2 <= nbi; ++n2) {
+                const float g1 = (float)n1, g2 = (float)n2;
+                const float fx0 = dx + g1 * Lf[0] + g2 * Lf[3], fy0 = dy + g1 * Lf[1] + g2 * Lf[4],
+                            fz0 = dz + g1 * Lf[2] + g2 * Lf[5];
                 for (int n3 = -nc; n3 <= nc; ++n3) {
                     if (n1 == 0 && n2 == 0 && n3 == 0 && i == j) continue;
-                    const double d1n = n1, d2n = n2, d3n = n3;
-                    // FP32 screen; the exact FP64 test (the oracle's operation order, no
-                    // fused multiply-add) only within 1e-4 (relative) of the cutoff
-                    const float fx = (float)(xj - xi) + (float)d1n * (float)L[0] + (float)d2n * (float)L[3] +
-                                     (float)d3n * (float)L[6];
-                    const float fy = (float)(yj - yi) + (float)d1n * (float)L[1] + (float)d2n * (float)L[4] +
-                                     (float)d3n * (float)L[7];
-                    const float fz = (float)(zj - zi) + (float)d1n * (float)L[2] + (float)d2n * (float)L[5] +
-                                     (float)d3n * (float)L[8];
+                    const float g3 = (float)n3;
+                    const float fx = fx0 + g3 * Lf[6], fy = fy0 + g3 * Lf[7], fz = fz0 + g3 * Lf[8];
                     const float rf = fx * fx + fy * fy + fz * fz;
                     if (rf > cut2f_hi) continue;
-                    if (rf < cut2f_lo) {
-                        if (cnt < M.maxnb) out[cnt] = pack_nb(j, n1, n2, n3);
-                        ++cnt;
-                        continue;
-                    }
-                    const double xt = __dadd_rn(__dadd_rn(__dadd_rn(xj, __dmul_rn(d1n, L[0])), __dmul_rn(d2n, L[3])),
-                                                __dmul_rn(d3n, L[6]));
-                    const double yt = __dadd_rn(__dadd_rn(__dadd_rn(yj, __dmul_rn(d1n, L[1])), __dmul_rn(d2n, L[4])),
-                                                __dmul_rn(d3n, L[7]));
-                    const double zt = __dadd_rn(__dadd_rn(__dadd_rn(zj, __dmul_rn(d1n, L[2])), __dmul_rn(d2n, L[5])),
-                                                __dmul_rn(d3n, L[8]));
-                    const double e1 = __dsub_rn(xt, xi), e2 = __dsub_rn(yt, yi), e3 = __dsub_rn(zt, zi);
-                    const double rr = __dadd_rn(__dadd_rn(__dmul_rn(e1, e1), __dmul_rn(e2, e2)), __dmul_rn(e3, e3));
-                    if (rr <= cut2) {
+                    if (rf < cut2f_lo || acsf_inside(xi, yi, zi, xj, yj, zj, n1, n2, n3, L, cut2)) {
                         if (cnt < M.maxnb) out[cnt] = pack_nb(j, n1, n2, n3);
                         ++cnt;
                     }
                 }
+            }
     }
     return cnt;
 }
@@ -273,7 +277,7 @@ __device__ __forceinline__ bool triplet_setup(const NNDev &M, const WarpCache<R>
     if (!(T.rjk2 <= rc * rc)) return false;
     T.rjk = NM<R>::sq(T.rjk2);
     cutoff_fn<R>(M, rc, T.rjk, T.fcjk, T.dfcjk);
-    T.rinv0 = R(1) / (T.a[3] * T.c[3]);
+    T.rinv0 = NM<R>::rc(T.a[3] * T.c[3]);
     T.cost0 = (T.a[0] * T.c[0] + T.a[1] * T.c[1] + T.a[2] * T.c[2]) * T.rinv0;
     T.pfc = T.a[4] * T.c[4] * T.fcjk;
     const int ng = M.ng3eta[ei];
@@ -538,7 +542,7 @@ __device__ __forceinline__ bool triplet_geom(const NNDev &M, const WarpCache<R> 
     if (!(T.rjk2 <= rc * rc)) return false;
     T.rjk = NM<R>::sq(T.rjk2);
     cutoff_fn<R>(M, rc, T.rjk, T.fcjk, T.dfcjk);
-    T.rinv0 = R(1) / (T.a[3] * T.c[3]);
+    T.rinv0 = NM<R>::rc(T.a[3] * T.c[3]);
     T.cost0 = (T.a[0] * T.c[0] + T.a[1] * T.c[1] + T.a[2] * T.c[2]) * T.rinv0;
     T.pfc = T.a[4] * T.c[4] * T.fcjk;
     return true;
@@ -573,8 +577,15 @@ __device__ __forceinline__ void ladder_make(const GridConst<R> &g, R cost, Ladde
 
 template <typename R> __device__ __forceinline__ R ladder_pow(const Ladder<R> &L, int l, int e) {
     R r = R(1);
+    if constexpr (sizeof(R) == 8) {
+        // the exponent is the same for the whole warp: only the powers it holds are multiplied
 #pragma unroll
-    for (int b = 0; b < 5; ++b) r *= ((e >> b) & 1) ? L.pw[l][b] : R(1);
+        for (int b = 0; b < 5; ++b)
+            if ((e >> b) & 1) r *= L.pw[l][b];
+    } else {
+#pragma unroll
+        for (int b = 0; b < 5; ++b) r *= ((e >> b) & 1) ? L.pw[l][b] : R(1);
+    }
     return r;
 }
 
@@ -701,11 +712,20 @@ __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
                 A3 += plam * pp * S;
             }
             const R rij = T.a[3], rik = T.c[3];
-            const R P1 = T.pfc * (T.rinv0 - T.cost0 / (rij * rij)) * A1 - R(2) * T.pfc * A2 +
-                         T.c[4] * T.fcjk * T.a[5] / rij * A3;
-            const R P2 = T.pfc * (T.rinv0 - T.cost0 / (rik * rik)) * A1 - R(2) * T.pfc * A2 +
-                         T.a[4] * T.fcjk * T.c[5] / rik * A3;
-            const R P3 = T.pfc * T.rinv0 * A1 + R(2) * T.pfc * A2 - T.a[4] * T.c[4] * T.dfcjk / T.rjk * A3;
+            R P1, P2, P3;
+            if constexpr (sizeof(R) == 8) {
+                // 1/r_ij = r_ik/(r_ij r_ik) and so on: products for the five divisions
+                const R iij = T.rinv0 * rik, iik = T.rinv0 * rij, ijk = NM<R>::rc(T.rjk), w = R(2) * T.pfc * A2;
+                P1 = T.pfc * (T.rinv0 - T.cost0 * (iij * iij)) * A1 - w + T.c[4] * T.fcjk * T.a[5] * iij * A3;
+                P2 = T.pfc * (T.rinv0 - T.cost0 * (iik * iik)) * A1 - w + T.a[4] * T.fcjk * T.c[5] * iik * A3;
+                P3 = T.pfc * T.rinv0 * A1 + w - T.a[4] * T.c[4] * T.dfcjk * ijk * A3;
+            } else {
+                P1 = T.pfc * (T.rinv0 - T.cost0 / (rij * rij)) * A1 - R(2) * T.pfc * A2 +
+                     T.c[4] * T.fcjk * T.a[5] / rij * A3;
+                P2 = T.pfc * (T.rinv0 - T.cost0 / (rik * rik)) * A1 - R(2) * T.pfc * A2 +
+                     T.a[4] * T.fcjk * T.c[5] / rik * A3;
+                P3 = T.pfc * T.rinv0 * A1 + R(2) * T.pfc * A2 - T.a[4] * T.c[4] * T.dfcjk / T.rjk * A3;
+            }
             fix += T.a[0] * P1 + T.c[0] * P2;
             fiy += T.a[1] * P1 + T.c[1] * P2;
             fiz += T.a[2] * P1 + T.c[2] * P2;

@@ -337,11 +337,20 @@ int ensure_nn_scratch(mdt_ctx *c) {
     return MDT_OK;
 }
 
-LaunchCfg nn_cfg(mdt_ctx *c, int precision) {
+// split: force calls of single-bead MDT_PES_NENE trajectories may spread each trajectory's central
+// atoms over several CTAs, for at least two waves of the resident CTAs.  64 H/graphene
+// trajectories in FP64 occupied 64 of 152 SMs with one 4-warp CTA each.
+LaunchCfg nn_cfg(mdt_ctx *c, int precision, bool split = false) {
     const int per_sm = nn_resident_ctas(c->M, c->max_atoms, c->max_beads, c->ngeta_max, precision,
                                         c->pes_kind == MDT_PES_SURROGATE);
-    const int grid = std::max(1, std::min(c->T, c->num_sms * per_sm));
-    return LaunchCfg{c->stream, grid, c->order, c->counter};
+    const int slots = c->num_sms * per_sm;
+    LaunchCfg g{c->stream, std::max(1, std::min(c->T, slots)), c->order, c->counter};
+    if (split && c->pes_kind == MDT_PES_NENE && c->max_beads == 1) {
+        g.parts = std::max(1, std::min((2 * slots + c->T - 1) / c->T, (c->max_atoms + kNNWarps - 1) / kNNWarps));
+        g.grid = std::max(1, std::min(c->T * g.parts, slots));
+        g.total_ba = c->total_ba;
+    }
+    return g;
 }
 
 // Scaling of the fast path in FP32: scaled = x g + y, range flag outside [z, w], and the
@@ -1327,7 +1336,7 @@ int run_tc_generic(mdt_ctx *c, const PropParams &P, int mode, int tcm) {
     RadialNN R = c->RG;
     R.tc = tcm;
     if (nn_tc_smem(R.nin, R.nh, tcm) > (size_t)optin) return fail(c, MDT_ERR_UNSUPPORTED, kBf16Scope);
-    const LaunchCfg g = nn_cfg(c, MDT_PREC_FP32);
+    const LaunchCfg g = nn_cfg(c, MDT_PREC_FP32, true);
     NNScratch X = c->X;
     X.gout = c->tc_G;
     e = launch_nn(g, c->B, c->M, c->E, X, P, c->ngeta_max, 0, 1, MDT_PREC_FP32, false);  // descriptors
@@ -1367,7 +1376,7 @@ int32_t mdt_calc_force(mdt_ctx *c, int32_t flag, int32_t precision, const mdt_pr
         cudaError_t e = fast
                             ? launch_nnf(fcfg, c->B, c->M, c->F, c->E, c->X, P, 0,
                                          flag == MDT_ENERGY_ONLY ? 1 : 0, surr)
-                            : launch_nn(nn_cfg(c, precision), c->B, c->M, c->E, c->X, P, c->ngeta_max, 0,
+                            : launch_nn(nn_cfg(c, precision, true), c->B, c->M, c->E, c->X, P, c->ngeta_max, 0,
                                         flag == MDT_ENERGY_ONLY ? 1 : 0, precision, surr);
         c->launches++;
         return e == cudaSuccess ? MDT_OK : cuda_fail(c, e, "mdt_calc_force (network)");

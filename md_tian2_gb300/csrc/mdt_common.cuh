@@ -43,6 +43,16 @@ constexpr int kStatusStepLimit = 3;   // nsteps reached (the loop of md_tian2.f9
 constexpr int kStatusErrDensity = -10;  // ldfa: negative EMT density (md_algo.f90:551-554)
 constexpr int kStatusErrNonFinite = -11;
 
+// The pair loops' constants in the type of their arithmetic, per species slot.  Formed on the host:
+// converted in the kernel, the compiler repeats the conversions (FP64 pipe) in the loops rather
+// than hold them in registers.
+template <typename R> struct EmtPairs {
+    R acut, rcut, cut2;
+    R eta[2], etaq[2], b[2], kb[2];  // eta2, the density derivative's eta2, beta s0, kappa/beta
+    R g[2], c[2];                    // 1/gamma1, v0/gamma2
+    R gx[2], cx[2];                  // the same times chi towards the other species
+};
+
 // Derived EMT constants, computed on the host exactly like
 // compute_emt_2species (src/pes_emt_mod.f90:521-592).  Species slot 0 is the
 // reference's "type1" (first type with pes(i,i)==emt), slot 1 its "type2".
@@ -60,6 +70,8 @@ struct EmtConst {
     double n0[2], e0[2], lambda[2], kappa[2], v0[2], dens_exp[2];
     double chi[2][2];             // density at a from neighbour b scaled by chi[a][b]
     double ibe[2], e0l2[2], v6[2], v6k[2];  // 1/betaeta2, e0 lambda^2, 6 v0, 6 v0 kappa
+    EmtPairs<double> pd;
+    EmtPairs<float> pf;
 };
 
 // Everything a kernel needs to address the batch.  Passed by value.

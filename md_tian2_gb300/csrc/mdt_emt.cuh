@@ -2,7 +2,6 @@
 // the EMT kernels and the surrogate's EMT fallback).
 #pragma once
 #include "mdt_common.cuh"
-#include "mdt_exp2tab.cuh"
 #include "mdt_fastmath.cuh"
 
 namespace mdt {
@@ -24,50 +23,6 @@ constexpr int kBlock = 128;  // threads per CTA (one trajectory per CTA)
 //    applied in FP64; when FP32 cannot decide the rounding (fractional part within
 //    1e-4 of 1/2) the fractional coordinate is recomputed in FP64.
 // ---------------------------------------------------------------------------
-static __device__ __forceinline__ double rcp_nr(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);  // 1/x = y (1 + e + e^2 + ...)
-    return fma(y, fma(e, e, e), y);
-}
-
-static __device__ __forceinline__ double rsqrt_nr(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y * y, 1.0);  // 1/sqrt(x) = y (1 + e/2 + 3 e^2/8 + ...)
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
-// n/d from the reciprocal id of d (within an ulp or two): the residual's correction makes the
-// quotient round as a division does, in 3 FP64 instructions instead of about 10
-static __device__ __forceinline__ double div_by(double n, double d, double id) {
-    const double q = n * id;
-    return fma(fma(-q, d, n), id, q);
-}
-
-// FP64 exp by the table-driven method of Tang (ACM TOMS 15(2), 1989): x = (512 n_hi + j)
-// ln2/512 + r with |r| <= ln2/1024, exp(x) = 2^n_hi 2^(j/512) (1 + p(r)), p the Taylor series
-// of exp(r) - 1 to r^4 (truncation below 2^-59).  ln2/512 enters in two parts (its double,
-// then the remainder) so that r is exact to ~2^-100, and n = round(512 x / ln2) comes from
-// adding 1.5 * 2^52.  10 FP64 instructions (13 with 64 entries and r^5, ~19 for exp()); the
-// range test reads the high word, because a FP64 comparison costs as much as an addition.
-// Outside [-700, 700], and for NaN, exp() itself.
-static __device__ __forceinline__ double exp_t64(double x) {
-    if ((__double2hiint(x) & 0x7fffffff) >= 0x4085e000) return exp(x);  // |x| >= 700
-    const double shifter = 6755399441055744.0;
-    const double t = fma(x, 738.65986093514926, shifter);
-    const int n = __double2loint(t);
-    const double nd = t - shifter;
-    double r = fma(-nd, 0x1.62e42fefa39efp-10, x);
-    r = fma(-nd, 0x1.abc9e3b39803fp-65, r);
-    double q = fma(r, 1.0 / 24.0, 1.0 / 6.0);
-    q = fma(r, q, 0.5);
-    const double pr = fma(r * r, q, r);
-    const double tj = __ldg(kExp2Tab + (n & 511));
-    const double y = fma(tj, pr, tj);
-    return __hiloint2double(__double2hiint(y) + (n >> 9) * (1 << 20), __double2loint(y));
-}
-
 template <typename R> struct Math;
 template <> struct Math<double> {
     static __device__ __forceinline__ double ex(double x) { return exp_t64(x); }
@@ -84,10 +39,12 @@ struct Cell;
 
 template <typename R> struct SmemEmt {
     double *px, *py, *pz;  // staged bead positions
-    float *xh, *yh, *zh, *xl, *yl, *zl;  // FP32 forces (R = float): their FP32 hi/lo split
+    float4 *ph, *pl;       // FP32 forces (R = float): their FP32 hi/lo split
     R *sig, *A, *fx, *fy, *fz;
     Cell *cell;
-    int16_t *perm;         // atom of each staged place (places: species slot 0, slot 1, none)
+    double *en;            // per place: the bead's energies (several beads at a time)
+    int places;            // staged atoms the arrays hold (beads at a time x atoms)
+    int16_t *perm;         // atom of each place of a bead (places: species slot 0, slot 1, none)
     int *seg;              // first place of each of the three groups, N, runs per atom of slots 0 and 1
     double *red;           // 64 doubles for block reductions
     double *img;           // the 27 image-shift vectors of |n| <= 1 per direction (FP64 forces)
@@ -100,8 +57,14 @@ __host__ __device__ constexpr size_t rp_cells(int max_beads) {
     return (size_t)max_beads * max_beads + 5 * (size_t)kMaxTypes * max_beads;
 }
 
+// staged atoms of the EMT kernels: the beads of a ring polymer are evaluated several at a time
+// (their per-atom FP64 work fills warps, and the CTA's barriers are shared), up to 512 atoms
+__host__ __device__ constexpr int emt_places(int max_atoms, int max_beads) {
+    return max_atoms * max_beads <= 512 ? max_atoms * max_beads : max_atoms <= 512 ? 512 / max_atoms * max_atoms : max_atoms;
+}
+
 template <typename R>
-static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int max_beads) {
+static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int max_beads, int places) {
     SmemEmt<R> s;
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -109,34 +72,34 @@ static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int 
         off += (bytes + 15) & ~size_t(15);
         return p;
     };
-    s.px = (double *)take(sizeof(double) * max_atoms);
-    s.py = (double *)take(sizeof(double) * max_atoms);
-    s.pz = (double *)take(sizeof(double) * max_atoms);
-    const size_t nf = sizeof(R) == 4 ? sizeof(float) * max_atoms : 0;
-    s.xh = (float *)take(nf);
-    s.yh = (float *)take(nf);
-    s.zh = (float *)take(nf);
-    s.xl = (float *)take(nf);
-    s.yl = (float *)take(nf);
-    s.zl = (float *)take(nf);
+    const int dp = sizeof(R) == 8 ? places : 0;  // FP64 forces: FP64 positions; FP32: their hi/lo split
+    s.places = places;
+    s.px = (double *)take(sizeof(double) * dp);
+    s.py = (double *)take(sizeof(double) * dp);
+    s.pz = (double *)take(sizeof(double) * dp);
+    const size_t nf = sizeof(R) == 4 ? sizeof(float4) * places : 0;
+    s.ph = (float4 *)take(nf);
+    s.pl = (float4 *)take(nf);
     s.red = (double *)take(sizeof(double) * 64);
     s.img = (double *)take(sizeof(double) * 81);
     s.cjk = (double *)take(sizeof(double) * rp_cells(max_beads));
-    s.sig = (R *)take(sizeof(R) * max_atoms);
-    s.A = (R *)take(sizeof(R) * max_atoms);
-    s.fx = (R *)take(sizeof(R) * max_atoms);
-    s.fy = (R *)take(sizeof(R) * max_atoms);
-    s.fz = (R *)take(sizeof(R) * max_atoms);
+    s.sig = (R *)take(sizeof(R) * places);
+    s.A = (R *)take(sizeof(R) * places);
+    s.fx = (R *)take(sizeof(R) * places);
+    s.fy = (R *)take(sizeof(R) * places);
+    s.fz = (R *)take(sizeof(R) * places);
+    s.en = (double *)take(max_beads > 1 ? sizeof(double) * places : 0);
     s.cell = (Cell *)take(256);
     s.perm = (int16_t *)take(sizeof(int16_t) * max_atoms);
     s.seg = (int *)take(sizeof(int) * 6);
     return s;
 }
 
-inline size_t smem_bytes(int max_atoms, int max_beads, size_t rsize) {
+inline size_t smem_bytes(int max_atoms, int max_beads, size_t rsize, int places) {
     auto r16 = [](size_t b) { return (b + 15) & ~size_t(15); };
-    return 3 * r16(8 * max_atoms) + (rsize == 4 ? 6 * r16(4 * max_atoms) : 0) + r16(8 * 64) + r16(8 * 81) +
-           r16(8 * rp_cells(max_beads)) + 5 * r16(rsize * max_atoms) + 256 + r16(2 * max_atoms) + 32;
+    return (rsize == 8 ? 3 * r16(8 * places) : 32 * (size_t)places) + r16(8 * 64) + r16(8 * 81) +
+           r16(8 * rp_cells(max_beads)) + 5 * r16(rsize * places) + (max_beads > 1 ? r16(8 * places) : 0) + 256 +
+           r16(2 * max_atoms) + 32;
 }
 
 // Block-wide sum of a double; every thread gets the result.
@@ -210,27 +173,87 @@ static __device__ __forceinline__ double image_shift(float wf, const double *hi_
     return round(w);
 }
 
-// FP32 bead forces: the minimum image of r_i - r_j from the FP32 hi/lo split of the
-// positions, with the image chosen as min_image chooses it (FP32, exact ties in FP64)
-// and applied in FP32: no FP64 instruction per pair unless a pair sits on a tie.
-template <typename S_>
-static __device__ __forceinline__ void min_image_f(const Cell &c, const S_ &S, int i, int j, float &dx, float &dy,
-                                            float &dz) {
-    const float ex = (S.xh[i] - S.xh[j]) + (S.xl[i] - S.xl[j]);
-    const float ey = (S.yh[i] - S.yh[j]) + (S.yl[i] - S.yl[j]);
-    const float ez = (S.zh[i] - S.zh[j]) + (S.zl[i] - S.zl[j]);
-    float n[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const float w = c.hif[r] * ex + c.hif[r + 3] * ey + c.hif[r + 6] * ez;
-        n[r] = roundf(w);
-        if (!(fabsf(fabsf(w - n[r]) - 0.5f) > 1e-4f))
-            n[r] = (float)image_shift(w, c.hi, S.px[i] - S.px[j], S.py[i] - S.py[j], S.pz[i] - S.pz[j], r);
-    }
-    dx = ex - (c.hf[0] * n[0] + c.hf[3] * n[1] + c.hf[6] * n[2]);
-    dy = ey - (c.hf[1] * n[0] + c.hf[4] * n[1] + c.hf[7] * n[2]);
-    dz = ez - (c.hf[2] * n[0] + c.hf[5] * n[1] + c.hf[8] * n[2]);
+// all three image indices of a pair of which one sits on a tie
+static __device__ __noinline__ float3 image_exact(const Cell &c, float3 w, double ex, double ey, double ez) {
+    return make_float3((float)image_shift(w.x, c.hi, ex, ey, ez, 0), (float)image_shift(w.y, c.hi, ex, ey, ez, 1),
+                       (float)image_shift(w.z, c.hi, ex, ey, ez, 2));
 }
+
+// nearest integer of an image coordinate |w| < 2^21 (ties to even; the caller treats ties)
+static __device__ __forceinline__ float image_round(float w) { return (w + 12582912.f) - 12582912.f; }
+
+// Minimum image of one staged place against others, the place and the cell held in registers (the
+// pair loops write the scratch, so nothing read through pointers stays in a register by itself).
+template <typename R> struct PlaceDiff;
+
+// FP32 forces, from the FP32 hi/lo split of the positions, with the image chosen as min_image
+// chooses it (FP32, exact ties in FP64) and applied in FP32: no FP64 instruction per pair unless
+// a pair sits on a tie.
+template <> struct PlaceDiff<float> {
+    float xh, yh, zh, xl, yl, zl, h[9], hi[9];
+    int i;
+    bool slab;                   // in-plane cell vectors and one along z: the other entries are zero
+    const double *rx, *ry, *rz;  // positions of the bead in global memory (ties)
+    const int16_t *perm;
+    const Cell *cell;
+    template <typename S_>
+    __device__ __forceinline__ PlaceDiff(const Batch &B, const S_ &S, int64_t base0)
+        : rx(B.rx + base0), ry(B.ry + base0), rz(B.rz + base0), perm(S.perm), cell(S.cell) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            h[k] = S.cell->hf[k];
+            hi[k] = S.cell->hif[k];
+        }
+        slab = h[2] == 0.f && h[5] == 0.f && h[6] == 0.f && h[7] == 0.f && hi[2] == 0.f && hi[5] == 0.f &&
+               hi[6] == 0.f && hi[7] == 0.f;
+    }
+    template <typename S_> __device__ __forceinline__ void set(const S_ &S, int place) {
+        i = place;
+        const float4 a = S.ph[place], b = S.pl[place];
+        xh = a.x;
+        yh = a.y;
+        zh = a.z;
+        xl = b.x;
+        yl = b.y;
+        zl = b.z;
+    }
+    // N: atoms of a bead; places i and j belong to the same one
+    template <typename S_>
+    __device__ __forceinline__ void diff(const S_ &S, int j, int N, float &dx, float &dy, float &dz) const {
+        const float4 a = S.ph[j], b = S.pl[j];
+        const float ex = (xh - a.x) + (xl - b.x), ey = (yh - a.y) + (yl - b.y), ez = (zh - a.z) + (zl - b.z);
+        float n[3], w[3];
+        if (slab) {  // the same sums without their zero terms
+            w[0] = hi[0] * ex + hi[3] * ey;
+            w[1] = hi[1] * ex + hi[4] * ey;
+            w[2] = hi[8] * ez;
+        } else {
+#pragma unroll
+            for (int r = 0; r < 3; ++r) w[r] = hi[r] * ex + hi[r + 3] * ey + hi[r + 6] * ez;
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) n[r] = image_round(w[r]);
+        const float off = fmaxf(fabsf(w[0] - n[0]), fmaxf(fabsf(w[1] - n[1]), fabsf(w[2] - n[2])));
+        const float big = fmaxf(fabsf(w[0]), fmaxf(fabsf(w[1]), fabsf(w[2])));
+        if (!(off < 0.4999f && big < 2097152.f)) {
+            const int g = i / N * N;  // the bead's slots follow each other as its places do
+            const int64_t p = g + perm[i - g], q = g + perm[j - g];
+            const float3 m = image_exact(*cell, make_float3(w[0], w[1], w[2]), rx[p] - rx[q], ry[p] - ry[q], rz[p] - rz[q]);
+            n[0] = m.x;
+            n[1] = m.y;
+            n[2] = m.z;
+        }
+        if (slab) {
+            dx = ex - (h[0] * n[0] + h[3] * n[1]);
+            dy = ey - (h[1] * n[0] + h[4] * n[1]);
+            dz = ez - h[8] * n[2];
+        } else {
+            dx = ex - (h[0] * n[0] + h[3] * n[1] + h[6] * n[2]);
+            dy = ey - (h[1] * n[0] + h[4] * n[1] + h[7] * n[2]);
+            dz = ez - (h[2] * n[0] + h[5] * n[1] + h[8] * n[2]);
+        }
+    }
+};
 
 // minimum image of e = r_i - r_j, src/universe_mod.f90:411-428
 static __device__ __forceinline__ void min_image(const Cell &c, double ex, double ey, double ez, double &dx, double &dy,
@@ -262,6 +285,12 @@ static __device__ __forceinline__ void min_image(const Cell &c, double ex, doubl
     }
 }
 
+static __device__ __noinline__ double3 min_image_far(const Cell &c, double ex, double ey, double ez) {
+    double3 d;
+    min_image(c, ex, ey, ez, d.x, d.y, d.z);
+    return d;
+}
+
 // the 27 shifts h n of |n| <= 1 per direction, entry 9 (n0 + 1) + 3 (n1 + 1) + (n2 + 1); by the
 // first warp, after load_cell
 static __device__ __forceinline__ void image_table(const Cell &c, double *img) {
@@ -271,54 +300,82 @@ static __device__ __forceinline__ void image_table(const Cell &c, double *img) {
     for (int d = 0; d < 3; ++d) img[3 * k + d] = fma(c.h[d], n0, fma(c.h[d + 3], n1, c.h[d + 6] * n2));
 }
 
-// min_image with its shift from the table: no FP64 conversion, comparison or product.  A
-// fractional coordinate near a tie, or an image further away, takes min_image itself.
-static __device__ __forceinline__ void min_image_t(const Cell &c, const double *img, double ex, double ey, double ez,
-                                                   double &dx, double &dy, double &dz) {
-    const float fx = f32_of(ex), fy = f32_of(ey), fz = f32_of(ez);
-    int n[3];
-    bool plain = true;
+// FP64 forces: min_image with its shift from the table: no FP64 conversion, comparison or product.
+// A fractional coordinate near a tie, or an image further away, takes min_image itself.
+template <> struct PlaceDiff<double> {
+    double x, y, z;
+    float hi[9];
+    const Cell *cell;
+    const double *img;
+    template <typename S_>
+    __device__ __forceinline__ PlaceDiff(const Batch &, const S_ &S, int64_t) : cell(S.cell), img(S.img) {
 #pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        const float w = c.hif[r] * fx + c.hif[r + 3] * fy + c.hif[r + 6] * fz;
-        const float f = rintf(w);
-        plain = plain && fabsf(fabsf(w - f) - 0.5f) > 1e-4f && fabsf(f) <= 1.f;
-        n[r] = (int)f;
+        for (int k = 0; k < 9; ++k) hi[k] = S.cell->hif[k];
     }
-    dx = ex;
-    dy = ey;
-    dz = ez;
-    if (plain) {
-        const int k = 9 * n[0] + 3 * n[1] + n[2] + 13;
-        if (k != 13) {
-            dx -= img[3 * k];
-            dy -= img[3 * k + 1];
-            dz -= img[3 * k + 2];
+    template <typename S_> __device__ __forceinline__ void set(const S_ &S, int place) {
+        x = S.px[place];
+        y = S.py[place];
+        z = S.pz[place];
+    }
+    template <typename S_>
+    __device__ __forceinline__ void diff(const S_ &S, int j, int, double &dx, double &dy, double &dz) const {
+        const double ex = x - S.px[j], ey = y - S.py[j], ez = z - S.pz[j];
+        const float fx = f32_of(ex), fy = f32_of(ey), fz = f32_of(ez);
+        float n[3], w[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            w[r] = hi[r] * fx + hi[r + 3] * fy + hi[r + 6] * fz;
+            n[r] = image_round(w[r]);
         }
-    } else {
-        min_image(c, ex, ey, ez, dx, dy, dz);
+        const float off = fmaxf(fabsf(w[0] - n[0]), fmaxf(fabsf(w[1] - n[1]), fabsf(w[2] - n[2])));
+        const float big = fmaxf(fabsf(w[0]), fmaxf(fabsf(w[1]), fabsf(w[2])));
+        dx = ex;
+        dy = ey;
+        dz = ez;
+        if (off < 0.4999f && big < 1.5f) {
+            const float kf = 9.f * n[0] + 3.f * n[1] + n[2];
+            if (kf != 0.f) {
+                const double *v = img + 3 * ((int)kf + 13);
+                dx -= v[0];
+                dy -= v[1];
+                dz -= v[2];
+            }
+        } else {
+            const double3 d = min_image_far(*cell, ex, ey, ez);
+            dx = d.x;
+            dy = d.y;
+            dz = d.z;
+        }
     }
-}
+};
 
 // ---------------------------------------------------------------------------
-// EMT for one bead of one trajectory.  Adds forces into B.f* (stores them when `store`), sets
-// dens, adds the bead's energy into B.epot.  Must be called by all threads of the CTA.
+// EMT for G beads (b0 ..) of one trajectory, G N <= S.places.  Adds forces into B.f* (stores them
+// when `store`), sets dens, adds the beads' energies into B.epot.  Must be called by all threads
+// of the CTA.
 //
-// Atoms are staged by species: places [seg[0], seg[1]) hold the atoms of species slot 0,
-// [seg[1], seg[2]) those of slot 1, the rest are not EMT.  Almost every pair has two atoms of
+// Atoms are staged by species: places [seg[0], seg[1]) of a bead hold the atoms of species slot 0,
+// [seg[1], seg[2]) those of slot 1, the rest are not EMT; bead g follows at place g N.  Almost every pair has two atoms of
 // the metal, so pairs are walked per species with the species' constants in registers and no
 // branch; the few pairs of the two species run in a loop of their own (in one common walk nearly
 // every warp met one of them, and took both branches).
 //
-// Pairs of one species (M atoms): (i, j = (i+k) mod M), k = 1..M/2, in scratch slot
+// Pairs of one species, FP32 forces: a thread takes one atom i and a run of partners j and keeps
+// its sums in registers; every pair is evaluated from both ends, in the density pass and again in
+// the force pass (about 80 and 100 instructions).  Storing a pair's six values and reading them
+// back by both ends took as many instructions and waited on the L2 for them.
+// Pairs of one species, FP64 forces (M atoms): (i, j = (i+k) mod M), k = 1..M/2, in scratch slot
 // (k-1) M + i (the k = M/2 row holds only i < M/2 when M is even).  A thread takes one atom i
 // and a run of k: its side of a pair sums in registers, the other side is read back from the
 // scratch by the thread that owns j (lanes hold consecutive i: every access coalesces).  A
 // shared-memory FP64 addition costs 137 cycles a warp, reading the value back 5.
 //   pass 1  distance, density term rho, pair energy, and the scalars q = -rho'/r, fv of the force
 //   epilogue (per atom) sigma -> s, cohesive energy, embedded density, A = (dE/ds)/(beta eta2 sigma)
-//   pass 2  cc = (A_i + A_j) q + fv, force += cc d on i; cc left in q's slot; then -cc d on j
+//   pass 2  cc = (A_i + A_j) q + fv, force += cc d on i; FP64: cc left in q's slot, then -cc d on j
 // ---------------------------------------------------------------------------
+static __device__ __forceinline__ const EmtPairs<double> &emt_pairs(const EmtConst &E, double) { return E.pd; }
+static __device__ __forceinline__ const EmtPairs<float> &emt_pairs(const EmtConst &E, float) { return E.pf; }
+
 template <typename R> struct PairK {
     R acut, rcut, eta, etaq, b, kb, g, c;
 };
@@ -346,6 +403,7 @@ template <typename R> struct EnergySum;
 template <> struct EnergySum<double> {
     double s = 0.0;
     __device__ __forceinline__ void add(double x) { s += x; }
+    __device__ __forceinline__ void join(const EnergySum &o) { s += o.s; }
     __device__ __forceinline__ double value() const { return s; }
 };
 template <> struct EnergySum<float> {
@@ -355,21 +413,31 @@ template <> struct EnergySum<float> {
         c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z)));
         s = t;
     }
-    __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+    __device__ __forceinline__ void join(const EnergySum &o) {
+        add(o.s);
+        c = __fadd_rn(c, o.c);
+    }
+    __device__ __forceinline__ double value() const { return f64_of(s) + f64_of(c); }
 };
 
-__device__ __forceinline__ bool is_zero(double x) {
+static __device__ __forceinline__ bool is_zero(double x) {
     return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
 }
-__device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
+static __device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
+static __device__ __forceinline__ double wide(double x) { return x; }
+static __device__ __forceinline__ double wide(float x) { return f64_of(x); }
 
-// displacement (minimum image) of staged places i, j
-template <typename R>
-static __device__ __forceinline__ void place_diff(const SmemEmt<R> &S, int i, int j, R &rx, R &ry, R &rz) {
-    if constexpr (sizeof(R) == 4)
-        min_image_f(*S.cell, S, i, j, rx, ry, rz);
-    else
-        min_image_t(*S.cell, S.img, S.px[i] - S.px[j], S.py[i] - S.py[j], S.pz[i] - S.pz[j], rx, ry, rz);
+// acc[place] += the sum of v over the lanes of each place (a warp's lanes hold one, or a few where
+// it spans beads): one shared-memory addition per place.
+template <typename R> static __device__ __forceinline__ void warp_add(R *acc, int place, R v) {
+    for (unsigned left = 0xffffffffu; left;) {
+        const int src = __ffs(left) - 1, pl = __shfl_sync(0xffffffffu, place, src);
+        const bool mine = place == pl;
+        R s = mine ? v : R(0);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31) == src && !is_zero(s)) atomicAdd(&acc[pl], s);
+        left &= ~__ballot_sync(0xffffffffu, mine);
+    }
 }
 
 // Beyond the cutoff, like the reference's `if (r > cutoff*rcut) cycle` (pes_emt_mod.f90:660): a
@@ -381,20 +449,233 @@ static __device__ __forceinline__ bool beyond(double r2, double cut2) {
 }
 static __device__ __forceinline__ bool beyond(float r2, float cut2) { return r2 > cut2; }
 
-// Runs of k per atom (1..16) so that the M C work items of the pair loops fill the CTA's rounds
-// best (cost: rounds x run length; a run also pays its sums once).  One warp, lane = candidate.
-static __device__ __forceinline__ int pair_chunks(int M, int nt) {
-    const int C = (threadIdx.x & 15) + 1, K = M / 2;
-    const int cost = C <= K || C == 1 ? ((M * C + nt - 1) / nt) * (2 * ((K + C - 1) / C) + 1) : 1 << 26;
-    const int best = __reduce_min_sync(0xffffffffu, cost << 4 | (C - 1));
+// Runs per atom (1..16) of its `span` partners so that the G M C work items of the pair loops fill
+// the CTA's rounds best (cost: rounds x run length; a run also pays its sums once).  One warp,
+// lane = candidate.
+static __device__ __forceinline__ int pair_chunks(int M, int span, int G, int nt) {
+    const int C = (threadIdx.x & 15) + 1;
+    const int64_t cost =
+        C <= span || C == 1 ? (int64_t)((G * M * C + nt - 1) / nt) * (2 * ((span + C - 1) / C) + 1) : 1 << 26;
+    const int best = __reduce_min_sync(0xffffffffu, (int)min(cost, (int64_t)1 << 26) << 4 | (C - 1));
     return (best & 15) + 1;
 }
 
+// One species' places in the staged beads (m0 .. m0 + M - 1 of each), the runs per atom and, FP64
+// forces, the scratch records of its pairs: (d, q) at rec4 + 4 slot, (fv, rho) at rec2 + 2 slot,
+// `stride` values per bead.
+template <typename R> struct Species {
+    int N, G, m0, M, C;
+    R *rec4, *rec2;
+    int64_t stride;
+    R cut2;
+};
+
+// calls f(bead, atom, first, last) for this thread's runs; `span` partners per atom
+template <typename F> static __device__ __forceinline__ void for_runs(int G, int M, int C, int span, F f) {
+    const int per = (span + C - 1) / C, GM = G * M;
+    for (int w = threadIdx.x; w < GM * C; w += blockDim.x) {
+        const int c = w / GM, g = (w - c * GM) / M;
+        f(g, w - c * GM - g * M, c * per, min((c + 1) * per, span));
+    }
+}
+
+// ---- FP32 forces: pairs of one species from both ends -------------------------------------
+static __device__ __forceinline__ void pairs_density(const SmemEmt<float> &S, PlaceDiff<float> &D, const PairK<float> &k,
+                                                     const Species<float> &A, bool, EnergySum<float> &) {
+    for_runs(A.G, A.M, A.C, A.M, [&](int g, int i, int j0, int j1) {
+        const int gp = g * A.N + A.m0;
+        float acc = 0.f;
+        D.set(S, gp + i);
+        for (int j = j0; j < j1; ++j) {
+            if (j == i) continue;
+            float rx, ry, rz;
+            D.diff(S, gp + j, A.N, rx, ry, rz);
+            const float r2 = rx * rx + ry * ry + rz * rz;
+            if (beyond(r2, A.cut2)) continue;
+            const float r = r2 * Math<float>::rsq(r2);
+            float theta, rt1;
+            emt_theta<float>(k.acut, k.rcut, r, theta, rt1);
+            acc += k.g * (theta * Math<float>::ex(-k.eta * (r - k.b)));
+        }
+        if (A.C == 1) S.sig[gp + i] = acc;
+        else atomicAdd(&S.sig[gp + i], acc);
+    });
+}
+static __device__ __forceinline__ void pairs_density_2(const SmemEmt<float> &, const Species<float> &) {}
+
+// forces and pair energies (a pair's energy from its first end)
+static __device__ __forceinline__ void pairs_force(const SmemEmt<float> &S, PlaceDiff<float> &D, const PairK<float> &k,
+                                                   const Species<float> &A, bool do_forces, EnergySum<float> &e_pair) {
+    for_runs(A.G, A.M, A.C, A.M, [&](int g, int i, int j0, int j1) {
+        const int gp = g * A.N + A.m0;
+        const float Ai = S.A[gp + i];
+        float fx = 0.f, fy = 0.f, fz = 0.f;
+        EnergySum<float> e_run;
+        D.set(S, gp + i);
+        for (int j = j0; j < j1; ++j) {
+            if (j == i) continue;
+            float rx, ry, rz;
+            D.diff(S, gp + j, A.N, rx, ry, rz);
+            const float r2 = rx * rx + ry * ry + rz * rz;
+            if (beyond(r2, A.cut2)) continue;
+            const float ir = Math<float>::rsq(r2), r = r2 * ir;
+            float theta, rt1;
+            emt_theta<float>(k.acut, k.rcut, r, theta, rt1);
+            const float phi = theta * Math<float>::ex(-k.eta * (r - k.b));
+            const float psi = theta * Math<float>::ex(-k.kb * (r - k.b));
+            if (i < j) e_run.add(-(k.c * psi));
+            const float q = k.g * (k.etaq + rt1) * phi * ir, fv = -(k.c * (k.kb + rt1) * psi * ir);
+            const float cc = Ai * q + S.A[gp + j] * q + fv;
+            fx += cc * rx;
+            fy += cc * ry;
+            fz += cc * rz;
+        }
+        if (do_forces) {
+            atomicAdd(&S.fx[gp + i], fx);
+            atomicAdd(&S.fy[gp + i], fy);
+            atomicAdd(&S.fz[gp + i], fz);
+        }
+        if (A.G == 1) e_pair.join(e_run);
+        else atomicAdd(&S.en[gp + i], e_run.value());
+    });
+}
+static __device__ __forceinline__ void pairs_force_2(const SmemEmt<float> &, const Species<float> &) {}
+
+// ---- FP64 forces: each pair once, its other end through the scratch ----------------------
+static __device__ __forceinline__ void pairs_density(const SmemEmt<double> &S, PlaceDiff<double> &D,
+                                                     const PairK<double> &k, const Species<double> &A, bool do_forces,
+                                                     EnergySum<double> &e_pair) {
+    const int M = A.M, K = M / 2;
+    for_runs(A.G, M, A.C, K, [&](int g, int i, int k0, int k1) {
+        const int gp = g * A.N + A.m0;
+        double acc = 0.0;
+        EnergySum<double> e_run;
+        D.set(S, gp + i);
+        if (2 * K == M && i >= K) k1 = min(k1, K - 1);  // the last row of an even M holds each pair once
+        for (int kk = k0; kk < k1; ++kk) {
+            int j = i + kk + 1;
+            if (j >= M) j -= M;
+            double q = 0.0, fv = 0.0, rho = 0.0, rx, ry, rz;
+            D.diff(S, gp + j, A.N, rx, ry, rz);
+            const double r2 = rx * rx + ry * ry + rz * rz;
+            if (!beyond(r2, A.cut2)) {
+                const double ir = Math<double>::rsq(r2), r = r2 * ir;
+                double theta, rt1;
+                emt_theta<double>(k.acut, k.rcut, r, theta, rt1);
+                const double phi = theta * Math<double>::ex(-k.eta * (r - k.b));
+                const double psi = theta * Math<double>::ex(-k.kb * (r - k.b));
+                rho = k.g * phi;
+                acc += rho;
+                e_run.add(-(k.c * psi));
+                q = (k.etaq + rt1) * rho * ir;
+                fv = -(k.c * (k.kb + rt1) * psi * ir);
+            }
+            const int64_t slot = A.stride * g + kk * M + i;
+            *reinterpret_cast<double2 *>(A.rec2 + 2 * slot) = make_double2(fv, rho);
+            if (do_forces) {
+                double2 *p = reinterpret_cast<double2 *>(A.rec4 + 4 * slot);
+                p[0] = make_double2(rx, ry);
+                p[1] = make_double2(rz, q);
+            }
+        }
+        if (A.C == 1) S.sig[gp + i] = acc;
+        else atomicAdd(&S.sig[gp + i], acc);
+        if (A.G == 1) e_pair.join(e_run);
+        else if (A.C == 1) S.en[gp + i] = e_run.value();
+        else atomicAdd(&S.en[gp + i], e_run.value());
+    });
+}
+
+// the densities' other end
+static __device__ __forceinline__ void pairs_density_2(const SmemEmt<double> &S, const Species<double> &A) {
+    const int M = A.M, K = M / 2;
+    for_runs(A.G, M, A.C, K, [&](int g, int j, int k0, int k1) {
+        double acc = 0.0;
+        // row k holds the pair whose second atom is j at place j - k (mod M); the last row of an
+        // even M only for places below K
+        if (2 * K == M && k1 == K && j < K) k1 = K - 1;
+#pragma unroll 4
+        for (int kk = k0; kk < k1; ++kk) {
+            int m = j - kk - 1;
+            if (m < 0) m += M;
+            const double rho = A.rec2[2 * (A.stride * g + kk * M + m) + 1];
+            if (!is_zero(rho)) acc += rho;
+        }
+        if (A.C == 1) S.sig[g * A.N + A.m0 + j] += acc;
+        else atomicAdd(&S.sig[g * A.N + A.m0 + j], acc);
+    });
+}
+
+static __device__ __forceinline__ void pairs_force(const SmemEmt<double> &S, PlaceDiff<double> &, const PairK<double> &,
+                                                   const Species<double> &A, bool do_forces, EnergySum<double> &) {
+    if (!do_forces) return;
+    const int M = A.M, K = M / 2;
+    for_runs(A.G, M, A.C, K, [&](int g, int i, int k0, int k1) {
+        const int gp = g * A.N + A.m0;
+        const double Ai = S.A[gp + i];
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        if (2 * K == M && i >= K) k1 = min(k1, K - 1);
+#pragma unroll 2
+        for (int kk = k0; kk < k1; ++kk) {
+            int j = i + kk + 1;
+            if (j >= M) j -= M;
+            const int64_t slot = A.stride * g + kk * M + i;
+            double2 *p = reinterpret_cast<double2 *>(A.rec4 + 4 * slot);
+            const double2 a = p[0], c = p[1];
+            if (is_zero(c.y)) continue;  // beyond the cutoff: the 0 stays in q's place
+            const double cc = (Ai + S.A[gp + j]) * c.y + A.rec2[2 * slot];
+            A.rec4[4 * slot + 3] = cc;
+            fx += cc * a.x;
+            fy += cc * a.y;
+            fz += cc * c.x;
+        }
+        if (A.C == 1) {
+            S.fx[gp + i] = fx;
+            S.fy[gp + i] = fy;
+            S.fz[gp + i] = fz;
+        } else {
+            atomicAdd(&S.fx[gp + i], fx);
+            atomicAdd(&S.fy[gp + i], fy);
+            atomicAdd(&S.fz[gp + i], fz);
+        }
+    });
+}
+
+// the forces' other end
+static __device__ __forceinline__ void pairs_force_2(const SmemEmt<double> &S, const Species<double> &A) {
+    const int M = A.M, K = M / 2;
+    for_runs(A.G, M, A.C, K, [&](int g, int j, int k0, int k1) {
+        double fx = 0.0, fy = 0.0, fz = 0.0;
+        if (2 * K == M && k1 == K && j < K) k1 = K - 1;
+#pragma unroll 2
+        for (int kk = k0; kk < k1; ++kk) {
+            int m = j - kk - 1;
+            if (m < 0) m += M;
+            const double2 *p = reinterpret_cast<const double2 *>(A.rec4 + 4 * (A.stride * g + kk * M + m));
+            const double2 a = p[0], c = p[1];
+            if (is_zero(c.y)) continue;
+            fx -= c.y * a.x;
+            fy -= c.y * a.y;
+            fz -= c.y * c.x;
+        }
+        const int i = g * A.N + A.m0 + j;
+        if (A.C == 1) {
+            S.fx[i] += fx;
+            S.fy[i] += fy;
+            S.fz[i] += fz;
+        } else {
+            atomicAdd(&S.fx[i], fx);
+            atomicAdd(&S.fy[i], fy);
+            atomicAdd(&S.fz[i], fz);
+        }
+    });
+}
+
 template <typename R>
-static __device__ void emt_bead(const Batch &B, const EmtConst &E, const SmemEmt<R> &S, int t, int b,
-                         bool do_forces, bool store = false) {
-    const int N = B.natoms[t];
-    const int64_t base = B.ba_off[t] + (int64_t)b * N;
+static __device__ void emt_beads(const Batch &B, const EmtConst &E, const SmemEmt<R> &S, int t, int b0, int G,
+                                 bool do_forces, bool store = false) {
+    const int N = B.natoms[t], GN = G * N;
+    const int64_t base = B.ba_off[t] + (int64_t)b0 * N;
     const int aoff = B.atom_off[t];
     const int tid = threadIdx.x, nt = blockDim.x;
 
@@ -427,28 +708,30 @@ static __device__ void emt_bead(const Batch &B, const EmtConst &E, const SmemEmt
         }
         __syncthreads();
     }
-    for (int p = tid; p < N; p += nt) {
-        const int64_t k = base + S.perm[p];
+    for (int p = tid; p < GN; p += nt) {
+        const int g0 = p / N * N;
+        const int64_t k = base + g0 + S.perm[p - g0];
         const double x = B.rx[k], y = B.ry[k], z = B.rz[k];
-        S.px[p] = x;
-        S.py[p] = y;
-        S.pz[p] = z;
         if constexpr (sizeof(R) == 4) {
-            S.xh[p] = (float)x;
-            S.yh[p] = (float)y;
-            S.zh[p] = (float)z;
-            S.xl[p] = (float)(x - (double)S.xh[p]);
-            S.yl[p] = (float)(y - (double)S.yh[p]);
-            S.zl[p] = (float)(z - (double)S.zh[p]);
+            const float xh = f32_of(x), yh = f32_of(y), zh = f32_of(z);
+            S.ph[p] = make_float4(xh, yh, zh, 0.f);
+            S.pl[p] = make_float4(f32_of(x - f64_of(xh)), f32_of(y - f64_of(yh)), f32_of(z - f64_of(zh)), 0.f);
+        } else {
+            S.px[p] = x;
+            S.py[p] = y;
+            S.pz[p] = z;
         }
         S.sig[p] = R(0);
         S.A[p] = R(0);
         S.fx[p] = R(0);
         S.fy[p] = R(0);
         S.fz[p] = R(0);
+        if (G > 1) S.en[p] = 0.0;
     }
     if (tid < 32) {
-        const int c0 = pair_chunks(S.seg[1], nt), c1 = pair_chunks(S.seg[2] - S.seg[1], nt);
+        const int m0 = S.seg[1], m1 = S.seg[2] - m0;
+        const int c0 = pair_chunks(m0, sizeof(R) == 8 ? m0 / 2 : m0, G, nt),
+                  c1 = pair_chunks(m1, sizeof(R) == 8 ? m1 / 2 : m1, G, nt);
         if (tid == 0) {
             S.seg[4] = c0;
             S.seg[5] = c1;
@@ -456,136 +739,98 @@ static __device__ void emt_bead(const Batch &B, const EmtConst &E, const SmemEmt
     }
     __syncthreads();
     const int n0 = S.seg[1], n1 = S.seg[2] - S.seg[1];
-    const int chunks[2] = {S.seg[4], S.seg[5]};
 
     const int NK = N * (N / 2);
-    R *scr = (R *)B.pair_scratch + 6 * (B.pair_off[t] + (int64_t)b * NK);
-    R *s_dx = scr, *s_dy = scr + NK, *s_dz = scr + 2 * NK, *s_q = scr + 3 * NK, *s_fv = scr + 4 * NK,
-      *s_rho = scr + 5 * NK;
-    const R cut2 = (R)E.cut2;
-    EnergySum<R> e_pair;
+    R *const rec4 = (R *)B.pair_scratch + 6 * (B.pair_off[t] + (int64_t)b0 * NK), *const rec2 = rec4 + 4 * (int64_t)G * NK;
+    const EmtPairs<R> &Q = emt_pairs(E, R(0));
+    const R cut2 = Q.cut2;
+    PlaceDiff<R> D(B, S, base);
+    EnergySum<R> e_pair;  // one bead: this thread's pair energies
+    // calls f(constants, places) for each species that has pairs
+    auto each_species = [&](auto f) {
+        for (int s = 0, off = 0; s < E.nspecies; ++s) {
+            const int m0 = S.seg[s], M = S.seg[s + 1] - m0;
+            if (M < 2) continue;
+            const PairK<R> k{Q.acut, Q.rcut, Q.eta[s], Q.etaq[s], Q.b[s], Q.kb[s], Q.g[s], Q.c[s]};
+            const Species<R> A{N, G, m0, M, S.seg[4 + s], rec4 + 4 * off, rec2 + 2 * off, NK, cut2};
+            f(k, A);
+            off += M * (M - 1) / 2;
+        }
+    };
 
     // ---- pass 1, pairs of one species -------------------------------------------------
-    for (int s = 0, off = 0; s < E.nspecies; ++s) {
-        const int m0 = S.seg[s], M = S.seg[s + 1] - m0, K = M / 2;
-        if (K == 0) continue;
-        // QUIRK kept from pes_emt_mod.f90:705: the type1-type1 density derivative uses eta2 of
-        // type2.
-        const PairK<R> k{(R)E.acut,    (R)E.rcut,          (R)E.eta2[s],    (R)E.eta2[E.hh_quirk && s == 0 ? 1 : s],
-                         (R)E.betas0[s], (R)E.kappadbeta[s], (R)E.igamma1[s], (R)E.g2v0[s]};
-        const int C = chunks[s], per = (K + C - 1) / C;
-        for (int w = tid; w < M * C; w += nt) {
-            const int c = w / M, i = w - c * M;
-            const int k1 = min((c + 1) * per, (2 * K == M && i >= K) ? K - 1 : K);
-            R acc = R(0);
-            for (int kk = 1 + c * per; kk <= k1; ++kk) {
-                int j = i + kk;
-                if (j >= M) j -= M;
-                const int p = off + (kk - 1) * M + i;
-                R q = R(0), fv = R(0), rho = R(0), rx, ry, rz;
-                place_diff<R>(S, m0 + i, m0 + j, rx, ry, rz);
-                const R r2 = rx * rx + ry * ry + rz * rz;
-                if (!beyond(r2, cut2)) {
-                    const R ir = Math<R>::rsq(r2), r = r2 * ir;
-                    R theta, rt1;
-                    emt_theta<R>(k.acut, k.rcut, r, theta, rt1);
-                    const R phi = theta * Math<R>::ex(-k.eta * (r - k.b));
-                    const R psi = theta * Math<R>::ex(-k.kb * (r - k.b));
-                    rho = k.g * phi;
-                    acc += rho;
-                    e_pair.add(-(k.c * psi));
-                    q = k.g * (k.etaq + rt1) * phi * ir;
-                    fv = -(k.c * (k.kb + rt1) * psi * ir);
-                }
-                s_rho[p] = rho;
-                if (do_forces) {
-                    s_dx[p] = rx;
-                    s_dy[p] = ry;
-                    s_dz[p] = rz;
-                    s_q[p] = q;
-                    s_fv[p] = fv;
-                }
-            }
-            if (C == 1) S.sig[m0 + i] = acc;
-            else atomicAdd(&S.sig[m0 + i], acc);
-        }
-        off += M * (M - 1) / 2;
-    }
+    each_species([&](const PairK<R> &k, const Species<R> &A) { pairs_density(S, D, k, A, do_forces, e_pair); });
     // ---- pass 1, pairs of the two species: a warp's lanes over the slot-1 atoms ----------
     const int t0 = E.type_of_slot[0], t1 = E.type_of_slot[1];
     const int xoff = n0 * (n0 - 1) / 2 + n1 * (n1 - 1) / 2;  // cross pairs follow in the scratch
+    const bool cross = n0 > 0 && n1 > 0;
     __syncthreads();
-    for (int a = 0; a < n0 && n1 > 0; ++a) {
-        const int ia = S.perm[a];
-        R sa = R(0);
-        for (int jj = tid; jj < n1; jj += nt) {
-            const int j = n0 + jj, p = xoff + a * n1 + jj;
-            R q_a = R(0), q_j = R(0), fv = R(0), rx = R(0), ry = R(0), rz = R(0);
-            // pes(ti, tj) of the pair's first atom in the (i, i+k mod N) order, should the table not
-            // be symmetric
-            const int d = S.perm[j] - ia, dk = d > 0 ? d : d + N;
-            const bool a_first = 2 * dk < N || (2 * dk == N && ia < S.perm[j]);
-            if ((E.pair_mask >> (a_first ? t0 * kMaxTypes + t1 : t1 * kMaxTypes + t0)) & 1u) {
-                place_diff<R>(S, a, j, rx, ry, rz);
-                const R r2 = rx * rx + ry * ry + rz * rz;
-                if (!beyond(r2, cut2)) {
-                    const R ir = Math<R>::rsq(r2), r = r2 * ir;
-                    R theta, rt1;
-                    emt_theta<R>((R)E.acut, (R)E.rcut, r, theta, rt1);
-                    const R phi_j = theta * Math<R>::ex(-(R)E.eta2[1] * (r - (R)E.betas0[1]));
-                    const R psi_j = theta * Math<R>::ex(-(R)E.kappadbeta[1] * (r - (R)E.betas0[1]));
-                    const R phi_a = theta * Math<R>::ex(-(R)E.eta2[0] * (r - (R)E.betas0[0]));
-                    const R psi_a = theta * Math<R>::ex(-(R)E.kappadbeta[0] * (r - (R)E.betas0[0]));
-                    const R gaj = (R)(E.igamma1[0] * E.chi[0][1]), gja = (R)(E.igamma1[1] * E.chi[1][0]);
-                    const R caj = (R)(E.g2v0[0] * E.chi[0][1]), cja = (R)(E.g2v0[1] * E.chi[1][0]);
-                    sa += gaj * phi_j;
-                    S.sig[j] += gja * phi_a;  // this thread alone owns j here
-                    e_pair.add(-R(0.5) * (caj * psi_j + cja * psi_a));
-                    fv = -R(0.5) * (caj * ((R)E.kappadbeta[1] + rt1) * psi_j +
-                                    cja * ((R)E.kappadbeta[0] + rt1) * psi_a) * ir;
-                    q_a = gaj * ((R)E.eta2[1] + rt1) * phi_j * ir;
-                    q_j = gja * ((R)E.eta2[0] + rt1) * phi_a * ir;
+    if (cross) {
+        const R acut = Q.acut, rcut = Q.rcut, eta0 = Q.eta[0], eta1 = Q.eta[1], bs0 = Q.b[0], bs1 = Q.b[1],
+                kb0 = Q.kb[0], kb1 = Q.kb[1], gaj = Q.gx[0], gja = Q.gx[1], caj = Q.cx[0], cja = Q.cx[1];
+        // work items (bead, slot-1 atom), walked in whole warps: each item meets the bead's slot-0 atoms
+        const int items = G * n1;
+        for (int w0 = tid & ~31; w0 < items; w0 += nt) {
+            const int w = w0 + (tid & 31);
+            const bool on = w < items;
+            const int g = on ? w / n1 : G - 1, jj = on ? w - g * n1 : 0;
+            const int j = g * N + n0 + jj;
+            for (int a = 0; a < n0; ++a) {
+                R sa = R(0);
+                EnergySum<R> e_run;
+                if (on) {
+                    R q_a = R(0), q_j = R(0), fv = R(0), rx = R(0), ry = R(0), rz = R(0);
+                    // pes(ti, tj) of the pair's first atom in the (i, i+k mod N) order, should the table
+                    // not be symmetric
+                    const int ia = S.perm[a], ij = S.perm[n0 + jj], d = ij - ia, dk = d > 0 ? d : d + N;
+                    const bool a_first = 2 * dk < N || (2 * dk == N && ia < ij);
+                    if ((E.pair_mask >> (a_first ? t0 * kMaxTypes + t1 : t1 * kMaxTypes + t0)) & 1u) {
+                        D.set(S, g * N + a);
+                        D.diff(S, j, N, rx, ry, rz);
+                        const R r2 = rx * rx + ry * ry + rz * rz;
+                        if (!beyond(r2, cut2)) {
+                            const R ir = Math<R>::rsq(r2), r = r2 * ir;
+                            R theta, rt1;
+                            emt_theta<R>(acut, rcut, r, theta, rt1);
+                            const R phi_j = theta * Math<R>::ex(-eta1 * (r - bs1));
+                            const R psi_j = theta * Math<R>::ex(-kb1 * (r - bs1));
+                            const R phi_a = theta * Math<R>::ex(-eta0 * (r - bs0));
+                            const R psi_a = theta * Math<R>::ex(-kb0 * (r - bs0));
+                            sa = gaj * phi_j;
+                            S.sig[j] += gja * phi_a;  // this thread alone owns j here
+                            e_run.add(-R(0.5) * (caj * psi_j + cja * psi_a));
+                            fv = -R(0.5) * (caj * (kb1 + rt1) * psi_j + cja * (kb0 + rt1) * psi_a) * ir;
+                            q_a = gaj * (eta1 + rt1) * phi_j * ir;
+                            q_j = gja * (eta0 + rt1) * phi_a * ir;
+                        }
+                    }
+                    if (do_forces) {
+                        const int64_t slot = (int64_t)NK * g + xoff + a * n1 + jj;
+                        R *const p = rec4 + 4 * slot, *const p2 = rec2 + 2 * slot;
+                        p[0] = rx;
+                        p[1] = ry;
+                        p[2] = rz;
+                        p[3] = q_a;
+                        p2[0] = fv;
+                        p2[1] = q_j;
+                    }
+                    if (G == 1) e_pair.join(e_run);
+                    else S.en[j] += e_run.value();  // this thread alone owns j here
                 }
-            }
-            if (do_forces) {
-                s_dx[p] = rx;
-                s_dy[p] = ry;
-                s_dz[p] = rz;
-                s_q[p] = q_a;
-                s_fv[p] = fv;
-                s_rho[p] = q_j;
+                warp_add<R>(S.sig, g * N + a, sa);
             }
         }
-        for (int o = 16; o > 0; o >>= 1) sa += __shfl_xor_sync(0xffffffffu, sa, o);
-        if ((tid & 31) == 0 && !is_zero(sa)) atomicAdd(&S.sig[a], sa);
     }
     __syncthreads();
-    // ---- densities, the other side of each pair ----------------------------------------
-    for (int s = 0, off = 0; s < E.nspecies; ++s) {
-        const int m0 = S.seg[s], M = S.seg[s + 1] - m0, K = M / 2;
-        if (K == 0) continue;
-        const int C = chunks[s], per = (K + C - 1) / C;
-        for (int w = tid; w < M * C; w += nt) {
-            const int c = w / M, j = w - c * M;
-            const int k1 = min((c + 1) * per, K);
-            R acc = R(0);
-            for (int kk = 1 + c * per; kk <= k1; ++kk) {
-                int m = j - kk;
-                if (m < 0) m += M;
-                if (2 * kk == M && m >= K) continue;
-                const R rho = s_rho[off + (kk - 1) * M + m];
-                if (!is_zero(rho)) acc += rho;
-            }
-            atomicAdd(&S.sig[m0 + j], acc);
-        }
-        off += M * (M - 1) / 2;
-    }
+    each_species([&](const PairK<R> &, const Species<R> &A) { pairs_density_2(S, A); });
     __syncthreads();
 
     // ---- per-atom epilogue ---------------------------------------------------
     double e_atom = 0.0;
-    for (int i = tid; i < n0 + n1; i += nt) {
-        const int s = i >= n0;
+    const int ne = n0 + n1;
+    for (int w = tid; w < G * ne; w += nt) {
+        const int g = w / ne, p = w - g * ne, i = g * N + p;
+        const int s = p >= n0;
         double sc = (double)S.sig[i], cl = sc;
         // above 1e-9 (by its high word) neither floor of pes_emt_mod.f90:793 acts
         if (__double2hiint(sc) <= 0x3e112e0b || __double2hiint(sc) >= 0x7ff00000) {
@@ -594,112 +839,75 @@ static __device__ void emt_bead(const Batch &B, const EmtConst &E, const SmemEmt
         }
         const double be = E.betaeta2[s], sa = div_by(-log(cl * kTwelfth), be, E.ibe[s]);
         const double lsa = E.lambda[s] * sa, el = exp_t64(-lsa), ek = exp_t64(-E.kappa[s] * sa);
-        e_atom += E.e0[s] * (fma(lsa, el, el) - 1.0) + E.v6[s] * ek;
+        const double e = E.e0[s] * (fma(lsa, el, el) - 1.0) + E.v6[s] * ek;
         const double bs = be * sc;
         S.A[i] = (R)div_by(E.e0l2[s] * sa * el + E.v6k[s] * ek, bs, rcp_nr(bs));
-        B.dens[base + S.perm[i]] = E.n0[s] * exp_t64(E.dens_exp[s] * sa);
+        B.dens[base + g * N + S.perm[p]] = E.n0[s] * exp_t64(E.dens_exp[s] * sa);
+        if (G == 1) e_atom += e;
+        else S.en[i] += e;
     }
-    const double etot = block_sum(e_pair.value() + e_atom, S.red);  // contains __syncthreads
-    if (tid == 0) B.epot[B.bead_off[t] + b] += etot;
-    if (!do_forces) return;
+    __syncthreads();
 
     // ---- pass 2 ----------------------------------------------------------------------
-    for (int s = 0, off = 0; s < E.nspecies; ++s) {  // the first atom's side
-        const int m0 = S.seg[s], M = S.seg[s + 1] - m0, K = M / 2;
-        if (K == 0) continue;
-        const int C = chunks[s], per = (K + C - 1) / C;
-        for (int w = tid; w < M * C; w += nt) {
-            const int c = w / M, i = w - c * M;
-            const int k1 = min((c + 1) * per, (2 * K == M && i >= K) ? K - 1 : K);
-            const R Ai = S.A[m0 + i];
-            R fx = R(0), fy = R(0), fz = R(0);
-            for (int kk = 1 + c * per; kk <= k1; ++kk) {
-                int j = i + kk;
-                if (j >= M) j -= M;
-                const int p = off + (kk - 1) * M + i;
-                const R q = s_q[p], fv = s_fv[p];
-                if (is_zero(q) && is_zero(fv)) continue;  // beyond the cutoff: q's slot holds the 0
-                const R cc = Ai * q + S.A[m0 + j] * q + fv;
-                s_q[p] = cc;
-                fx += cc * s_dx[p];
-                fy += cc * s_dy[p];
-                fz += cc * s_dz[p];
-            }
-            if (C == 1) {
-                S.fx[m0 + i] = fx;
-                S.fy[m0 + i] = fy;
-                S.fz[m0 + i] = fz;
-            } else {
-                atomicAdd(&S.fx[m0 + i], fx);
-                atomicAdd(&S.fy[m0 + i], fy);
-                atomicAdd(&S.fz[m0 + i], fz);
-            }
+    if (do_forces || sizeof(R) == 4)
+        each_species([&](const PairK<R> &k, const Species<R> &A) { pairs_force(S, D, k, A, do_forces, e_pair); });
+    if (G == 1) {
+        const double etot = block_sum(e_pair.value() + e_atom, S.red);  // contains __syncthreads
+        if (tid == 0) B.epot[B.bead_off[t] + b0] += etot;
+    } else {
+        __syncthreads();
+        for (int g = tid >> 5; g < G; g += nt >> 5) {  // a warp per bead
+            double e = 0.0;
+            for (int i = tid & 31; i < ne; i += 32) e += S.en[g * N + i];
+            for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+            if ((tid & 31) == 0) B.epot[B.bead_off[t] + b0 + g] += e;
         }
-        off += M * (M - 1) / 2;
     }
-    __syncthreads();
-    for (int a = 0; a < n0 && n1 > 0; ++a) {  // pairs of the two species
-        const R Aa = S.A[a];
-        R fx = R(0), fy = R(0), fz = R(0);
-        for (int jj = tid; jj < n1; jj += nt) {
-            const int j = n0 + jj, p = xoff + a * n1 + jj;
-            const R cc = Aa * s_q[p] + S.A[j] * s_rho[p] + s_fv[p];
-            const R gx = cc * s_dx[p], gy = cc * s_dy[p], gz = cc * s_dz[p];
-            fx += gx;
-            fy += gy;
-            fz += gz;
-            S.fx[j] -= gx;  // this thread alone owns j here
-            S.fy[j] -= gy;
-            S.fz[j] -= gz;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            fx += __shfl_xor_sync(0xffffffffu, fx, o);
-            fy += __shfl_xor_sync(0xffffffffu, fy, o);
-            fz += __shfl_xor_sync(0xffffffffu, fz, o);
-        }
-        if ((tid & 31) == 0) {
-            atomicAdd(&S.fx[a], fx);
-            atomicAdd(&S.fy[a], fy);
-            atomicAdd(&S.fz[a], fz);
+    if (!do_forces) {
+        __syncthreads();
+        return;
+    }
+    if (cross) {  // pairs of the two species
+        const int items = G * n1;
+        for (int w0 = tid & ~31; w0 < items; w0 += nt) {
+            const int w = w0 + (tid & 31);
+            const bool on = w < items;
+            const int g = on ? w / n1 : G - 1, jj = on ? w - g * n1 : 0;
+            const int j = g * N + n0 + jj;
+            for (int a = 0; a < n0; ++a) {
+                R gx = R(0), gy = R(0), gz = R(0);
+                if (on) {
+                    const int64_t slot = (int64_t)NK * g + xoff + a * n1 + jj;
+                    const R *const p = rec4 + 4 * slot, *const p2 = rec2 + 2 * slot;
+                    const R cc = S.A[g * N + a] * p[3] + S.A[j] * p2[1] + p2[0];
+                    gx = cc * p[0];
+                    gy = cc * p[1];
+                    gz = cc * p[2];
+                    S.fx[j] -= gx;  // this thread alone owns j here
+                    S.fy[j] -= gy;
+                    S.fz[j] -= gz;
+                }
+                warp_add<R>(S.fx, g * N + a, gx);
+                warp_add<R>(S.fy, g * N + a, gy);
+                warp_add<R>(S.fz, g * N + a, gz);
+            }
         }
     }
     __syncthreads();
-    for (int s = 0, off = 0; s < E.nspecies; ++s) {  // the second atom's side
-        const int m0 = S.seg[s], M = S.seg[s + 1] - m0, K = M / 2;
-        if (K == 0) continue;
-        const int C = chunks[s], per = (K + C - 1) / C;
-        for (int w = tid; w < M * C; w += nt) {
-            const int c = w / M, j = w - c * M;
-            const int k1 = min((c + 1) * per, K);
-            R fx = R(0), fy = R(0), fz = R(0);
-            for (int kk = 1 + c * per; kk <= k1; ++kk) {
-                int m = j - kk;
-                if (m < 0) m += M;
-                if (2 * kk == M && m >= K) continue;
-                const int p = off + (kk - 1) * M + m;
-                const R cc = s_q[p];
-                if (is_zero(cc)) continue;
-                fx -= cc * s_dx[p];
-                fy -= cc * s_dy[p];
-                fz -= cc * s_dz[p];
-            }
-            atomicAdd(&S.fx[m0 + j], fx);
-            atomicAdd(&S.fy[m0 + j], fy);
-            atomicAdd(&S.fz[m0 + j], fz);
-        }
-        off += M * (M - 1) / 2;
-    }
+    each_species([&](const PairK<R> &, const Species<R> &A) { pairs_force_2(S, A); });
     __syncthreads();
-    for (int p = tid; p < N; p += nt) {
-        const int64_t k = base + S.perm[p];
+    for (int p = tid; p < GN; p += nt) {
+        const int g0 = p / N * N;
+        const int64_t k = base + g0 + S.perm[p - g0];
+        const double fx = wide(S.fx[p]), fy = wide(S.fy[p]), fz = wide(S.fz[p]);
         if (store) {
-            B.fx[k] = (double)S.fx[p];
-            B.fy[k] = (double)S.fy[p];
-            B.fz[k] = (double)S.fz[p];
+            B.fx[k] = fx;
+            B.fy[k] = fy;
+            B.fz[k] = fz;
         } else {
-            B.fx[k] += (double)S.fx[p];
-            B.fy[k] += (double)S.fy[p];
-            B.fz[k] += (double)S.fz[p];
+            B.fx[k] += fx;
+            B.fy[k] += fy;
+            B.fz[k] += fz;
         }
     }
     __syncthreads();

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "mdt_common.cuh"
+#include "mdt_exp2tab.cuh"
 
 namespace mdt {
 
@@ -109,6 +110,55 @@ static __device__ __forceinline__ double f64_of(float f) {
 // exponent of the largest magnitudes: infinity or NaN (a FP64 comparison runs on the FP64 pipe)
 static __device__ __forceinline__ bool not_finite(double x) {
     return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000;
+}
+
+// ---- FP64 building blocks ------------------------------------------------------------
+static __device__ __forceinline__ double rcp_nr(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);  // 1/x = y (1 + e + e^2 + ...)
+    return fma(y, fma(e, e, e), y);
+}
+
+static __device__ __forceinline__ double rsqrt_nr(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);  // 1/sqrt(x) = y (1 + e/2 + 3 e^2/8 + ...)
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// n/d from the reciprocal id of d (within an ulp or two): the residual's correction makes the
+// quotient round as a division does, in 3 FP64 instructions instead of about 10
+static __device__ __forceinline__ double div_by(double n, double d, double id) {
+    const double q = n * id;
+    return fma(fma(-q, d, n), id, q);
+}
+
+// Rare paths of the pair loops are calls: inlined, the compiler predicates their FP64 instructions
+// and every pair issues them.
+static __device__ __noinline__ double exp_far(double x) { return exp(x); }
+
+// FP64 exp by the table-driven method of Tang (ACM TOMS 15(2), 1989): x = (512 n_hi + j)
+// ln2/512 + r with |r| <= ln2/1024, exp(x) = 2^n_hi 2^(j/512) (1 + p(r)), p the Taylor series
+// of exp(r) - 1 to r^4 (truncation below 2^-59).  ln2/512 enters in two parts (its double,
+// then the remainder) so that r is exact to ~2^-100, and n = round(512 x / ln2) comes from
+// adding 1.5 * 2^52.  10 FP64 instructions (13 with 64 entries and r^5, ~19 for exp()); the
+// range test reads the high word, because a FP64 comparison costs as much as an addition.
+// Outside [-700, 700], and for NaN, exp() itself.
+static __device__ __forceinline__ double exp_t64(double x) {
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x4085e000) return exp_far(x);  // |x| >= 700
+    const double shifter = 6755399441055744.0;
+    const double t = fma(x, 738.65986093514926, shifter);
+    const int n = __double2loint(t);
+    const double nd = t - shifter;
+    double r = fma(-nd, 0x1.62e42fefa39efp-10, x);
+    r = fma(-nd, 0x1.abc9e3b39803fp-65, r);
+    double q = fma(r, 1.0 / 24.0, 1.0 / 6.0);
+    q = fma(r, q, 0.5);
+    const double pr = fma(r * r, q, r);
+    const double tj = __ldg(kExp2Tab + (n & 511));
+    const double y = fma(tj, pr, tj);
+    return __hiloint2double(__double2hiint(y) + (n >> 9) * (1 << 20), __double2loint(y));
 }
 
 }  // namespace mdt

@@ -14,6 +14,8 @@ struct LaunchCfg {
     int grid;
     const int *order;  // trajectory work order (largest first)
     int *counter;      // device work-queue counter (reset by the launcher)
+    int parts = 1;     // generic HDNNP force calls: CTAs per trajectory (single beads)
+    int64_t total_ba = 0;
 };
 
 cudaError_t launch_phase(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P, int phase,

@@ -40,7 +40,8 @@ __device__ void calc_force(const Batch &B, const EmtConst &E, const PropParams &
     for (int b = threadIdx.x; b < T.nb; b += blockDim.x) B.epot[B.bead_off[T.t] + b] = 0.0;
     __syncthreads();
     if (T.nb > 1) ring_polymer_step(B, P, T, S.cjk);
-    for (int b = 0; b < T.nb; ++b) emt_bead<R>(B, E, S, T.t, b, do_forces, single);
+    const int G = min(T.nb, S.places / T.N);
+    for (int b = 0; b < T.nb; b += G) emt_beads<R>(B, E, S, T.t, b, min(G, T.nb - b), do_forces, single);
     if (do_forces) set_acceleration(B, T);
     __syncthreads();
 }
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(kBlock, 4) phase_kernel(Batch B, EmtConst E, P
                                                     int *counter, int phase) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
-    SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads);
+    SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads, emt_places(B.max_atoms, B.max_beads));
     for (;;) {
         const int w = next_work(counter, &work_slot);
         if (w >= B.ntraj) break;
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(kBlock, 4) md_steps_kernel(Batch B, EmtConst E
                                                        int *counter, int nsteps) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
-    SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads);
+    SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads, emt_places(B.max_atoms, B.max_beads));
     for (;;) {
         const int w = next_work(counter, &work_slot);
         if (w >= B.ntraj) break;
@@ -404,7 +405,7 @@ cudaError_t launch_summary(cudaStream_t s, const Batch &B, const PropParams &P, 
 template <typename R>
 static cudaError_t launch_phase_t(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P,
                                   int phase) {
-    const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R));
+    const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R), emt_places(B.max_atoms, B.max_beads));
     cudaError_t e = cudaFuncSetAttribute(phase_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
@@ -421,7 +422,7 @@ cudaError_t launch_phase(const LaunchCfg &c, const Batch &B, const EmtConst &E, 
 template <typename R>
 static cudaError_t launch_md_t(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P,
                                int nsteps) {
-    const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R));
+    const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R), emt_places(B.max_atoms, B.max_beads));
     cudaError_t e = cudaFuncSetAttribute(md_steps_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
@@ -464,7 +465,7 @@ cudaError_t launch_pack_scalar(cudaStream_t s, const Batch &B, double *dst, cons
 }
 
 int max_resident_ctas(int max_atoms, int max_beads, int precision) {
-    const size_t sm = smem_bytes(max_atoms, max_beads, precision == 1 ? 4 : 8);
+    const size_t sm = smem_bytes(max_atoms, max_beads, precision == 1 ? 4 : 8, emt_places(max_atoms, max_beads));
     int n = 0;
     if (precision == 1) {
         cudaFuncSetAttribute(md_steps_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -1,5 +1,6 @@
 // mdt_nn.cu -- HDNNP (RuNNer-style) force evaluation and the NN-surrogate MD step.
 // See mdt_nn.cuh for the per-warp descriptor/network design.
+#include <algorithm>
 #include <cstdio>
 
 #include "mdt_common.cuh"
@@ -79,11 +80,12 @@ __device__ SmemNN<R> carve_nn(unsigned char *base, const NNDev &M, int max_atoms
 // ---------------------------------------------------------------------------
 // One bead: wrapped positions, neighbour lists, descriptors, network, forces.
 // Adds eV and eV/A into B.epot / B.f*.  Returns (in S.flag) whether a descriptor left
-// the scaling range widened by M.margin.
+// the scaling range widened by M.margin.  `part` of `parts`: the CTA's share of the bead's central
+// atoms, groups of kNNWarps dealt in turn; with several parts the sums meet in global memory.
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ bool nn_bead(const Batch &B, const NNDev &M, const NNScratch &X, const SmemNN<R> &S, int t, int b,
-                        bool do_forces, bool skip_if_flagged) {
+                        bool do_forces, bool skip_if_flagged, int part = 0, int parts = 1) {
     const int N = B.natoms[t];
     const int64_t base = B.ba_off[t] + (int64_t)b * N;
     const int aoff = B.atom_off[t];
@@ -105,7 +107,9 @@ __device__ bool nn_bead(const Batch &B, const NNDev &M, const NNScratch &X, cons
     __syncthreads();
     // ---- neighbour lists ----------------------------------------------------------
     const int na = X.img[3 * t], nbi = X.img[3 * t + 1], nc = X.img[3 * t + 2];
-    for (int i = tid; i < N; i += nt) {
+    for (int q = tid; q < N; q += nt) {
+        const int i = parts == 1 ? q : (q / kNNWarps * parts + part) * kNNWarps + q % kNNWarps;
+        if (i >= N) continue;
         int cnt = acsf_neighbors_one(M, i, N, S.px, S.py, S.pz, S.lat, na, nbi, nc,
                                      X.nbw + (base + i) * (int64_t)M.maxnb);
         if (cnt > M.maxnb) {
@@ -125,7 +129,7 @@ __device__ bool nn_bead(const Batch &B, const NNDev &M, const NNScratch &X, cons
     R *hv = S.hv + warp * (kMaxLayers + 1) * kMaxNodes;
     double e_warp = 0.0;
 
-    for (int i = warp; i < N; i += kNNWarps) {
+    for (int i = part * kNNWarps + warp; i < N; i += parts * kNNWarps) {
         const int ei = S.elem[i];
         if (ei < 0) continue;
         const int cnt = X.nbcnt[base + i];
@@ -231,9 +235,19 @@ __device__ bool nn_bead(const Batch &B, const NNDev &M, const NNScratch &X, cons
         __syncthreads();
         return true;
     }
+    const double c = kHa2eV * kAng2BohrD;
+    if (parts > 1) {
+        if (tid == 0) atomicAdd(&B.epot[B.bead_off[t] + b], etot * kHa2eV);
+        for (int i = tid; do_forces && i < N; i += nt) {
+            if (S.fx[i] != R(0)) atomicAdd(&B.fx[base + i], (double)S.fx[i] * c);
+            if (S.fy[i] != R(0)) atomicAdd(&B.fy[base + i], (double)S.fy[i] * c);
+            if (S.fz[i] != R(0)) atomicAdd(&B.fz[base + i], (double)S.fz[i] * c);
+        }
+        __syncthreads();
+        return flagged;
+    }
     if (tid == 0) B.epot[B.bead_off[t] + b] += etot * kHa2eV;
     if (do_forces) {
-        const double c = kHa2eV * kAng2BohrD;
         for (int i = tid; i < N; i += nt) {
             B.fx[base + i] += (double)S.fx[i] * c;
             B.fy[base + i] += (double)S.fy[i] * c;
@@ -270,27 +284,31 @@ __device__ void nn_calc_force(const Batch &B, const NNDev &M, const EmtConst &E,
     for (int b = 0; b < T.nb; ++b) {
         const bool flagged = nn_bead<R>(B, M, X, S, T.t, b, do_forces, SURR);
         if (SURR && flagged) {
-            emt_bead<double>(B, E, SE, T.t, b, do_forces);
+            emt_beads<double>(B, E, SE, T.t, b, 1, do_forces);
             if (threadIdx.x == 0) X.fallback[T.t] += 1;
         }
     }
-    if (do_forces) {
-        for (int s = threadIdx.x; s < tot; s += blockDim.x) {
-            const int64_t k = T.base + s;
-            const int i = s % T.N;
-            const double m = B.mass[T.aoff + i];
-            const uint8_t fx = B.fixed[k];
-            if (!(fx & 1)) B.ax[k] = B.fx[k] / m;
-            if (!(fx & 2)) B.ay[k] = B.fy[k] / m;
-            if (!(fx & 4)) B.az[k] = B.fz[k] / m;
-        }
-    }
+    if (do_forces) set_acceleration(B, T);
     __syncthreads();
 }
 
 struct NNLaunch {
     int max_atoms, ngeta;
+    int parts;  // CTAs per trajectory
 };
+
+// before and after a force call whose trajectories are split over several CTAs (single beads)
+__global__ void nn_zero_kernel(Batch B, int64_t total) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
+        B.fx[k] = 0.0; B.fy[k] = 0.0; B.fz[k] = 0.0;
+        B.ax[k] = 0.0; B.ay[k] = 0.0; B.az[k] = 0.0;
+        if (k < B.ntraj) B.epot[B.bead_off[k]] = 0.0;
+    }
+}
+
+__global__ void nn_accel_kernel(Batch B) {
+    for (int t = blockIdx.x; t < B.ntraj; t += gridDim.x) set_acceleration(B, traj_view(B, t));
+}
 
 template <typename R, bool SURR>
 __global__ void __launch_bounds__(kNNBlock) nn_force_kernel(Batch B, NNDev M, EmtConst E, NNScratch X, PropParams P,
@@ -300,15 +318,19 @@ __global__ void __launch_bounds__(kNNBlock) nn_force_kernel(Batch B, NNDev M, Em
     SmemNN<R> S = carve_nn<R>(smem_raw, M, LN.max_atoms, LN.ngeta);
     SmemEmt<double> SE = carve_smem<double>(smem_raw + nn_smem_bytes(LN.max_atoms, M.maxnb, LN.ngeta, M.nelem,
                                                                      M.maxweights, sizeof(R)),
-                                            B.max_atoms, B.max_beads);
+                                            B.max_atoms, B.max_beads, B.max_atoms);
     load_weights_nn(M, S.w);
     for (;;) {
         if (threadIdx.x == 0) work_slot = atomicAdd(counter, 1);
         __syncthreads();
         const int w = work_slot;
         __syncthreads();
-        if (w >= B.ntraj) break;
-        const int t = order[w];
+        if (w >= B.ntraj * LN.parts) break;
+        const int t = order[w / LN.parts];
+        if (LN.parts > 1) {
+            nn_bead<R>(B, M, X, S, t, 0, do_forces != 0, false, w % LN.parts, LN.parts);
+            continue;
+        }
         const TrajView T = traj_view(B, t);
         load_cjk(B, t, SE.cjk);
         nn_calc_force<R, SURR>(B, M, E, X, P, S, SE, T, do_forces != 0);
@@ -324,7 +346,7 @@ __global__ void __launch_bounds__(kNNBlock) nn_md_steps_kernel(Batch B, NNDev M,
     SmemNN<R> S = carve_nn<R>(smem_raw, M, LN.max_atoms, LN.ngeta);
     SmemEmt<double> SE = carve_smem<double>(smem_raw + nn_smem_bytes(LN.max_atoms, M.maxnb, LN.ngeta, M.nelem,
                                                                      M.maxweights, sizeof(R)),
-                                            B.max_atoms, B.max_beads);
+                                            B.max_atoms, B.max_beads, B.max_atoms);
     load_weights_nn(M, S.w);
     for (;;) {
         if (threadIdx.x == 0) work_slot = atomicAdd(counter, 1);
@@ -354,21 +376,26 @@ __global__ void __launch_bounds__(kNNBlock) nn_md_steps_kernel(Batch B, NNDev M,
 
 size_t nn_total_smem(const NNDev &M, int max_atoms, int max_beads, int ngeta, int precision) {
     const size_t rs = precision == 1 ? 4 : 8;
-    return nn_smem_bytes(max_atoms, M.maxnb, ngeta, M.nelem, M.maxweights, rs) + smem_bytes(max_atoms, max_beads, 8);
+    return nn_smem_bytes(max_atoms, M.maxnb, ngeta, M.nelem, M.maxweights, rs) + smem_bytes(max_atoms, max_beads, 8, max_atoms);
 }
 
 template <typename R, bool SURR>
 static cudaError_t nn_launch_t(const LaunchCfg &c, const Batch &B, const NNDev &M, const EmtConst &E,
                                const NNScratch &X, const PropParams &P, int ngeta, int nsteps, int mode) {
     const size_t sm = nn_total_smem(M, B.max_atoms, B.max_beads, ngeta, sizeof(R) == 4 ? 1 : 0);
-    NNLaunch LN{B.max_atoms, ngeta};
+    NNLaunch LN{B.max_atoms, ngeta, SURR || mode == 2 ? 1 : c.parts};
     cudaError_t e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
     if (e != cudaSuccess) return e;
+    if (LN.parts > 1) {
+        const int64_t total = c.total_ba;
+        nn_zero_kernel<<<(int)std::min<int64_t>((total + 255) / 256, 4096), 256, 0, c.stream>>>(B, total);
+    }
     if (mode == 0 || mode == 1) {
         e = cudaFuncSetAttribute(nn_force_kernel<R, SURR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
         nn_force_kernel<R, SURR><<<c.grid, kNNBlock, sm, c.stream>>>(B, M, E, X, P, LN, c.order, c.counter,
                                                                      mode == 0 ? 1 : 0);
+        if (LN.parts > 1 && mode == 0) nn_accel_kernel<<<std::min(B.ntraj, 4096), 128, 0, c.stream>>>(B);
     } else {
         e = cudaFuncSetAttribute(nn_md_steps_kernel<R, SURR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;

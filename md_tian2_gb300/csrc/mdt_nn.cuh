@@ -18,6 +18,7 @@
 //                   same forces).
 #pragma once
 #include "mdt_common.cuh"
+#include "mdt_fastmath.cuh"
 
 namespace mdt {
 
@@ -198,8 +199,9 @@ struct NNScratch {
 // ---------------------------------------------------------------------------
 template <typename R> struct NM;
 template <> struct NM<double> {
-    static __device__ __forceinline__ double ex(double x) { return exp(x); }
+    static __device__ __forceinline__ double ex(double x) { return exp_t64(x); }
     static __device__ __forceinline__ double sq(double x) { return sqrt(x); }
+    static __device__ __forceinline__ double rc(double x) { return rcp_nr(x); }
     static __device__ __forceinline__ void sc(double x, double *s, double *c) { sincospi(x, s, c); }
     static __device__ __forceinline__ double th(double x) { return tanh(x); }
     static __device__ __forceinline__ double lg(double x) { return log(x); }
@@ -209,6 +211,7 @@ template <> struct NM<double> {
 template <> struct NM<float> {
     static __device__ __forceinline__ float ex(float x) { return __expf(x); }
     static __device__ __forceinline__ float sq(float x) { return sqrtf(x); }
+    static __device__ __forceinline__ float rc(float x) { return 1.f / x; }
     static __device__ __forceinline__ void sc(float x, float *s, float *c) { sincospif(x, s, c); }
     static __device__ __forceinline__ float th(float x) { return tanhf(x); }
     static __device__ __forceinline__ float lg(float x) { return __logf(x); }

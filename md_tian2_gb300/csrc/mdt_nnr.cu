@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
     constexpr int KT = KA + KB, bs = kRS;
     const int tid = threadIdx.x;
     const SmemR S = carve_r<KT, NH, TC>(smem_raw);
-    SmemEmt<double> SE = carve_smem<double>(S.emt, B.max_atoms, B.max_beads);
+    SmemEmt<double> SE = carve_smem<double>(S.emt, B.max_atoms, B.max_beads, B.max_atoms);
     SE.red = S.red;
     SE.cjk = S.red;  // single-bead trajectories only: the ring-polymer table is never read
     TcCtx C{0u, S.tcbar, X.tcerr};
@@ -1299,7 +1299,7 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                         if (!stat[s] || !flag[s]) continue;
                         const int t = S.tr_t[s];
                         __syncthreads();
-                        emt_bead<double>(B, E, SE, t, 0, do_forces);
+                        emt_beads<double>(B, E, SE, t, 0, 1, do_forces);
                         if (tid == 0) X.fallback[t] += 1;
                         if (A.s == s && do_forces) {
                             const int64_t k = A.base + A.i;
@@ -1418,7 +1418,7 @@ size_t nnr_smem(const RadialNN &R) { return smem_r(R.nin, R.nh, R.tc); }
 
 size_t nnr_hb_bytes(const RadialNN &R) { return hb_bytes(R.nin, R.nh, R.tc); }
 
-size_t nnr_emt_smem(int max_atoms) { return smem_bytes(max_atoms, 1, 8); }
+size_t nnr_emt_smem(int max_atoms) { return smem_bytes(max_atoms, 1, 8, max_atoms); }
 
 int nnr_resident_ctas(const RadialNN &R) {
     const size_t sm = nnr_smem(R);

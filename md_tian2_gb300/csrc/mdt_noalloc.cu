@@ -101,6 +101,22 @@ int emt_derive_constants(int32_t ntypes, const double *eta2, const double *n0, c
         E.chi[1][0] = chi_21;
         E.hh_quirk = 1;
     }
+    EmtPairs<double> &d = E.pd;
+    EmtPairs<float> &f = E.pf;
+    f.acut = (float)(d.acut = E.acut);
+    f.rcut = (float)(d.rcut = E.rcut);
+    f.cut2 = (float)(d.cut2 = E.cut2);
+    for (int s = 0; s < ns; ++s) {
+        f.eta[s] = (float)(d.eta[s] = E.eta2[s]);
+        // QUIRK kept from pes_emt_mod.f90:705: the type1-type1 density derivative uses eta2 of type2
+        f.etaq[s] = (float)(d.etaq[s] = E.eta2[E.hh_quirk && s == 0 ? 1 : s]);
+        f.b[s] = (float)(d.b[s] = E.betas0[s]);
+        f.kb[s] = (float)(d.kb[s] = E.kappadbeta[s]);
+        f.g[s] = (float)(d.g[s] = E.igamma1[s]);
+        f.c[s] = (float)(d.c[s] = E.g2v0[s]);
+        f.gx[s] = (float)(d.gx[s] = E.igamma1[s] * E.chi[s][1 - s]);
+        f.cx[s] = (float)(d.cx[s] = E.g2v0[s] * E.chi[s][1 - s]);
+    }
     return MDT_OK;
 }
 
@@ -142,7 +158,7 @@ struct CellArg {
 constexpr int kNoAllocBlock = 128;
 
 // One CTA evaluates the configuration with the same device function as the context
-// path (emt_bead), pointed at caller buffers and the file-scope scratch.
+// path (emt_beads), pointed at caller buffers and the file-scope scratch.
 __global__ void __launch_bounds__(kNoAllocBlock) emt_noalloc_kernel(int N, int ntypes, CellArg cell, EmtConst E,
                                                                      const double *x,
                                                                      const double *y, const double *z,
@@ -204,8 +220,8 @@ __global__ void __launch_bounds__(kNoAllocBlock) emt_noalloc_kernel(int N, int n
     B.pair_scratch = scratch;
     B.max_atoms = N;
     B.max_beads = 1;
-    SmemEmt<double> S = carve_smem<double>(emt_base, N, 1);
-    emt_bead<double>(B, E, S, 0, 0, true);
+    SmemEmt<double> S = carve_smem<double>(emt_base, N, 1, N);
+    emt_beads<double>(B, E, S, 0, 0, 1, true);
     if (threadIdx.x == 0 && s_bad) *energy = NAN;
 }
 
@@ -242,7 +258,7 @@ extern "C" int32_t mdt_emt_force_noalloc(int32_t natoms, const int32_t *idx, con
         }
         scratch = g_scratch_addr[dev];
     }
-    const size_t sm = ((natoms + 15) & ~15) + ((8 * (size_t)natoms + 15) & ~size_t(15)) + smem_bytes(natoms, 1, 8);
+    const size_t sm = ((natoms + 15) & ~15) + ((8 * (size_t)natoms + 15) & ~size_t(15)) + smem_bytes(natoms, 1, 8, natoms);
     emt_noalloc_kernel<<<1, kNoAllocBlock, sm, (cudaStream_t)stream>>>(natoms, ntypes, cell, E, x, y, z, idx, fx, fy, fz,
                                                                        energy, dens, scratch);
     return cudaGetLastError() == cudaSuccess ? MDT_OK : MDT_ERR_CUDA;

@@ -490,11 +490,15 @@ static __device__ void pile_tables(const Batch &B, const PropParams &P, const Tr
 
 // Normal-mode transforms with the table cjk(j, m) (column major: cjk[m nb + j - 1], beads
 // j = 1..nb, modes m = 0..nb-1).  nm_forward: y_m = sum_j x_j cjk(j, m); nm_back:
-// x_j = sum_m y_m cjk(j, m).  For an even nb >= 4 the table's symmetry halves the products:
-// cjk(nb - j, m) = cjk(j, m) for m <= nb/2 (cosines, the constant and the alternating
-// mode) and -cjk(j, m) for m > nb/2 (sines), j = 1..nb/2-1; beads nb/2 and nb pair with
-// themselves and carry no sine modes (their sine entries are zero up to the rounding of
-// the table).  The sums are the reference's matrix products in another order.
+// x_j = sum_m y_m cjk(j, m).  The table's symmetries fold the sums (the products are FP64, the
+// slowest pipe): with h = nb/2, for m <= h (cosines, the constant and the alternating mode) and
+// m > h (sines),
+//   even nb >= 4:  cjk(nb - j, m) = +-cjk(j, m), halving the products;
+//   nb = 4 q:      also cjk(j + h, m) = (-1)^m cjk(j, m), so of the four beads j, h - j, h + j,
+//                  nb - j only the first is multiplied: nb^2/4 products instead of nb^2/2
+//                  (beads q and h pair with themselves; their entries that vanish, up to the
+//                  rounding of the table, are left out).
+// The sums are the reference's matrix products in another order.
 static __device__ __forceinline__ void nm_forward(const double *cjk, int nb, const double *x, double *y) {
     if ((nb & 1) || nb < 4) {
         for (int m = 0; m < nb; ++m) {
@@ -505,21 +509,50 @@ static __device__ __forceinline__ void nm_forward(const double *cjk, int nb, con
         return;
     }
     const int h = nb / 2;
-    double sp[16], sm[16];  // x_j + x_(nb-j), x_j - x_(nb-j) at j - 1 (nb <= 32)
-    for (int j = 1; j < h; ++j) {
-        sp[j - 1] = x[j - 1] + x[nb - j - 1];
-        sm[j - 1] = x[j - 1] - x[nb - j - 1];
+    if (nb & 2) {
+        double sp[16], sm[16];  // x_j + x_(nb-j), x_j - x_(nb-j) at j - 1 (nb <= 32)
+        for (int j = 1; j < h; ++j) {
+            sp[j - 1] = x[j - 1] + x[nb - j - 1];
+            sm[j - 1] = x[j - 1] - x[nb - j - 1];
+        }
+        for (int m = 0; m <= h; ++m) {
+            const double *c = cjk + m * nb;
+            double s = c[h - 1] * x[h - 1] + c[nb - 1] * x[nb - 1];
+            for (int j = 1; j < h; ++j) s = s + c[j - 1] * sp[j - 1];
+            y[m] = s;
+        }
+        for (int m = h + 1; m < nb; ++m) {
+            const double *c = cjk + m * nb;
+            double s = 0.0;
+            for (int j = 1; j < h; ++j) s = s + c[j - 1] * sm[j - 1];
+            y[m] = s;
+        }
+        return;
     }
-    for (int m = 0; m <= h; ++m) {
-        const double *c = cjk + m * nb;
-        double s = c[h - 1] * x[h - 1] + c[nb - 1] * x[nb - 1];
-        for (int j = 1; j < h; ++j) s = s + c[j - 1] * sp[j - 1];
-        y[m] = s;
+    const int q = h / 2;
+    // combinations of the four beads of j < q: cosine and sine sums of even and of odd modes
+    double ce[8], se[8], co[8], so[8];
+    for (int j = 1; j < q; ++j) {
+        const double u = x[j - 1] + x[j + h - 1], v = x[j - 1] - x[j + h - 1];
+        const double u2 = x[h - j - 1] + x[nb - j - 1], v2 = x[h - j - 1] - x[nb - j - 1];
+        ce[j] = u + u2;
+        se[j] = u - u2;
+        co[j] = v - v2;
+        so[j] = v + v2;
     }
-    for (int m = h + 1; m < nb; ++m) {
+    const double uq = x[q - 1] + x[q + h - 1], vq = x[q - 1] - x[q + h - 1], uh = x[h - 1] + x[nb - 1],
+                 vh = x[h - 1] - x[nb - 1];
+    for (int m = 0; m < nb; ++m) {
         const double *c = cjk + m * nb;
-        double s = 0.0;
-        for (int j = 1; j < h; ++j) s = s + c[j - 1] * sm[j - 1];
+        double s;
+        if (m <= h) {
+            s = c[h - 1] * (m & 1 ? vh : uh);
+            if (!(m & 1)) s = s + c[q - 1] * uq;
+        } else {
+            s = m & 1 ? c[q - 1] * vq : 0.0;
+        }
+        const double *f = m <= h ? (m & 1 ? co : ce) : (m & 1 ? so : se);
+        for (int j = 1; j < q; ++j) s = s + c[j - 1] * f[j];
         y[m] = s;
     }
 }
@@ -534,20 +567,55 @@ static __device__ __forceinline__ void nm_back(const double *cjk, int nb, const 
         return;
     }
     const int h = nb / 2;
-    for (int j = 1; j < h; ++j) {
+    if (nb & 2) {
+        for (int j = 1; j < h; ++j) {
+            double a = 0.0, c = 0.0;
+            for (int m = 0; m <= h; ++m) a = a + y[m] * cjk[m * nb + j - 1];
+            for (int m = h + 1; m < nb; ++m) c = c + y[m] * cjk[m * nb + j - 1];
+            x[j - 1] = a + c;
+            x[nb - j - 1] = a - c;
+        }
         double a = 0.0, c = 0.0;
-        for (int m = 0; m <= h; ++m) a = a + y[m] * cjk[m * nb + j - 1];
-        for (int m = h + 1; m < nb; ++m) c = c + y[m] * cjk[m * nb + j - 1];
-        x[j - 1] = a + c;
-        x[nb - j - 1] = a - c;
+        for (int m = 0; m <= h; ++m) {
+            a = a + y[m] * cjk[m * nb + h - 1];
+            c = c + y[m] * cjk[m * nb + nb - 1];
+        }
+        x[h - 1] = a;
+        x[nb - 1] = c;
+        return;
     }
-    double a = 0.0, c = 0.0;
-    for (int m = 0; m <= h; ++m) {
-        a = a + y[m] * cjk[m * nb + h - 1];
-        c = c + y[m] * cjk[m * nb + nb - 1];
+    const int q = h / 2;
+    for (int j = 1; j <= q; ++j) {
+        const double *c = cjk + j - 1;
+        double ce = 0.0, co = 0.0, se = 0.0, so = 0.0;  // even and odd cosine modes, even and odd sine modes
+        for (int m = 0; m <= h; m += 2) ce = ce + y[m] * c[m * nb];
+        for (int m = h + 1; m < nb; m += 2) so = so + y[m] * c[m * nb];
+        if (j < q) {
+            for (int m = 1; m < h; m += 2) co = co + y[m] * c[m * nb];
+            for (int m = h + 2; m < nb; m += 2) se = se + y[m] * c[m * nb];
+            const double a = ce + co, e = se + so, a2 = ce - co, e2 = se - so;
+            x[j - 1] = a + e;
+            x[nb - j - 1] = a - e;
+            x[h + j - 1] = a2 + e2;
+            x[h - j - 1] = a2 - e2;
+        } else {
+            x[q - 1] = ce + so;
+            x[q + h - 1] = ce - so;
+        }
     }
-    x[h - 1] = a;
-    x[nb - 1] = c;
+    double ce = 0.0, co = 0.0;
+    for (int m = 0; m <= h; m += 2) ce = ce + y[m] * cjk[m * nb + h - 1];
+    for (int m = 1; m < h; m += 2) co = co + y[m] * cjk[m * nb + h - 1];
+    x[h - 1] = ce + co;
+    x[nb - 1] = ce - co;
+}
+
+// dimension d of atom i frozen in every bead
+static __device__ __forceinline__ bool frozen(const Batch &B, const TrajView &T, int i, int d) {
+    const uint8_t *fx = B.fixed + T.base + i;
+    for (int b = 0; b < T.nb; ++b)
+        if (!(fx[(int64_t)b * T.N] >> d & 1)) return false;
+    return true;
 }
 
 // pile_thermostat, md_algo.f90:440-502, for one dimension of an atom (the per-type, per-mode
@@ -560,6 +628,7 @@ static __device__ void pile(const Batch &B, const PropParams &P, const TrajView 
     const double betaN = 1.0 / (kBoltz * temp_of(B, P, ty) * nb);
     const double sq = sqrt(m / betaN);
     const double *c1t = rp_table(cjk, nb, kRpC1) + ty * nb, *c2t = rp_table(cjk, nb, kRpC2) + ty * nb;
+    if (frozen(B, T, i, d)) return;  // the half-step that follows sets its velocity to zero
     const double im = B.imass[T.aoff + i];
     double newP[32], atomP[32];
     for (int b = 0; b < nb; ++b) atomP[b] = m * comp(B.vx, B.vy, B.vz, d, T.base + (int64_t)b * T.N + i);
@@ -633,7 +702,9 @@ static __device__ void propagate_1(const Batch &B, const PropParams &P, const Tr
     // work items (dimension, atom): three times the threads of a loop over atoms, so that a small
     // trajectory's FP64 work spreads over the CTA's warps
     for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
-        const int d = w / T.N, i = w - d * T.N;
+        // (ring polymers: atom-major, so that the frozen layers, whose transforms are left out, make
+        // whole warps)
+        const int d = T.nb > 1 ? w % 3 : w / T.N, i = T.nb > 1 ? w / 3 : w - d * T.N;
         const int algo = B.algo[B.type[T.aoff + i]];
         switch (algo) {
             case kPropVerlet: verlet_half(B, P, T, i, d, true); break;
@@ -702,6 +773,9 @@ static __device__ void ring_polymer_step(const Batch &B, const PropParams &P, co
     for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
         const int i = w / 3, d = w - 3 * (w / 3);
         const int ty = B.type[T.aoff + i];
+        const int algo = B.algo[ty];
+        const bool revert = (algo == kPropLangevin || algo == kPropLangevinConst);
+        if (!revert && frozen(B, T, i, d)) continue;  // keeps its positions and velocities
         const double m = B.mass[T.aoff + i], im = B.imass[T.aoff + i];
         double p[32], q[32], np[32], nq[32];
         for (int b = 0; b < nb; ++b) {
@@ -722,8 +796,6 @@ static __device__ void ring_polymer_step(const Batch &B, const PropParams &P, co
             nq[b] = np[b] * c2 + nq[b] * c3;
             np[b] = pn;
         }
-        const int algo = B.algo[ty];
-        const bool revert = (algo == kPropLangevin || algo == kPropLangevinConst);
         if (!revert) {
             // back to beads (p and q reused); v = sum_k p_k cjk(b,k) / m with the division
             // after the sum (one FP64 division per bead instead of per term)
