@@ -207,6 +207,11 @@ static __device__ int acsf_neighbors_one(const NNDev &M, int i, int N, const dou
     return cnt;
 }
 
+template <typename R> __device__ __forceinline__ R narrow(double x) {
+    if constexpr (sizeof(R) == 4) return f32_of(x);
+    else return x;
+}
+
 // neighbour cache of central atom i for its warp
 template <typename R>
 __device__ void acsf_cache(const NNDev &M, const WarpCache<R> &C, int i, int ei, int cnt, const int *words,
@@ -217,15 +222,17 @@ __device__ void acsf_cache(const NNDev &M, const WarpCache<R> &C, int i, int ei,
     for (int q = lane; q < cnt; q += 32) {
         const int w = words[q];
         const int j = w & 0xFFFF;
-        const double n1 = ((w >> 16) & 15) - 8, n2 = ((w >> 20) & 15) - 8, n3 = ((w >> 24) & 15) - 8;
+        const double n1 = f64_of((float)(((w >> 16) & 15) - 8)), n2 = f64_of((float)(((w >> 20) & 15) - 8)),
+                     n3 = f64_of((float)(((w >> 24) & 15) - 8));
         const double dx = px[j] + n1 * L[0] + n2 * L[3] + n3 * L[6] - px[i];
         const double dy = py[j] + n1 * L[1] + n2 * L[4] + n3 * L[7] - py[i];
         const double dz = pz[j] + n1 * L[2] + n2 * L[5] + n3 * L[8] - pz[i];
-        const R r = (R)sqrt(dx * dx + dy * dy + dz * dz);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const R r = narrow<R>(r2 * rsqrt_nr(r2));
         R *e = C.nb + q * C.st;
-        e[0] = (R)dx;
-        e[1] = (R)dy;
-        e[2] = (R)dz;
+        e[0] = narrow<R>(dx);
+        e[1] = narrow<R>(dy);
+        e[2] = narrow<R>(dz);
         e[3] = r;
         R fc = R(0), dfc = R(0);
         if (r <= rc) cutoff_fn<R>(M, rc, r, fc, dfc);
@@ -330,6 +337,10 @@ template <typename R> __device__ void acsf_forward(const NNDev &M, const WarpCac
         acc = warp_sum(acc);
         if (lane == 0) G[s] = acc;
     }
+    if (M.ng3eta[ei] == 0) {  // no angular functions: no triplets to walk
+        __syncwarp();
+        return;
+    }
     if (M.g3fast[ei]) {
         acsf_g3_forward_fast<R>(M, C, ei, cnt, G);
         return;
@@ -391,8 +402,8 @@ __device__ void acsf_vjp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
         fiz += fr * e[2];
     }
     __syncwarp();
-    if (M.g3fast[ei]) {
-        acsf_g3_vjp_fast<R>(M, C, ei, cnt, c, fix, fiy, fiz);
+    if (M.ng3eta[ei] == 0 || M.g3fast[ei]) {
+        if (M.ng3eta[ei]) acsf_g3_vjp_fast<R>(M, C, ei, cnt, c, fix, fiy, fiz);
         __syncwarp();
         fix = warp_sum(fix);
         fiy = warp_sum(fiy);
@@ -467,6 +478,10 @@ __device__ void acsf_jvp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
         }
         acc = warp_sum(acc);
         if (lane == 0) v[s] = acc;
+    }
+    if (M.ng3eta[ei] == 0) {
+        __syncwarp();
+        return;
     }
     if (M.g3fast[ei]) {
         acsf_g3_jvp_fast<R>(M, C, ei, cnt, i, ux, uy, uz, v);

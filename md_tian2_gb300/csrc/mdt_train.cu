@@ -60,6 +60,7 @@ template <typename R> struct SmemTrain {
     int8_t *nbelem;
     R *buf;   // per warp: G, c/v, then 6 x (L+1) x kMaxNodes network buffers
     double *scal;  // 0: a (dL/dE in Ha^-1 units)
+    double *smn, *sk;  // scaling per element and function: scaled = (G - smn) sk + scmin
     int stride;
 };
 
@@ -70,7 +71,7 @@ __host__ __device__ inline size_t train_smem_bytes(int max_atoms, int maxnb, int
     s += r16(rs * (size_t)nelem * maxweights) * (1 + warps);
     s += r16(rs * warps * maxnb * (6 + ngeta)) + r16(rs * warps * maxnb * 3) + r16(4 * warps * maxnb) +
          r16(warps * maxnb);
-    s += r16(rs * warps * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes)) + r16(8 * 4);
+    s += r16(rs * warps * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes)) + r16(8 * 4) + 2 * r16(8 * nelem * kMaxSF);
     return s;
 }
 
@@ -106,6 +107,8 @@ __device__ SmemTrain<R> carve_train(unsigned char *base, const NNDev &M, int max
     s.nbelem = (int8_t *)take(W * M.maxnb);
     s.buf = (R *)take(sizeof(R) * W * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes));
     s.scal = (double *)take(8 * 4);
+    s.smn = (double *)take(8 * M.nelem * kMaxSF);
+    s.sk = (double *)take(8 * M.nelem * kMaxSF);
     return s;
 }
 
@@ -148,6 +151,15 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
     const size_t nw = (size_t)M.nelem * M.maxweights;
     for (size_t k = tid; k < nw; k += nt) S.w[k] = (R)D.theta[k];
     for (size_t k = tid; k < nw * W; k += nt) S.gradw[k] = R(0);
+    // the scaling's FP64 divisions once per CTA, not per atom and pass
+    for (int k = tid; k < M.nelem * kMaxSF; k += nt) {
+        const int e = k / kMaxSF, f = k - e * kMaxSF;
+        if (f >= M.nsf[e]) continue;
+        const double mn = M.smin[e * M.maxsf + f];
+        S.smn[k] = mn;
+        S.sk[k] = (M.scmax - M.scmin) / (M.smax[e * M.maxsf + f] - mn);
+    }
+    __syncthreads();
     WarpCache<R> C{S.nb + (size_t)warp * M.maxnb * S.stride, S.slotf + (size_t)warp * M.maxnb * 3,
                    S.nbatom + warp * M.maxnb, S.nbelem + warp * M.maxnb, S.stride};
     R *wb = S.buf + (size_t)warp * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes);
@@ -182,7 +194,7 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
             const int ei = S.elem[i];
             if (ei < 0) continue;
             const int cnt = X.nbcnt[base + i];
-            const int nsf = M.nsf[ei], sfb = ei * M.maxsf;
+            const int nsf = M.nsf[ei], sfb = ei * kMaxSF;
             const R *we = S.w + (size_t)ei * M.maxweights;
             acsf_cache<R>(M, C, i, ei, cnt, X.nbw + (base + i) * (int64_t)M.maxnb, S.px, S.py, S.pz, S.elem, S.lat);
             if (D.dgin) {  // the network ran outside: its output and dE/dG
@@ -191,10 +203,8 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
                 for (int s = lane; s < nsf; s += 32) cv[s] = (R)D.dgin[(base + i) * M.maxsf + s];
                 __syncwarp();
             } else {
-                for (int s = lane; s < nsf; s += 32) {
-                    const double mn = M.smin[sfb + s], w = M.smax[sfb + s] - mn;
-                    h[s] = (R)((D.G[(base + i) * M.maxsf + s] - mn) / w * (M.scmax - M.scmin) + M.scmin);
-                }
+                for (int s = lane; s < nsf; s += 32)
+                    h[s] = (R)((D.G[(base + i) * M.maxsf + s] - S.smn[sfb + s]) * S.sk[sfb + s] + M.scmin);
                 __syncwarp();
                 net_forward<R>(M, we, ei, z, h, zd, hd, false);
                 if (lane == 0) e_warp += (double)h[M.nlayers * kMaxNodes] + (M.remove_atom_energies ? M.atom_energy[ei] : 0.0);
@@ -208,7 +218,8 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
                             const int nn = M.nodes[ei][l + 1];
                             const R *wl = we + M.woff[ei][l + 1];
                             up = R(0);
-                            for (int m = 0; m < nn; ++m) up += wl[n * nn + m] * dl[(l + 1) * kMaxNodes + m];
+                            for (int q = 0, m = n % nn; q < nn; ++q, m = m + 1 == nn ? 0 : m + 1)
+                                up += wl[n * nn + m] * dl[(l + 1) * kMaxNodes + m];
                         }
                         dl[l * kMaxNodes + n] = dn * up;
                     }
@@ -219,8 +230,10 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
                     const R *wl = we + M.woff[ei][1];
                     for (int s = lane; s < nsf; s += 32) {
                         R v = R(0);
-                        for (int n = 0; n < n1; ++n) v += wl[s * n1 + n] * dl[1 * kMaxNodes + n];
-                        cv[s] = v * (R)((M.scmax - M.scmin) / (M.smax[sfb + s] - M.smin[sfb + s]));
+                        // (each lane starts at its own column: rows of 32 weights share their banks)
+                        for (int q = 0, n = s % n1; q < n1; ++q, n = n + 1 == n1 ? 0 : n + 1)
+                            v += wl[s * n1 + n] * dl[1 * kMaxNodes + n];
+                        cv[s] = v * (R)S.sk[sfb + s];
                     }
                 }
                 __syncwarp();
@@ -269,25 +282,21 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
             const int ei = S.elem[i];
             if (ei < 0) continue;
             const int cnt = X.nbcnt[base + i];
-            const int nsf = M.nsf[ei], sfb = ei * M.maxsf;
+            const int nsf = M.nsf[ei], sfb = ei * kMaxSF;
             const R *we = S.w + (size_t)ei * M.maxweights;
             R *gwe = gw + (size_t)ei * M.maxweights;
             acsf_cache<R>(M, C, i, ei, cnt, X.nbw + (base + i) * (int64_t)M.maxnb, S.px, S.py, S.pz, S.elem, S.lat);
             acsf_jvp<R>(M, C, ei, cnt, i, S.ux, S.uy, S.uz, cv);
             if (D.xdot) {  // the network's sweep runs outside: its inputs
-                for (int s = lane; s < nsf; s += 32) {
-                    const double w = M.smax[sfb + s] - M.smin[sfb + s];
-                    D.xdot[(base + i) * M.maxsf + s] = (float)(cv[s] * (R)((M.scmax - M.scmin) / w));
-                }
+                for (int s = lane; s < nsf; s += 32)
+                    D.xdot[(base + i) * M.maxsf + s] = (float)(cv[s] * (R)S.sk[sfb + s]);
                 if (lane == 0) D.arow[base + i] = (double)a;
                 __syncwarp();
                 continue;
             }
             for (int s = lane; s < nsf; s += 32) {
-                const double mn = M.smin[sfb + s], w = M.smax[sfb + s] - mn;
-                const R sc = (R)((M.scmax - M.scmin) / w);
-                h[s] = (R)((D.G[(base + i) * M.maxsf + s] - mn) / w * (M.scmax - M.scmin) + M.scmin);
-                hd[s] = cv[s] * sc;
+                h[s] = (R)((D.G[(base + i) * M.maxsf + s] - S.smn[sfb + s]) * S.sk[sfb + s] + M.scmin);
+                hd[s] = cv[s] * (R)S.sk[sfb + s];
             }
             __syncwarp();
             net_forward<R>(M, we, ei, z, h, zd, hd, true);
@@ -313,7 +322,7 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
                     const R *wl = we + wo;
                     for (int p = lane; p < nprev; p += 32) {
                         R gd = R(0), gp = R(0);
-                        for (int n = 0; n < ncur; ++n) {
+                        for (int q = 0, n = p % ncur; q < ncur; ++q, n = n + 1 == ncur ? 0 : n + 1) {
                             gd += wl[p * ncur + n] * dl[l * kMaxNodes + n];
                             gp += wl[p * ncur + n] * dp[l * kMaxNodes + n];
                         }
