@@ -32,7 +32,7 @@
 #include <cstdio>
 
 #include "mdt_common.cuh"
-#include "mdt_emt.cuh"
+#include "mdt_emt_plain.cuh"
 #include "mdt_fastmath.cuh"
 #include "mdt_internal.h"
 #include "mdt_nn.cuh"
@@ -1155,19 +1155,20 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                 const int64_t k = A.base + A.i;
                 const double rx = B.rx[k], ry = B.ry[k], rz = B.rz[k];
                 const double x = rx * kAng2BohrD, y = ry * kAng2BohrD, z = rz * kAng2BohrD;
-                A.xhi = (float)x;
-                A.yhi = (float)y;
-                A.zhi = (float)z;
-                A.xli = (float)(x - (double)A.xhi);
-                A.yli = (float)(y - (double)A.yhi);
-                A.zli = (float)(z - (double)A.zhi);
+                A.xhi = f32_of(x);
+                A.yhi = f32_of(y);
+                A.zhi = f32_of(z);
+                A.xli = f32_of(x - f64_of(A.xhi));
+                A.yli = f32_of(y - f64_of(A.yhi));
+                A.zli = f32_of(z - f64_of(A.zhi));
                 S.ph[tid] = make_float4(A.xhi, A.yhi, A.zhi, 0.f);
                 S.pl[tid] = make_float4(A.xli, A.yli, A.zli, 0.f);
-                if (mode == 2 && !isfinite((rx + ry) + (rz + B.vx[k]) + (B.vy[k] + B.vz[k])))
+                if (mode == 2 && (not_finite(rx) || not_finite(ry) || not_finite(rz) || not_finite(B.vx[k]) ||
+                                  not_finite(B.vy[k]) || not_finite(B.vz[k])))
                     S.tr_bad[cur * kRMaxTraj + A.s] = 1;
                 if (R.skin > 0.f) {
                     const double *r0 = X.skref + 3 * k;
-                    const float ddx = (float)(rx - r0[0]), ddy = (float)(ry - r0[1]), ddz = (float)(rz - r0[2]);
+                    const float ddx = f32_of(rx - r0[0]), ddy = f32_of(ry - r0[1]), ddz = f32_of(rz - r0[2]);
                     atomicMax(&d2[A.s], __float_as_int(ddx * ddx + ddy * ddy + ddz * ddz));
                 }
             }
@@ -1247,7 +1248,7 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                 for (int q = 0; q < KT; ++q) dG[q] = S.hb[q * bs + tid];
             }
             if (active) {
-                S.ea[tid] = (double)e_at + R.atom_energy[A.ei];
+                S.ea[tid] = f64_of(e_at) + R.atom_energy[A.ei];
                 if (do_forces) nnr_forces<KA, KB, BLA, BLB, TC ? 1 : 3>(R, S, A, sk, cnt, dG, fix, fiy, fiz);
             }
             __syncthreads();  // (B)
@@ -1276,9 +1277,9 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                 const double c = kHa2eVR * kAng2BohrD;
                 double fx = 0.0, fy = 0.0, fz = 0.0;
                 if (do_forces && !fb) {
-                    fx = (double)(S.f3[tid] + fix) * c;
-                    fy = (double)(S.f3[bs + tid] + fiy) * c;
-                    fz = (double)(S.f3[2 * bs + tid] + fiz) * c;
+                    fx = f64_of(S.f3[tid] + fix) * c;
+                    fy = f64_of(S.f3[bs + tid] + fiy) * c;
+                    fz = f64_of(S.f3[2 * bs + tid] + fiz) * c;
                 }
                 B.fx[k] = fx;
                 B.fy[k] = fy;
@@ -1299,7 +1300,7 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                         if (!stat[s] || !flag[s]) continue;
                         const int t = S.tr_t[s];
                         __syncthreads();
-                        emt_beads<double>(B, E, SE, t, 0, 1, do_forces);
+                        emt_bead_plain(B, E, SE, t, 0, do_forces);
                         if (tid == 0) X.fallback[t] += 1;
                         if (A.s == s && do_forces) {
                             const int64_t k = A.base + A.i;
