@@ -14,7 +14,7 @@ struct LaunchCfg {
     int grid;
     const int *order;  // trajectory work order (largest first)
     int *counter;      // device work-queue counter (reset by the launcher)
-    int parts = 1;     // generic HDNNP force calls: CTAs per trajectory (single beads)
+    int parts = 1;     // CTAs per trajectory (EMT ring polymers: a cluster; generic HDNNP force calls, single beads)
     int64_t total_ba = 0;
 };
 

@@ -15,6 +15,9 @@
 //     (3,nb,N,N) derivative tensors (src/pes_emt_mod.f90:483-1027).
 // The fused kernel runs propagate_1 -> calc_force -> propagate_2 for many steps
 // without leaving the CTA (md_tian2.f90:78-92).
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cstdio>
 
 #include "mdt_common.cuh"
@@ -32,26 +35,49 @@ __device__ void calc_force(const Batch &B, const EmtConst &E, const PropParams &
     const int tot = T.N * T.nb;
     const bool single = T.nb == 1 && do_forces;  // no spring forces: the bead's forces are stored, not added
     if (!single)
-        for (int s = threadIdx.x; s < tot; s += blockDim.x) {
+        for (int s = T.first(); s < tot; s += T.stride()) {
             const int64_t k = T.base + s;
             B.fx[k] = 0.0; B.fy[k] = 0.0; B.fz[k] = 0.0;
             B.ax[k] = 0.0; B.ay[k] = 0.0; B.az[k] = 0.0;
         }
-    for (int b = threadIdx.x; b < T.nb; b += blockDim.x) B.epot[B.bead_off[T.t] + b] = 0.0;
-    __syncthreads();
+    for (int b = T.first(); b < T.nb; b += T.stride()) B.epot[B.bead_off[T.t] + b] = 0.0;
+    team_sync(T);
     if (T.nb > 1) ring_polymer_step(B, P, T, S.cjk);
-    const int G = min(T.nb, S.places / T.N);
-    for (int b = 0; b < T.nb; b += G) emt_beads<R>(B, E, S, T.t, b, min(G, T.nb - b), do_forces, single);
-    if (do_forces) set_acceleration(B, T);
-    __syncthreads();
+    // this CTA's beads, several at a time
+    const int per = (T.nb + T.size - 1) / T.size, b0 = min(T.rank * per, T.nb), b1 = min(b0 + per, T.nb);
+    const int G = min(per, S.places / T.N);
+    for (int b = b0; b < b1; b += G) emt_beads<R>(B, E, S, T.t, b, min(G, b1 - b), do_forces, single);
+    if (do_forces) set_acceleration(B, T, b0, b1);
+    team_sync(T);
 }
 
-__device__ __forceinline__ int next_work(int *counter, int *shared_slot) {
-    if (threadIdx.x == 0) *shared_slot = atomicAdd(counter, 1);
-    __syncthreads();
-    const int w = *shared_slot;
-    __syncthreads();
+// The next trajectory of the work queue, for every CTA of the team (a cluster: its first CTA asks,
+// the others read its answer).
+__device__ __forceinline__ int next_work(int *counter, int *shared_slot, int rank, int size) {
+    if (size == 1) {
+        if (threadIdx.x == 0) *shared_slot = atomicAdd(counter, 1);
+        __syncthreads();
+        const int w = *shared_slot;
+        __syncthreads();
+        return w;
+    }
+    const cooperative_groups::cluster_group team = cooperative_groups::this_cluster();
+    if (rank == 0 && threadIdx.x == 0) *shared_slot = atomicAdd(counter, 1);
+    team.sync();
+    const int w = *team.map_shared_rank(shared_slot, 0);
+    team.sync();
     return w;
+}
+
+__device__ __forceinline__ int cluster_rank() {
+    int r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ int cluster_size() {
+    int n;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+    return n;
 }
 
 // ---------------------------------------------------------------------------
@@ -63,11 +89,12 @@ __global__ void __launch_bounds__(kBlock, 4) phase_kernel(Batch B, EmtConst E, P
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
     SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads, emt_places(B.max_atoms, B.max_beads));
+    const int rank = cluster_rank(), size = cluster_size();
     for (;;) {
-        const int w = next_work(counter, &work_slot);
+        const int w = next_work(counter, &work_slot, rank, size);
         if (w >= B.ntraj) break;
         const int t = order[w];
-        const TrajView T = traj_view(B, t);
+        const TrajView T = traj_view(B, t, rank, size);
         load_cjk(B, t, S.cjk);
         const int step = B.steps_done[t] + 1;
         if (phase == kPhaseForce || phase == kPhaseEnergyOnly)
@@ -76,7 +103,7 @@ __global__ void __launch_bounds__(kBlock, 4) phase_kernel(Batch B, EmtConst E, P
             propagate_1(B, P, T, S.cjk, step, S.red);
         else {
             propagate_2(B, P, T, step);
-            if (threadIdx.x == 0) B.steps_done[t] = step;
+            if (T.first() == 0) B.steps_done[t] = step;
             __syncthreads();
         }
     }
@@ -89,11 +116,12 @@ __global__ void __launch_bounds__(kBlock, 4) md_steps_kernel(Batch B, EmtConst E
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
     SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads, emt_places(B.max_atoms, B.max_beads));
+    const int rank = cluster_rank(), size = cluster_size();
     for (;;) {
-        const int w = next_work(counter, &work_slot);
+        const int w = next_work(counter, &work_slot, rank, size);
         if (w >= B.ntraj) break;
         const int t = order[w];
-        const TrajView T = traj_view(B, t);
+        const TrajView T = traj_view(B, t, rank, size);
         load_cjk(B, t, S.cjk);
         for (int s = 0; s < nsteps; ++s) {
             if (B.status[t] != kStatusRunning) break;
@@ -101,13 +129,14 @@ __global__ void __launch_bounds__(kBlock, 4) md_steps_kernel(Batch B, EmtConst E
             propagate_1(B, P, T, S.cjk, step, S.red);
             calc_force<R>(B, E, P, S, T, true);
             propagate_2(B, P, T, step);
-            {
+            if (rank == 0) {
                 int near;
                 double rv[3];
                 const double dmin = closest_approach_step(B, T, S.cell, S.red, &near, rv);
                 if (threadIdx.x == 0) observe_step(B, P, T, step, dmin, near, rv[0], rv[1], rv[2]);
             }
-            end_of_step(B, P, T, step);
+            if (rank == 0) end_of_step(B, P, T, step);
+            if (size > 1) team_sync(T);
         }
     }
 }
@@ -402,6 +431,23 @@ cudaError_t launch_summary(cudaStream_t s, const Batch &B, const PropParams &P, 
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
+// c.grid CTAs in clusters of c.parts
+template <typename... P, typename... A>
+static cudaError_t launch_team(const LaunchCfg &c, void (*kernel)(P...), size_t smem, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(c.grid);
+    cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = c.parts;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = c.parts > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <typename R>
 static cudaError_t launch_phase_t(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P,
                                   int phase) {
@@ -410,8 +456,7 @@ static cudaError_t launch_phase_t(const LaunchCfg &c, const Batch &B, const EmtC
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
     if (e != cudaSuccess) return e;
-    phase_kernel<R><<<c.grid, kBlock, sm, c.stream>>>(B, E, P, c.order, c.counter, phase);
-    return cudaGetLastError();
+    return launch_team(c, phase_kernel<R>, sm, B, E, P, c.order, c.counter, phase);
 }
 
 cudaError_t launch_phase(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P, int phase,
@@ -427,8 +472,7 @@ static cudaError_t launch_md_t(const LaunchCfg &c, const Batch &B, const EmtCons
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
     if (e != cudaSuccess) return e;
-    md_steps_kernel<R><<<c.grid, kBlock, sm, c.stream>>>(B, E, P, c.order, c.counter, nsteps);
-    return cudaGetLastError();
+    return launch_team(c, md_steps_kernel<R>, sm, B, E, P, c.order, c.counter, nsteps);
 }
 
 cudaError_t launch_md_steps(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P, int nsteps,

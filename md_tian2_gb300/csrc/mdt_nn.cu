@@ -288,7 +288,7 @@ __device__ void nn_calc_force(const Batch &B, const NNDev &M, const EmtConst &E,
             if (threadIdx.x == 0) X.fallback[T.t] += 1;
         }
     }
-    if (do_forces) set_acceleration(B, T);
+    if (do_forces) set_acceleration(B, T, 0, T.nb);
     __syncthreads();
 }
 
@@ -307,7 +307,7 @@ __global__ void nn_zero_kernel(Batch B, int64_t total) {
 }
 
 __global__ void nn_accel_kernel(Batch B) {
-    for (int t = blockIdx.x; t < B.ntraj; t += gridDim.x) set_acceleration(B, traj_view(B, t));
+    for (int t = blockIdx.x; t < B.ntraj; t += gridDim.x) set_acceleration(B, traj_view(B, t), 0, 1);
 }
 
 template <typename R, bool SURR>

@@ -10,13 +10,27 @@ namespace mdt {
 // ---------------------------------------------------------------------------
 // Propagators (src/md_algo.f90).  Thread per atom, all beads of the atom.
 // ---------------------------------------------------------------------------
+// A trajectory as its team of CTAs sees it: one CTA, or the CTAs of a cluster that share a ring
+// polymer (their work items interleave, their state meets in global memory, team_sync orders it).
 struct TrajView {
     int t, N, nb, aoff;
     int64_t base;
+    int rank, size;  // this CTA of the team
+    __device__ __forceinline__ int first() const { return rank * (int)blockDim.x + (int)threadIdx.x; }
+    __device__ __forceinline__ int stride() const { return size * (int)blockDim.x; }
 };
 
-static __device__ __forceinline__ TrajView traj_view(const Batch &B, int t) {
-    return TrajView{t, B.natoms[t], B.nbeads[t], B.atom_off[t], B.ba_off[t]};
+static __device__ __forceinline__ TrajView traj_view(const Batch &B, int t, int rank = 0, int size = 1) {
+    return TrajView{t, B.natoms[t], B.nbeads[t], B.atom_off[t], B.ba_off[t], rank, size};
+}
+
+static __device__ __forceinline__ void team_sync(const TrajView &T) {
+    if (T.size > 1) {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
 }
 
 static __device__ __forceinline__ double temp_of(const Batch &B, const PropParams &P, int ty) {
@@ -644,10 +658,9 @@ static __device__ void pile(const Batch &B, const PropParams &P, const TrajView 
     }
 }
 
-// set_acceleration, force.f90:89-98
-static __device__ __forceinline__ void set_acceleration(const Batch &B, const TrajView &T) {
-    const int tot = T.N * T.nb;
-    for (int s = threadIdx.x; s < tot; s += blockDim.x) {
+// set_acceleration, force.f90:89-98, for beads b0 .. b1 - 1
+static __device__ __forceinline__ void set_acceleration(const Batch &B, const TrajView &T, int b0, int b1) {
+    for (int s = b0 * T.N + threadIdx.x; s < b1 * T.N; s += blockDim.x) {
         const int64_t k = T.base + s;
         const int i = s % T.N;
         const double m = B.mass[T.aoff + i], im = B.imass[T.aoff + i];
@@ -676,17 +689,18 @@ static __device__ void remove_com(const Batch &B, const TrajView &T, double *red
         v[2] += az * m;
         v[3] += m;
     }
-    block_sum4(v, red);
+    block_sum4(v, red);  // (each CTA of a team sums all of it)
+    if (T.size > 1) team_sync(T);
     const double n = (double)T.N, ms = v[3], fac = B.comfac[T.t];
     const double cx = v[0] / ms / T.nb / n * fac, cy = v[1] / ms / T.nb / n * fac, cz = v[2] / ms / T.nb / n * fac;
     const int tot = T.N * T.nb;
-    for (int s = threadIdx.x; s < tot; s += blockDim.x) {
+    for (int s = T.first(); s < tot; s += T.stride()) {
         const int64_t k = T.base + s;
         B.vx[k] -= cx;
         B.vy[k] -= cy;
         B.vz[k] -= cz;
     }
-    __syncthreads();
+    team_sync(T);
 }
 
 static __device__ bool traj_has_algo(const Batch &B, int id) {
@@ -701,7 +715,7 @@ static __device__ void propagate_1(const Batch &B, const PropParams &P, const Tr
     if (traj_has_algo(B, kPropPile)) pile_tables(B, P, T, cjk);
     // work items (dimension, atom): three times the threads of a loop over atoms, so that a small
     // trajectory's FP64 work spreads over the CTA's warps
-    for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
+    for (int w = T.first(); w < 3 * T.N; w += T.stride()) {
         // (ring polymers: atom-major, so that the frozen layers, whose transforms are left out, make
         // whole warps)
         const int d = T.nb > 1 ? w % 3 : w / T.N, i = T.nb > 1 ? w / 3 : w - d * T.N;
@@ -721,29 +735,29 @@ static __device__ void propagate_1(const Batch &B, const PropParams &P, const Tr
         }
     }
     if (traj_has_algo(B, kPropLangevin))  // LDFA: an atom's coefficients serve its three dimensions
-        for (int i = threadIdx.x; i < T.N; i += blockDim.x)
+        for (int i = T.first(); i < T.N; i += T.stride())
             if (B.algo[B.type[T.aoff + i]] == kPropLangevin) langevin_1(B, P, T, i, step, kPropLangevin);
-    __syncthreads();
+    team_sync(T);
     if (traj_has_algo(B, kPropAndersen) || traj_has_algo(B, kPropPile)) remove_com(B, T, red);
 }
 
 // propagate_2, md_algo.f90:80-106
 static __device__ void propagate_2(const Batch &B, const PropParams &P, const TrajView &T, int step) {
     bool bad = false;
-    for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
+    for (int w = T.first(); w < 3 * T.N; w += T.stride()) {
         const int d = w / T.N, i = w - d * T.N;
         const int algo = B.algo[B.type[T.aoff + i]];
         if (algo == kPropLangevinConst) lc_half2(B, P, T, i, d, step);
         else if (algo != kPropLangevin) verlet_half(B, P, T, i, d, false);
     }
     if (traj_has_algo(B, kPropLangevin))
-        for (int i = threadIdx.x; i < T.N; i += blockDim.x)
+        for (int i = T.first(); i < T.N; i += T.stride())
             if (B.algo[B.type[T.aoff + i]] == kPropLangevin) {
                 if (!ldfa(B, T, i)) bad = true;
                 langevin_2(B, P, T, i, step, kPropLangevin);
             }
     if (bad) B.status[T.t] = kStatusErrDensity;
-    __syncthreads();
+    team_sync(T);
 }
 
 // do_ring_polymer_step, rpmd.f90:309-452.  Thread per (atom, dimension); the free
@@ -770,7 +784,7 @@ static __device__ void ring_polymer_step(const Batch &B, const PropParams &P, co
         swt[w] = sw;
     }
     __syncthreads();
-    for (int w = threadIdx.x; w < 3 * T.N; w += blockDim.x) {
+    for (int w = T.first(); w < 3 * T.N; w += T.stride()) {
         const int i = w / 3, d = w - 3 * (w / 3);
         const int ty = B.type[T.aoff + i];
         const int algo = B.algo[ty];
@@ -818,7 +832,7 @@ static __device__ void ring_polymer_step(const Batch &B, const PropParams &P, co
             }
         }
     }
-    __syncthreads();
+    team_sync(T);
 }
 
 // End of one fused MD step of the CTA that owns trajectory T (md_tian2.f90:78-92): the step
