@@ -10,6 +10,7 @@
 
 #include "../../include/mdt_gpu.h"
 #include "mdt_common.cuh"
+#include "mdt_emt.cuh"
 #include "mdt_internal.h"
 
 using namespace mdt;
@@ -54,6 +55,7 @@ struct mdt_ctx {
     double *rnd[4] = {nullptr, nullptr, nullptr, nullptr};
     double *summary = nullptr;
     size_t scratch_prec_bytes = 0;
+    int emt_per_sm[2] = {0, 0};  // resident CTAs of the EMT kernels (FP64, FP32 forces); 0: not asked yet
 
     // HDNNP / surrogate
     bool have_nn = false;
@@ -167,6 +169,7 @@ void free_batch(mdt_ctx *c) {
     c->g_eat = c->g_arow = nullptr;
     c->have_labels = false;
     c->nn_maxnb_alloc = 0;
+    c->emt_per_sm[0] = c->emt_per_sm[1] = 0;
     for (auto &b : c->bufs) cudaFree(b.p);
     c->bufs.clear();
     c->have_batch = false;
@@ -269,9 +272,12 @@ int check_ready(mdt_ctx *c, bool need_emt) {
 // with one, 13.1 with 8; 1024 with FP32 forces 26.3 ms with one, 22.4 with 2, 33 with 4 (fewer beads at a
 // time fill fewer warps, and every CTA repeats the tables and sums of a step).
 LaunchCfg cfg(mdt_ctx *c, int precision) {
-    const int per_sm = max_resident_ctas(c->max_atoms, c->max_beads, precision);
+    int &per_sm = c->emt_per_sm[precision == MDT_PREC_FP32 ? 1 : 0];
+    if (!per_sm) per_sm = max_resident_ctas(c->max_atoms, c->max_beads, precision);
     const int slots = c->num_sms * per_sm;
     LaunchCfg g{c->stream, std::max(1, std::min(c->T, slots)), c->order, c->counter};
+    // at most one trajectory per SM: twice the warps shorten its chain of phases
+    if (c->max_beads == 1 && c->T <= c->num_sms) g.threads = kWideBlock;
     if (c->max_beads > 1) {
         g.parts = 1;
         while (g.parts < 8 && 2 * g.parts <= c->max_beads && (int64_t)c->T * 2 * g.parts <= 4 * (int64_t)slots)
@@ -1247,9 +1253,6 @@ int32_t mdt_state_upload(mdt_ctx *c, const double *r, const double *v) {
         e = launch_unpack_state(c->stream, B, sr, sv, c->tmpl, c->total_ba, c->ba_traj);
         c->launches++;
     }
-    if (e == cudaSuccess) e = cudaMemsetAsync(B.status, 0, sizeof(int) * c->T, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(B.steps_done, 0, sizeof(int) * c->T, c->stream);
-    if (e == cudaSuccess) e = launch_obs_reset(c->stream, B);
     // every trajectory runs again: a re-pack over the running ones gives way to a plan of all of
     // them (a plan of all trajectories stays: the cells did not change, and the skin lists
     // check every atom's displacement since their build, whatever moved it)
@@ -1269,19 +1272,15 @@ int32_t mdt_state_download(mdt_ctx *c, double *r, double *v, double *f, double *
     // back to back and one synchronisation ends the call
     double *sl[4];
     for (int k = 0; k < 4; ++k) sl[k] = outs[k] ? c->stage + 3 * (size_t)k * c->total_ba : nullptr;
-    if (r || v || f || a) {
-        e = launch_pack_state(c->stream, B, sl[0], sl[1], sl[2], sl[3], c->total_ba, c->ba_traj);
+    double *sd = dens ? c->stage + 12 * (size_t)c->total_ba : nullptr;
+    if (r || v || f || a || dens) {
+        e = launch_pack_state(c->stream, B, sl[0], sl[1], sl[2], sl[3], sd, c->total_ba, c->ba_traj);
         c->launches++;
     }
     for (int k = 0; k < 4 && e == cudaSuccess; ++k)
         if (outs[k]) e = cudaMemcpyAsync(outs[k], sl[k], bytes, cudaMemcpyDeviceToHost, c->stream);
-    if (dens && e == cudaSuccess) {
-        double *sd = c->stage + 12 * (size_t)c->total_ba;
-        e = launch_pack_scalar(c->stream, B, sd, B.dens, c->total_ba, c->ba_traj);
-        c->launches++;
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(dens, sd, sizeof(double) * c->total_ba, cudaMemcpyDeviceToHost, c->stream);
-    }
+    if (dens && e == cudaSuccess)
+        e = cudaMemcpyAsync(dens, sd, sizeof(double) * c->total_ba, cudaMemcpyDeviceToHost, c->stream);
     if (epot && e == cudaSuccess)
         e = cudaMemcpyAsync(epot, B.epot, sizeof(double) * c->total_beads, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);

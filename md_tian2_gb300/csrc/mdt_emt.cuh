@@ -6,7 +6,8 @@
 
 namespace mdt {
 
-constexpr int kBlock = 128;  // threads per CTA (one trajectory per CTA)
+constexpr int kBlock = 128;      // threads per CTA (one trajectory per CTA)
+constexpr int kWideBlock = 256;  // the same for batches of at most one trajectory per SM
 
 // ---------------------------------------------------------------------------
 // Arithmetic helpers.  On GB300 an FP64 instruction costs as much issue bandwidth as
@@ -29,10 +30,20 @@ template <> struct Math<double> {
     static __device__ __forceinline__ double rcp(double x) { return rcp_nr(x); }
     static __device__ __forceinline__ double rsq(double x) { return rsqrt_nr(x); }
 };
+// FP32: the hardware approximations behind __expf and rsqrtf without their steps for denormal
+// operands (results below 2^-126 flush to zero), and a reciprocal of x in [1, 2^126) that rounds
+// as a division does
 template <> struct Math<float> {
-    static __device__ __forceinline__ float ex(float x) { return __expf(x); }
-    static __device__ __forceinline__ float rcp(float x) { return __frcp_rn(x); }
-    static __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
+    static __device__ __forceinline__ float ex(float x) { return ex2a(x * kLog2eF); }
+    static __device__ __forceinline__ float rcp(float x) {
+        const float y = rcpa(x);
+        return fmaf(y, fmaf(-x, y, 1.f), y);
+    }
+    static __device__ __forceinline__ float rsq(float x) {
+        float y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
 };
 
 struct Cell;
@@ -487,15 +498,15 @@ static __device__ __forceinline__ void pairs_density(const SmemEmt<float> &S, Pl
         float acc = 0.f;
         D.set(S, gp + i);
         for (int j = j0; j < j1; ++j) {
-            if (j == i) continue;
             float rx, ry, rz;
             D.diff(S, gp + j, A.N, rx, ry, rz);
             const float r2 = rx * rx + ry * ry + rz * rz;
-            if (beyond(r2, A.cut2)) continue;
-            const float r = r2 * Math<float>::rsq(r2);
-            float theta, rt1;
-            emt_theta<float>(k.acut, k.rcut, r, theta, rt1);
-            acc += k.g * (theta * Math<float>::ex(-k.eta * (r - k.b)));
+            if (j != i && !beyond(r2, A.cut2)) {
+                const float r = r2 * Math<float>::rsq(r2);
+                float theta, rt1;
+                emt_theta<float>(k.acut, k.rcut, r, theta, rt1);
+                acc += k.g * (theta * Math<float>::ex(-k.eta * (r - k.b)));
+            }
         }
         if (A.C == 1) S.sig[gp + i] = acc;
         else atomicAdd(&S.sig[gp + i], acc);
@@ -513,22 +524,22 @@ static __device__ __forceinline__ void pairs_force(const SmemEmt<float> &S, Plac
         EnergySum<float> e_run;
         D.set(S, gp + i);
         for (int j = j0; j < j1; ++j) {
-            if (j == i) continue;
             float rx, ry, rz;
             D.diff(S, gp + j, A.N, rx, ry, rz);
             const float r2 = rx * rx + ry * ry + rz * rz;
-            if (beyond(r2, A.cut2)) continue;
-            const float ir = Math<float>::rsq(r2), r = r2 * ir;
-            float theta, rt1;
-            emt_theta<float>(k.acut, k.rcut, r, theta, rt1);
-            const float phi = theta * Math<float>::ex(-k.eta * (r - k.b));
-            const float psi = theta * Math<float>::ex(-k.kb * (r - k.b));
-            if (i < j) e_run.add(-(k.c * psi));
-            const float q = k.g * (k.etaq + rt1) * phi * ir, fv = -(k.c * (k.kb + rt1) * psi * ir);
-            const float cc = Ai * q + S.A[gp + j] * q + fv;
-            fx += cc * rx;
-            fy += cc * ry;
-            fz += cc * rz;
+            if (j != i && !beyond(r2, A.cut2)) {
+                const float ir = Math<float>::rsq(r2), r = r2 * ir;
+                float theta, rt1;
+                emt_theta<float>(k.acut, k.rcut, r, theta, rt1);
+                const float phi = theta * Math<float>::ex(-k.eta * (r - k.b));
+                const float psi = theta * Math<float>::ex(-k.kb * (r - k.b));
+                e_run.add(i < j ? -(k.c * psi) : 0.f);
+                const float q = k.g * (k.etaq + rt1) * phi * ir, fv = -(k.c * (k.kb + rt1) * psi * ir);
+                const float cc = Ai * q + S.A[gp + j] * q + fv;
+                fx += cc * rx;
+                fy += cc * ry;
+                fz += cc * rz;
+            }
         }
         if (do_forces) {
             atomicAdd(&S.fx[gp + i], fx);

@@ -16,6 +16,7 @@ struct LaunchCfg {
     int *counter;      // device work-queue counter (reset by the launcher)
     int parts = 1;     // CTAs per trajectory (EMT ring polymers: a cluster; generic HDNNP force calls, single beads)
     int64_t total_ba = 0;
+    int threads = 128; // EMT kernels: threads per CTA (kBlock or kWideBlock)
 };
 
 cudaError_t launch_phase(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P, int phase,
@@ -27,9 +28,7 @@ cudaError_t launch_unpack(cudaStream_t s, const Batch &B, const double *src, dou
 cudaError_t launch_unpack_state(cudaStream_t s, const Batch &B, const double *sr, const double *sv, double *tmpl,
                                 int64_t total_ba, const int *ba_traj);
 cudaError_t launch_pack_state(cudaStream_t s, const Batch &B, double *dr, double *dv, double *df, double *da,
-                              int64_t total_ba, const int *ba_traj);
-cudaError_t launch_pack_scalar(cudaStream_t s, const Batch &B, double *dst, const double *x, int64_t total_ba,
-                               const int *ba_traj);
+                              double *dd, int64_t total_ba, const int *ba_traj);
 // the constant-friction Langevin coefficients of every atom (kLcN each) for the parameters P: the
 // propagators read them instead of forming them (FP64 exp, sqrt and divisions) every half-step
 cudaError_t launch_lcoef(cudaStream_t s, const Batch &B, const PropParams &P, const int *ba_traj, int64_t total_ba,

@@ -83,8 +83,8 @@ __device__ __forceinline__ int cluster_size() {
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
-template <typename R>
-__global__ void __launch_bounds__(kBlock, 4) phase_kernel(Batch B, EmtConst E, PropParams P, const int *order,
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) phase_kernel(Batch B, EmtConst E, PropParams P, const int *order,
                                                     int *counter, int phase) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(kBlock, 4) phase_kernel(Batch B, EmtConst E, P
 }
 
 // Fused propagate_1 -> calc_force -> propagate_2 for nsteps steps per trajectory.
-template <typename R>
-__global__ void __launch_bounds__(kBlock, 4) md_steps_kernel(Batch B, EmtConst E, PropParams P, const int *order,
+template <typename R, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) md_steps_kernel(Batch B, EmtConst E, PropParams P, const int *order,
                                                        int *counter, int nsteps) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
@@ -272,7 +272,8 @@ __global__ void unpack_kernel(Batch B, const double *src, double *x, double *y, 
 }
 
 // A state upload in one pass: positions and velocities (each optional, null: kept) from
-// their stage slices into the SoA arrays, and all six into the refill template.
+// their stage slices into the SoA arrays, and all six into the refill template; every trajectory
+// runs again from step 0 with fresh observables.
 __global__ void unpack_state_kernel(Batch B, const double *sr, const double *sv, double *tmpl, int64_t total_ba,
                                     const int *ba_traj) {
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < total_ba;
@@ -313,12 +314,18 @@ __global__ void unpack_state_kernel(Batch B, const double *sr, const double *sv,
         tmpl[3 * total_ba + s] = x;
         tmpl[4 * total_ba + s] = y;
         tmpl[5 * total_ba + s] = z;
+        if (s < B.ntraj) {  // (every trajectory has a slot)
+            B.status[s] = kStatusRunning;
+            B.steps_done[s] = 0;
+            obs_reset_traj(B, (int)s);
+        }
     }
 }
 
-// A state download's packs in one pass: positions, velocities, forces, accelerations (each
-// optional, null: skipped) into their stage slices in the Fortran-order host layout.
-__global__ void pack_state_kernel(Batch B, double *dr, double *dv, double *df, double *da, int64_t total_ba,
+// A state download's packs in one pass: positions, velocities, forces, accelerations and the
+// embedded density (each optional, null: skipped) into their stage slices in the Fortran-order
+// host layout.
+__global__ void pack_state_kernel(Batch B, double *dr, double *dv, double *df, double *da, double *dd, int64_t total_ba,
                                   const int *ba_traj) {
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < total_ba;
          s += (int64_t)gridDim.x * blockDim.x) {
@@ -326,7 +333,8 @@ __global__ void pack_state_kernel(Batch B, double *dr, double *dv, double *df, d
         const int N = B.natoms[t];
         const int64_t loc = s - B.ba_off[t];
         const int b = (int)(loc / N), i = (int)(loc - (int64_t)b * N);
-        const int64_t f = (B.ba_off[t] + (int64_t)i * B.nbeads[t] + b) * 3;
+        const int64_t f1 = B.ba_off[t] + (int64_t)i * B.nbeads[t] + b, f = f1 * 3;
+        if (dd) dd[f1] = B.dens[s];
         if (dr) {
             dr[f] = B.rx[s];
             dr[f + 1] = B.ry[s];
@@ -347,18 +355,6 @@ __global__ void pack_state_kernel(Batch B, double *dr, double *dv, double *df, d
             da[f + 1] = B.ay[s];
             da[f + 2] = B.az[s];
         }
-    }
-}
-
-// scalar per bead-atom (dens) in Fortran (nb, N) order
-__global__ void pack_scalar_kernel(Batch B, double *dst, const double *x, int64_t total_ba, const int *ba_traj) {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < total_ba;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int t = ba_traj[s];
-        const int N = B.natoms[t];
-        const int64_t loc = s - B.ba_off[t];
-        const int b = (int)(loc / N), i = (int)(loc - (int64_t)b * N);
-        dst[B.ba_off[t] + (int64_t)i * B.nbeads[t] + b] = x[s];
     }
 }
 
@@ -436,7 +432,7 @@ template <typename... P, typename... A>
 static cudaError_t launch_team(const LaunchCfg &c, void (*kernel)(P...), size_t smem, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(c.grid);
-    cfg.blockDim = dim3(kBlock);
+    cfg.blockDim = dim3(c.threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
     cudaLaunchAttribute at{};
@@ -448,36 +444,49 @@ static cudaError_t launch_team(const LaunchCfg &c, void (*kernel)(P...), size_t 
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <typename R>
+// the work counter and, beyond the 48 KB that need no opt-in, the shared-memory limit of a kernel
+template <typename K> static cudaError_t prepare(const LaunchCfg &c, K kernel, size_t sm) {
+    if (sm > 47 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
+}
+
+template <typename R, int NT>
 static cudaError_t launch_phase_t(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P,
                                   int phase) {
     const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R), emt_places(B.max_atoms, B.max_beads));
-    cudaError_t e = cudaFuncSetAttribute(phase_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = prepare(c, phase_kernel<R, NT>, sm);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
-    if (e != cudaSuccess) return e;
-    return launch_team(c, phase_kernel<R>, sm, B, E, P, c.order, c.counter, phase);
+    return launch_team(c, phase_kernel<R, NT>, sm, B, E, P, c.order, c.counter, phase);
 }
 
 cudaError_t launch_phase(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P, int phase,
                          int precision) {
-    return precision == 1 ? launch_phase_t<float>(c, B, E, P, phase) : launch_phase_t<double>(c, B, E, P, phase);
+    if (c.threads == kWideBlock)
+        return precision == 1 ? launch_phase_t<float, kWideBlock>(c, B, E, P, phase)
+                              : launch_phase_t<double, kWideBlock>(c, B, E, P, phase);
+    return precision == 1 ? launch_phase_t<float, kBlock>(c, B, E, P, phase)
+                          : launch_phase_t<double, kBlock>(c, B, E, P, phase);
 }
 
-template <typename R>
+template <typename R, int NT>
 static cudaError_t launch_md_t(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P,
                                int nsteps) {
     const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R), emt_places(B.max_atoms, B.max_beads));
-    cudaError_t e = cudaFuncSetAttribute(md_steps_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = prepare(c, md_steps_kernel<R, NT>, sm);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
-    if (e != cudaSuccess) return e;
-    return launch_team(c, md_steps_kernel<R>, sm, B, E, P, c.order, c.counter, nsteps);
+    return launch_team(c, md_steps_kernel<R, NT>, sm, B, E, P, c.order, c.counter, nsteps);
 }
 
 cudaError_t launch_md_steps(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P, int nsteps,
                             int precision) {
-    return precision == 1 ? launch_md_t<float>(c, B, E, P, nsteps) : launch_md_t<double>(c, B, E, P, nsteps);
+    if (c.threads == kWideBlock)
+        return precision == 1 ? launch_md_t<float, kWideBlock>(c, B, E, P, nsteps)
+                              : launch_md_t<double, kWideBlock>(c, B, E, P, nsteps);
+    return precision == 1 ? launch_md_t<float, kBlock>(c, B, E, P, nsteps)
+                          : launch_md_t<double, kBlock>(c, B, E, P, nsteps);
 }
 
 cudaError_t launch_unpack(cudaStream_t s, const Batch &B, const double *src, double *x, double *y, double *z,
@@ -495,29 +504,21 @@ cudaError_t launch_unpack_state(cudaStream_t s, const Batch &B, const double *sr
 }
 
 cudaError_t launch_pack_state(cudaStream_t s, const Batch &B, double *dr, double *dv, double *df, double *da,
-                              int64_t total_ba, const int *ba_traj) {
+                              double *dd, int64_t total_ba, const int *ba_traj) {
     const int grid = (int)std::min<int64_t>((total_ba + 255) / 256, 4096);
-    pack_state_kernel<<<grid > 0 ? grid : 1, 256, 0, s>>>(B, dr, dv, df, da, total_ba, ba_traj);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack_scalar(cudaStream_t s, const Batch &B, double *dst, const double *x, int64_t total_ba,
-                               const int *ba_traj) {
-    const int grid = (int)std::min<int64_t>((total_ba + 255) / 256, 4096);
-    pack_scalar_kernel<<<grid > 0 ? grid : 1, 256, 0, s>>>(B, dst, x, total_ba, ba_traj);
+    pack_state_kernel<<<grid > 0 ? grid : 1, 256, 0, s>>>(B, dr, dv, df, da, dd, total_ba, ba_traj);
     return cudaGetLastError();
 }
 
 int max_resident_ctas(int max_atoms, int max_beads, int precision) {
     const size_t sm = smem_bytes(max_atoms, max_beads, precision == 1 ? 4 : 8, emt_places(max_atoms, max_beads));
     int n = 0;
-    if (precision == 1) {
-        cudaFuncSetAttribute(md_steps_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, md_steps_kernel<float>, kBlock, sm);
-    } else {
-        cudaFuncSetAttribute(md_steps_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, md_steps_kernel<double>, kBlock, sm);
-    }
+    auto ask = [&](auto kernel) {
+        if (sm > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kBlock, sm);
+    };
+    if (precision == 1) ask(md_steps_kernel<float, kBlock>);
+    else ask(md_steps_kernel<double, kBlock>);
     return n > 0 ? n : 1;
 }
 
