@@ -217,7 +217,8 @@ template <typename R>
 __device__ void acsf_cache(const NNDev &M, const WarpCache<R> &C, int i, int ei, int cnt, const int *words,
                            const double *px, const double *py, const double *pz, const int8_t *elem, const double *L) {
     const int lane = threadIdx.x & 31;
-    const R rc = (R)M.rc[ei];
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R rc = ck.rc;
     const int ng = M.ng3eta[ei];
     for (int q = lane; q < cnt; q += 32) {
         const int w = words[q];
@@ -235,10 +236,10 @@ __device__ void acsf_cache(const NNDev &M, const WarpCache<R> &C, int i, int ei,
         e[2] = narrow<R>(dz);
         e[3] = r;
         R fc = R(0), dfc = R(0);
-        if (r <= rc) cutoff_fn<R>(M, rc, r, fc, dfc);
+        if (r <= rc) cutoff_fn<R>(M, ck, r, fc, dfc);
         e[4] = fc;
         e[5] = dfc;
-        for (int m = 0; m < ng; ++m) e[6 + m] = NM<R>::ex(-(R)M.g3eta[ei][m] * r * r);
+        for (int m = 0; m < ng; ++m) e[6 + m] = NM<R>::ex(-g3_eta<R>(M, ei, m) * r * r);
         C.nbatom[q] = j;
         C.nbelem[q] = elem[j];
         C.slotf[3 * q] = R(0);
@@ -267,13 +268,14 @@ __device__ __forceinline__ G3List g3_list(const NNDev &M, int ei) {
 template <typename R> struct Triplet {
     const R *a, *c;  // cache rows of j and k
     R jx, jy, jz;    // d_j - d_k = x_j - x_k
-    R rjk2, rjk, fcjk, dfcjk, rinv0, cost0, pfc;
+    R rjk2, rjk, ijk, fcjk, dfcjk, rinv0, cost0, pfc;  // (ijk = 1/rjk: grid form, FP64)
     R ejk[kMaxEta];
 };
 
 template <typename R>
-__device__ __forceinline__ bool triplet_setup(const NNDev &M, const WarpCache<R> &C, int ei, int q3, int q4, R rc,
-                                              Triplet<R> &T) {
+__device__ __forceinline__ bool triplet_setup(const NNDev &M, const WarpCache<R> &C, int ei, int q3, int q4,
+                                              const CutK<R> &ck, Triplet<R> &T) {
+    const R rc = ck.rc;
     T.a = C.nb + q3 * C.st;
     T.c = C.nb + q4 * C.st;
     if (!(T.a[3] <= rc && T.c[3] <= rc)) return false;
@@ -283,12 +285,12 @@ __device__ __forceinline__ bool triplet_setup(const NNDev &M, const WarpCache<R>
     T.rjk2 = T.jx * T.jx + T.jy * T.jy + T.jz * T.jz;
     if (!(T.rjk2 <= rc * rc)) return false;
     T.rjk = NM<R>::sq(T.rjk2);
-    cutoff_fn<R>(M, rc, T.rjk, T.fcjk, T.dfcjk);
+    cutoff_fn<R>(M, ck, T.rjk, T.fcjk, T.dfcjk);
     T.rinv0 = NM<R>::rc(T.a[3] * T.c[3]);
     T.cost0 = (T.a[0] * T.c[0] + T.a[1] * T.c[1] + T.a[2] * T.c[2]) * T.rinv0;
     T.pfc = T.a[4] * T.c[4] * T.fcjk;
     const int ng = M.ng3eta[ei];
-    for (int m = 0; m < ng; ++m) T.ejk[m] = NM<R>::ex(-(R)M.g3eta[ei][m] * T.rjk2);
+    for (int m = 0; m < ng; ++m) T.ejk[m] = NM<R>::ex(-g3_eta<R>(M, ei, m) * T.rjk2);
     return true;
 }
 
@@ -322,11 +324,12 @@ __device__ void acsf_g3_jvp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
 // ---- forward ------------------------------------------------------------------------
 template <typename R> __device__ void acsf_forward(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, R *G) {
     const int lane = threadIdx.x & 31;
-    const R rc = (R)M.rc[ei];
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R rc = ck.rc;
     const int nsf = M.nsf[ei], sfb = ei * M.maxsf;
     for (int s = 0; s < nsf; ++s) {
         if (M.sftype[sfb + s] != 2) continue;
-        const R eta = (R)M.eta[sfb + s], rs = (R)M.rs[sfb + s];
+        const R eta = sf_eta<R>(M, sfb + s), rs = sf_rs<R>(M, sfb + s);
         const int e1 = M.e1[sfb + s];
         R acc = R(0);
         for (int q = lane; q < cnt; q += 32) {
@@ -353,7 +356,7 @@ template <typename R> __device__ void acsf_forward(const NNDev &M, const WarpCac
     tw.init(cnt, lane);
     while (tw.valid) {
         Triplet<R> T;
-        if (triplet_setup<R>(M, C, ei, tw.q3, tw.q4, rc, T)) {
+        if (triplet_setup<R>(M, C, ei, tw.q3, tw.q4, ck, T)) {
             const int ej = C.nbelem[tw.q3], ek = C.nbelem[tw.q4];
 #pragma unroll
             for (int u = 0; u < kMaxG3; ++u) {
@@ -380,7 +383,8 @@ template <typename R>
 __device__ void acsf_vjp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix, R &fiy,
                          R &fiz) {
     const int lane = threadIdx.x & 31;
-    const R rc = (R)M.rc[ei];
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R rc = ck.rc;
     const int nsf = M.nsf[ei], sfb = ei * M.maxsf;
     fix = fiy = fiz = R(0);
     for (int q = lane; q < cnt; q += 32) {
@@ -389,7 +393,7 @@ __device__ void acsf_vjp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
         R dsum = R(0);
         for (int s = 0; s < nsf; ++s) {
             if (M.sftype[sfb + s] != 2 || C.nbelem[q] != M.e1[sfb + s]) continue;
-            const R eta = (R)M.eta[sfb + s], rs = (R)M.rs[sfb + s];
+            const R eta = sf_eta<R>(M, sfb + s), rs = sf_rs<R>(M, sfb + s);
             const R ex = NM<R>::ex(-eta * (e[3] - rs) * (e[3] - rs));
             dsum += c[s] * (R(-2) * eta * (e[3] - rs) * ex * e[4] + ex * e[5]);
         }
@@ -415,7 +419,7 @@ __device__ void acsf_vjp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
     tw.init(cnt, lane);
     while (tw.valid) {
         Triplet<R> T;
-        if (triplet_setup<R>(M, C, ei, tw.q3, tw.q4, rc, T)) {
+        if (triplet_setup<R>(M, C, ei, tw.q3, tw.q4, ck, T)) {
             const int ej = C.nbelem[tw.q3], ek = C.nbelem[tw.q4];
             R A1 = R(0), A2 = R(0), A3 = R(0);
             for (int u = 0; u < g3.n; ++u) {
@@ -425,7 +429,7 @@ __device__ void acsf_vjp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
                 if (!g3_term<R>(M, k, T, plam, fgn)) continue;
                 const R us = c[s] * fgn;
                 A1 += us * (R)(M.zeta[k] * M.lam[k]);
-                A2 += us * (R)M.eta[k] * plam;
+                A2 += us * sf_eta<R>(M, k) * plam;
                 A3 += us * plam;
             }
             const R rij = T.a[3], rik = T.c[3];
@@ -459,13 +463,14 @@ template <typename R>
 __device__ void acsf_jvp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, int i, const R *ux, const R *uy,
                          const R *uz, R *v) {
     const int lane = threadIdx.x & 31;
-    const R rc = (R)M.rc[ei];
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R rc = ck.rc;
     const int nsf = M.nsf[ei], sfb = ei * M.maxsf;
     const R uix = ux[i], uiy = uy[i], uiz = uz[i];
     // G2: -dG/dx_i = (d/r) T', -dG/dx_j = -(d/r) T'  ->  v += T'/r d.(u_i - u_j)
     for (int s = 0; s < nsf; ++s) {
         if (M.sftype[sfb + s] != 2) continue;
-        const R eta = (R)M.eta[sfb + s], rs = (R)M.rs[sfb + s];
+        const R eta = sf_eta<R>(M, sfb + s), rs = sf_rs<R>(M, sfb + s);
         const int e1 = M.e1[sfb + s];
         R acc = R(0);
         for (int q = lane; q < cnt; q += 32) {
@@ -495,7 +500,7 @@ __device__ void acsf_jvp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
     tw.init(cnt, lane);
     while (tw.valid) {
         Triplet<R> T;
-        if (triplet_setup<R>(M, C, ei, tw.q3, tw.q4, rc, T)) {
+        if (triplet_setup<R>(M, C, ei, tw.q3, tw.q4, ck, T)) {
             const int ej = C.nbelem[tw.q3], ek = C.nbelem[tw.q4];
             const int j = C.nbatom[tw.q3], kk = C.nbatom[tw.q4];
             // q1 = dxij.(u_i-u_j), q2 = dxik.(u_i-u_k), q3 = dxjk.(u_k-u_j)
@@ -513,7 +518,7 @@ __device__ void acsf_jvp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
                 if (!g3_match(M, k, ej, ek)) continue;
                 R plam, fgn;
                 if (!g3_term<R>(M, k, T, plam, fgn)) continue;
-                const R zl = (R)(M.zeta[k] * M.lam[k]), e2 = R(2) * (R)M.eta[k] * plam * T.pfc;
+                const R zl = (R)(M.zeta[k] * M.lam[k]), e2 = R(2) * sf_eta<R>(M, k) * plam * T.pfc;
                 const R p1 = fgn * (b1 * zl - e2 + d1 * plam);
                 const R p2 = fgn * (b2 * zl - e2 + d2 * plam);
                 const R p3 = fgn * (T.pfc * T.rinv0 * zl + e2 - d3 * plam);
@@ -545,8 +550,9 @@ __device__ __forceinline__ bool fast_pair(const NNDev &M, int ei, int ej, int ek
 
 // geometry of a triplet without the per-eta exponentials (computed by the caller)
 template <typename R>
-__device__ __forceinline__ bool triplet_geom(const NNDev &M, const WarpCache<R> &C, int q3, int q4, R rc,
-                                             Triplet<R> &T) {
+__device__ __forceinline__ bool triplet_geom(const NNDev &M, const WarpCache<R> &C, int q3, int q4,
+                                             const CutK<R> &ck, Triplet<R> &T) {
+    const R rc = ck.rc;
     T.a = C.nb + q3 * C.st;
     T.c = C.nb + q4 * C.st;
     if (!(T.a[3] <= rc && T.c[3] <= rc)) return false;
@@ -555,8 +561,13 @@ __device__ __forceinline__ bool triplet_geom(const NNDev &M, const WarpCache<R> 
     T.jz = T.a[2] - T.c[2];
     T.rjk2 = T.jx * T.jx + T.jy * T.jy + T.jz * T.jz;
     if (!(T.rjk2 <= rc * rc)) return false;
-    T.rjk = NM<R>::sq(T.rjk2);
-    cutoff_fn<R>(M, rc, T.rjk, T.fcjk, T.dfcjk);
+    if constexpr (sizeof(R) == 8) {
+        T.ijk = rsqrt_nr(T.rjk2);
+        T.rjk = T.rjk2 * T.ijk;
+    } else {
+        T.rjk = NM<R>::sq(T.rjk2);
+    }
+    cutoff_fn<R>(M, ck, T.rjk, T.fcjk, T.dfcjk);
     T.rinv0 = NM<R>::rc(T.a[3] * T.c[3]);
     T.cost0 = (T.a[0] * T.c[0] + T.a[1] * T.c[1] + T.a[2] * T.c[2]) * T.rinv0;
     T.pfc = T.a[4] * T.c[4] * T.fcjk;
@@ -610,13 +621,13 @@ template <typename R> __device__ __forceinline__ GridConst<R> grid_const(const N
     g.nq = M.nlz[ei];
 #pragma unroll
     for (int q = 0; q < kGQ; ++q) {
-        g.lam[q] = (R)M.lz_lam[ei][q];
-        g.zl[q] = (R)M.lz_zl[ei][q];
-        g.pn[q] = (R)M.lz_pnorm[ei][q];
+        g.lam[q] = widen<R>(M.lz_lam[ei][q]);
+        g.zl[q] = widen<R>(M.lz_zl[ei][q]);
+        g.pn[q] = widen<R>(M.lz_pnorm[ei][q]);
         g.zm1[q] = M.lz_zm1[ei][q];
     }
 #pragma unroll
-    for (int m = 0; m < kGM; ++m) g.eta[m] = (R)(m < g.ng ? M.g3eta[ei][m] : 0.0);
+    for (int m = 0; m < kGM; ++m) g.eta[m] = m < g.ng ? g3_eta<R>(M, ei, m) : R(0);
     g.nl = 0;
     g.lams[0] = g.lams[1] = R(0);
 #pragma unroll
@@ -640,7 +651,8 @@ __device__ __forceinline__ void grid_pexp(const GridConst<R> &g, const Triplet<R
 template <typename R> __device__ void acsf_g3_forward_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
                                                            R *G) {
     const int lane = threadIdx.x & 31;
-    const R rc = (R)M.rc[ei];
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R rc = ck.rc;
     const GridConst<R> g = grid_const<R>(M, ei);
     R acc[kGM][kGQ];
 #pragma unroll
@@ -651,7 +663,7 @@ template <typename R> __device__ void acsf_g3_forward_fast(const NNDev &M, const
     tw.init(cnt, lane);
     while (tw.valid) {
         Triplet<R> T;
-        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, rc, T)) {
+        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
             R E[kGM];
             grid_pexp<R>(g, T, E);
 #pragma unroll
@@ -687,7 +699,8 @@ template <typename R>
 __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix, R &fiy,
                                  R &fiz) {
     const int lane = threadIdx.x & 31;
-    const R rc = (R)M.rc[ei];
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R rc = ck.rc;
     const GridConst<R> g = grid_const<R>(M, ei);
     R Wc[kGM][kGQ];
 #pragma unroll
@@ -702,7 +715,7 @@ __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
     tw.init(cnt, lane);
     while (tw.valid) {
         Triplet<R> T;
-        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, rc, T)) {
+        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
             R E[kGM];
             grid_pexp<R>(g, T, E);
             Ladder<R> L;
@@ -730,7 +743,7 @@ __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
             R P1, P2, P3;
             if constexpr (sizeof(R) == 8) {
                 // 1/r_ij = r_ik/(r_ij r_ik) and so on: products for the five divisions
-                const R iij = T.rinv0 * rik, iik = T.rinv0 * rij, ijk = NM<R>::rc(T.rjk), w = R(2) * T.pfc * A2;
+                const R iij = T.rinv0 * rik, iik = T.rinv0 * rij, ijk = T.ijk, w = R(2) * T.pfc * A2;
                 P1 = T.pfc * (T.rinv0 - T.cost0 * (iij * iij)) * A1 - w + T.c[4] * T.fcjk * T.a[5] * iij * A3;
                 P2 = T.pfc * (T.rinv0 - T.cost0 * (iik * iik)) * A1 - w + T.a[4] * T.fcjk * T.c[5] * iik * A3;
                 P3 = T.pfc * T.rinv0 * A1 + w - T.a[4] * T.c[4] * T.dfcjk * ijk * A3;
@@ -766,7 +779,8 @@ template <typename R>
 __device__ void acsf_g3_jvp_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, int i, const R *ux,
                                  const R *uy, const R *uz, R *v) {
     const int lane = threadIdx.x & 31;
-    const R rc = (R)M.rc[ei];
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R rc = ck.rc;
     const GridConst<R> g = grid_const<R>(M, ei);
     const R uix = ux[i], uiy = uy[i], uiz = uz[i];
     R acc[kGM][kGQ];
@@ -778,7 +792,7 @@ __device__ void acsf_g3_jvp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
     tw.init(cnt, lane);
     while (tw.valid) {
         Triplet<R> T;
-        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, rc, T)) {
+        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
             const int j = C.nbatom[tw.q3], kk = C.nbatom[tw.q4];
             const R q1 = -(T.a[0] * (uix - ux[j]) + T.a[1] * (uiy - uy[j]) + T.a[2] * (uiz - uz[j]));
             const R q2 = -(T.c[0] * (uix - ux[kk]) + T.c[1] * (uiy - uy[kk]) + T.c[2] * (uiz - uz[kk]));

@@ -1670,6 +1670,12 @@ int32_t mdt_nn_set_model(mdt_ctx *c, const mdt_nn_model *m, int32_t ntypes, cons
         }
         if (ng3 > 24) return fail(c, MDT_ERR_UNSUPPORTED, "more than 24 G3 functions per element");
         M.ng3eta[e] = ng;
+        for (int q = 0; q < ng; ++q) M.g3etaf[e][q] = (float)M.g3eta[e][q];
+        M.rci[e] = M.cutoff_alpha * M.rc[e];
+        M.icw[e] = 1.0 / (M.rc[e] - M.rci[e]);
+        M.rcf[e] = (float)M.rc[e];
+        M.rcif[e] = (float)M.cutoff_alpha * M.rcf[e];
+        M.icwf[e] = 1.f / (M.rcf[e] - M.rcif[e]);
         ngmax = std::max(ngmax, ng);
         M.maxcut = std::max(M.maxcut, M.rc[e]);
         int off = 0;
@@ -1750,6 +1756,9 @@ int32_t mdt_nn_set_model(mdt_ctx *c, const mdt_nn_model *m, int32_t ntypes, cons
     M.izeta = (const int *)up(izeta.data(), 4 * nk);
     M.etaslot = (const int *)up(etaslot.data(), 4 * nk);
     M.eta = (const double *)up(m->eta, 8 * nk);
+    std::vector<float> ef(m->eta, m->eta + nk), rf(m->rshift, m->rshift + nk);
+    M.etaf = (const float *)up(ef.data(), 4 * nk);
+    M.rsf = (const float *)up(rf.data(), 4 * nk);
     M.rs = (const double *)up(m->rshift, 8 * nk);
     M.lam = (const double *)up(m->lambda, 8 * nk);
     M.zeta = (const double *)up(m->zeta, 8 * nk);

@@ -37,6 +37,11 @@ struct NNDev {
     int scalesym, centersym, normnodes, remove_atom_energies;
     double scmin, scmax;
     double rc[kMaxElem];          // cutoff shared by all symmetry functions of an element (bohr)
+    double rci[kMaxElem], icw[kMaxElem];  // inner cutoff alpha rc and 1/(rc - rci)
+    // the same and the G3 etas in FP32, for the FP32 walks (converted in the kernel, the compiler
+    // repeats the conversions, FP64-pipe slots, per triplet)
+    float rcf[kMaxElem], rcif[kMaxElem], icwf[kMaxElem], g3etaf[kMaxElem][6];
+    const float *etaf, *rsf;      // eta and rs, FP32 copies
     double maxcut;                // neighbour-list cutoff (bohr)
     int ng3eta[kMaxElem];
     double g3eta[kMaxElem][kMaxEta];
@@ -219,10 +224,35 @@ template <> struct NM<float> {
     static __device__ __forceinline__ const float *w(const NNDev &M) { return M.wf; }
 };
 
+// constants of element e in the walk's type
+template <typename R> struct CutK {
+    R rc, rci, iw;
+};
+template <typename R> __device__ __forceinline__ CutK<R> cut_k(const NNDev &M, int e) {
+    if constexpr (sizeof(R) == 4) return CutK<R>{M.rcf[e], M.rcif[e], M.icwf[e]};
+    else return CutK<R>{M.rc[e], M.rci[e], M.icw[e]};
+}
+template <typename R> __device__ __forceinline__ R g3_eta(const NNDev &M, int e, int m) {
+    if constexpr (sizeof(R) == 4) return M.g3etaf[e][m];
+    else return M.g3eta[e][m];
+}
+template <typename R> __device__ __forceinline__ R sf_eta(const NNDev &M, int k) {
+    if constexpr (sizeof(R) == 4) return M.etaf[k];
+    else return M.eta[k];
+}
+template <typename R> __device__ __forceinline__ R sf_rs(const NNDev &M, int k) {
+    if constexpr (sizeof(R) == 4) return M.rsf[k];
+    else return M.rs[k];
+}
+template <typename R> __device__ __forceinline__ R widen(float x) {
+    if constexpr (sizeof(R) == 4) return x;
+    else return f64_of(x);
+}
+
 // cutoff function and derivative, RuNNer_src/getcutoff.f90:51-162
 template <typename R>
-__device__ __forceinline__ void cutoff_fn(const NNDev &M, R rc, R r, R &fc, R &dfc) {
-    const R rci = (R)M.cutoff_alpha * rc, iw = R(1) / (rc - rci);
+__device__ __forceinline__ void cutoff_fn(const NNDev &M, const CutK<R> &ck, R r, R &fc, R &dfc) {
+    const R rc = ck.rc, rci = ck.rci, iw = ck.iw;
     const int type = M.cutoff_type;
     if (type == 0) { fc = R(1); dfc = R(0); return; }
     if (type == 1) {
