@@ -648,8 +648,157 @@ __device__ __forceinline__ void grid_pexp(const GridConst<R> &g, const Triplet<R
     for (int m = 0; m < kGM; ++m) E[m] = (m < g.ng) ? T.a[6 + m] * T.c[6 + m] * NM<R>::ex(-g.eta[m] * T.rjk2) : R(0);
 }
 
+// forces of one triplet from its A1, A2, A3 (head of this file): on the centre, the row's neighbour
+// and the neighbour q4
+template <typename R>
+__device__ __forceinline__ void vjp_pairs(const Triplet<R> &T, R A1, R A2, R A3, const WarpCache<R> &C, int q4, R &fix,
+                                          R &fiy, R &fiz, R &sjx, R &sjy, R &sjz) {
+    const R rij = T.a[3], rik = T.c[3];
+    R P1, P2, P3;
+    if constexpr (sizeof(R) == 8) {
+        // 1/r_ij = r_ik/(r_ij r_ik) and so on: products for the five divisions
+        const R iij = T.rinv0 * rik, iik = T.rinv0 * rij, ijk = T.ijk, w = R(2) * T.pfc * A2;
+        P1 = T.pfc * (T.rinv0 - T.cost0 * (iij * iij)) * A1 - w + T.c[4] * T.fcjk * T.a[5] * iij * A3;
+        P2 = T.pfc * (T.rinv0 - T.cost0 * (iik * iik)) * A1 - w + T.a[4] * T.fcjk * T.c[5] * iik * A3;
+        P3 = T.pfc * T.rinv0 * A1 + w - T.a[4] * T.c[4] * T.dfcjk * ijk * A3;
+    } else {
+        P1 = T.pfc * (T.rinv0 - T.cost0 / (rij * rij)) * A1 - R(2) * T.pfc * A2 +
+             T.c[4] * T.fcjk * T.a[5] / rij * A3;
+        P2 = T.pfc * (T.rinv0 - T.cost0 / (rik * rik)) * A1 - R(2) * T.pfc * A2 +
+             T.a[4] * T.fcjk * T.c[5] / rik * A3;
+        P3 = T.pfc * T.rinv0 * A1 + R(2) * T.pfc * A2 - T.a[4] * T.c[4] * T.dfcjk / T.rjk * A3;
+    }
+    fix += T.a[0] * P1 + T.c[0] * P2;
+    fiy += T.a[1] * P1 + T.c[1] * P2;
+    fiz += T.a[2] * P1 + T.c[2] * P2;
+    sjx += -T.a[0] * P1 + T.jx * P3;
+    sjy += -T.a[1] * P1 + T.jy * P3;
+    sjz += -T.a[2] * P1 + T.jz * P3;
+    atomicAdd(&C.slotf[3 * q4], -T.c[0] * P2 - T.jx * P3);
+    atomicAdd(&C.slotf[3 * q4 + 1], -T.c[1] * P2 - T.jy * P3);
+    atomicAdd(&C.slotf[3 * q4 + 2], -T.c[2] * P2 - T.jz * P3);
+}
+
+// The set of the benchmark networks (NNDev::g3std): three etas, zeta 1, 4 and 16, lambda -1 and +1.
+// The same walks with the cells fixed at compile time: (1 + lambda cos)^(zeta-1) is a product of
+// the squares p, p^2, p^4, p^8 taken once per lambda (the general walk multiplies five factors per
+// cell), nothing is indexed at run time (the general walk keeps its ladder in local memory), and the
+// sums run in the general walk's order.
+template <typename R> struct StdCells {
+    R p[2], pp[2][3];  // 1 + lambda cos; its powers zeta - 1 (all zero where 1 + lambda cos <= 0)
+    __device__ __forceinline__ StdCells(R cost) {
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            p[l] = R(1) + R(l ? 1 : -1) * cost;
+            const bool on = p[l] > R(0);
+            const R p2 = p[l] * p[l], p4 = p2 * p2, p8 = p4 * p4, a = p[l] * p2;
+            pp[l][0] = on ? R(1) : R(0);
+            pp[l][1] = on ? a : R(0);
+            pp[l][2] = on ? a * p4 * p8 : R(0);
+        }
+    }
+};
+
+template <typename R> __device__ __forceinline__ void std_pexp(const R *eta, const Triplet<R> &T, R *E) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) E[m] = T.a[6 + m] * T.c[6 + m] * NM<R>::ex(-eta[m] * T.rjk2);
+}
+
+template <typename R>
+__device__ void acsf_g3_forward_std(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, R *G) {
+    const int lane = threadIdx.x & 31;
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R eta[3] = {g3_eta<R>(M, ei, 0), g3_eta<R>(M, ei, 1), g3_eta<R>(M, ei, 2)};
+    R acc[3][6];
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) acc[m][q] = R(0);
+    RowWalk tw;
+    tw.init(cnt, lane);
+    while (tw.valid) {
+        Triplet<R> T;
+        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
+            R E[3];
+            std_pexp<R>(eta, T, E);
+            const StdCells<R> L(T.cost0);
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const R pw = L.pp[q & 1][q >> 1] * L.p[q & 1];
+#pragma unroll
+                for (int m = 0; m < 3; ++m) acc[m][q] += E[m] * T.pfc * pw;
+            }
+        }
+        tw.next();
+    }
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const R v = warp_sum(acc[m][q]);
+            const int s = M.sf_of[ei][m][q];
+            if (lane == 0 && s >= 0) G[s] = v * (q < 2 ? R(1) : q < 4 ? R(0.125) : R(1.0 / 32768.0));
+        }
+    __syncwarp();
+}
+
+template <typename R>
+__device__ void acsf_g3_vjp_std(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix, R &fiy,
+                                R &fiz) {
+    const int lane = threadIdx.x & 31;
+    const CutK<R> ck = cut_k<R>(M, ei);
+    const R eta[3] = {g3_eta<R>(M, ei, 0), g3_eta<R>(M, ei, 1), g3_eta<R>(M, ei, 2)};
+    R Wc[3][6];
+#pragma unroll
+    for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const int s = M.sf_of[ei][m][q];
+            Wc[m][q] = s >= 0 ? c[s] * (q < 2 ? R(1) : q < 4 ? R(0.125) : R(1.0 / 32768.0)) : R(0);
+        }
+    R sjx = R(0), sjy = R(0), sjz = R(0);  // force on the current row's neighbour q3
+    RowWalk tw;
+    tw.init(cnt, lane);
+    while (tw.valid) {
+        Triplet<R> T;
+        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
+            R E[3];
+            std_pexp<R>(eta, T, E);
+            const StdCells<R> L(T.cost0);
+            R A1 = R(0), A2 = R(0), A3 = R(0);
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const R plam = L.p[q & 1], pp = L.pp[q & 1][q >> 1];
+                const R zl = R((q & 1 ? 1 : -1) * (q < 2 ? 1 : q < 4 ? 4 : 16));
+                R S = R(0), Tq = R(0);
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    const R w = Wc[m][q] * E[m];
+                    S += w;
+                    Tq += eta[m] * w;
+                }
+                A1 += zl * pp * S;
+                A2 += plam * pp * Tq;
+                A3 += plam * pp * S;
+            }
+            vjp_pairs<R>(T, A1, A2, A3, C, tw.q4, fix, fiy, fiz, sjx, sjy, sjz);
+        }
+        if (tw.row_end) {
+            atomicAdd(&C.slotf[3 * tw.q3], sjx);
+            atomicAdd(&C.slotf[3 * tw.q3 + 1], sjy);
+            atomicAdd(&C.slotf[3 * tw.q3 + 2], sjz);
+            sjx = sjy = sjz = R(0);
+        }
+        tw.next();
+    }
+}
+
 template <typename R> __device__ void acsf_g3_forward_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
                                                            R *G) {
+    if (M.g3std[ei]) {
+        acsf_g3_forward_std<R>(M, C, ei, cnt, G);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const CutK<R> ck = cut_k<R>(M, ei);
     const R rc = ck.rc;
@@ -698,6 +847,10 @@ template <typename R> __device__ void acsf_g3_forward_fast(const NNDev &M, const
 template <typename R>
 __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix, R &fiy,
                                  R &fiz) {
+    if (M.g3std[ei]) {
+        acsf_g3_vjp_std<R>(M, C, ei, cnt, c, fix, fiy, fiz);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const CutK<R> ck = cut_k<R>(M, ei);
     const R rc = ck.rc;
@@ -739,30 +892,7 @@ __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
                 A2 += plam * pp * Tq;
                 A3 += plam * pp * S;
             }
-            const R rij = T.a[3], rik = T.c[3];
-            R P1, P2, P3;
-            if constexpr (sizeof(R) == 8) {
-                // 1/r_ij = r_ik/(r_ij r_ik) and so on: products for the five divisions
-                const R iij = T.rinv0 * rik, iik = T.rinv0 * rij, ijk = T.ijk, w = R(2) * T.pfc * A2;
-                P1 = T.pfc * (T.rinv0 - T.cost0 * (iij * iij)) * A1 - w + T.c[4] * T.fcjk * T.a[5] * iij * A3;
-                P2 = T.pfc * (T.rinv0 - T.cost0 * (iik * iik)) * A1 - w + T.a[4] * T.fcjk * T.c[5] * iik * A3;
-                P3 = T.pfc * T.rinv0 * A1 + w - T.a[4] * T.c[4] * T.dfcjk * ijk * A3;
-            } else {
-                P1 = T.pfc * (T.rinv0 - T.cost0 / (rij * rij)) * A1 - R(2) * T.pfc * A2 +
-                     T.c[4] * T.fcjk * T.a[5] / rij * A3;
-                P2 = T.pfc * (T.rinv0 - T.cost0 / (rik * rik)) * A1 - R(2) * T.pfc * A2 +
-                     T.a[4] * T.fcjk * T.c[5] / rik * A3;
-                P3 = T.pfc * T.rinv0 * A1 + R(2) * T.pfc * A2 - T.a[4] * T.c[4] * T.dfcjk / T.rjk * A3;
-            }
-            fix += T.a[0] * P1 + T.c[0] * P2;
-            fiy += T.a[1] * P1 + T.c[1] * P2;
-            fiz += T.a[2] * P1 + T.c[2] * P2;
-            sjx += -T.a[0] * P1 + T.jx * P3;
-            sjy += -T.a[1] * P1 + T.jy * P3;
-            sjz += -T.a[2] * P1 + T.jz * P3;
-            atomicAdd(&C.slotf[3 * tw.q4], -T.c[0] * P2 - T.jx * P3);
-            atomicAdd(&C.slotf[3 * tw.q4 + 1], -T.c[1] * P2 - T.jy * P3);
-            atomicAdd(&C.slotf[3 * tw.q4 + 2], -T.c[2] * P2 - T.jz * P3);
+            vjp_pairs<R>(T, A1, A2, A3, C, tw.q4, fix, fiy, fiz, sjx, sjy, sjz);
         }
         if (tw.row_end) {
             atomicAdd(&C.slotf[3 * tw.q3], sjx);

@@ -1724,6 +1724,10 @@ int32_t mdt_nn_set_model(mdt_ctx *c, const mdt_nn_model *m, int32_t ntypes, cons
             M.nlz[e] = nq;
             M.g3pair[e][0] = pe1;
             M.g3pair[e][1] = pe2;
+            const int zm1[3] = {0, 3, 15};
+            M.g3std[e] = nq == 6 && M.ng3eta[e] == 3;
+            for (int q = 0; q < nq && M.g3std[e]; ++q)
+                M.g3std[e] = M.lz_zm1[e][q] == zm1[q >> 1] && M.lz_lam[e][q] == (q & 1 ? 1.f : -1.f);
         }
     }
     std::vector<uint8_t> act((size_t)ne * kMaxLayers * kMaxNodes, 'l');

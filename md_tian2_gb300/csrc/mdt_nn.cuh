@@ -65,6 +65,7 @@ struct NNDev {
     int lz_zm1[kMaxElem][8];             // zeta - 1 (integer)
     int8_t sf_of[kMaxElem][4][8];        // symmetry-function index of cell (m, q), -1 if none
     int g3pair[kMaxElem][2];             // the shared neighbour-element pair
+    int g3std[kMaxElem];                 // 1: three etas, cells (zeta 1, 4, 16) x (lambda -1, +1) in this order
 };
 
 // ---------------------------------------------------------------------------
