@@ -31,14 +31,13 @@ template <> struct Math<double> {
     static __device__ __forceinline__ double rsq(double x) { return rsqrt_nr(x); }
 };
 // FP32: the hardware approximations behind __expf and rsqrtf without their steps for denormal
-// operands (results below 2^-126 flush to zero), and a reciprocal of x in [1, 2^126) that rounds
-// as a division does
+// operands (results below 2^-126 flush to zero).  The reciprocal stays the correctly rounded one:
+// embedding and pair forces cancel to a hundredth, and a reciprocal one bit off in some pairs moved
+// the forces of the FP32 ring-polymer batch by 2.3e-5 instead of 1.2e-5 (relative; their FP32 error
+// is 1.8e-5).
 template <> struct Math<float> {
     static __device__ __forceinline__ float ex(float x) { return ex2a(x * kLog2eF); }
-    static __device__ __forceinline__ float rcp(float x) {
-        const float y = rcpa(x);
-        return fmaf(y, fmaf(-x, y, 1.f), y);
-    }
+    static __device__ __forceinline__ float rcp(float x) { return __frcp_rn(x); }
     static __device__ __forceinline__ float rsq(float x) {
         float y;
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -74,6 +73,9 @@ __host__ __device__ constexpr int emt_places(int max_atoms, int max_beads) {
     return max_atoms * max_beads <= 512 ? max_atoms * max_beads : max_atoms <= 512 ? 512 / max_atoms * max_atoms : max_atoms;
 }
 
+// the image-shift table, left out for large trajectories (whose shared memory may reach the limit)
+__host__ __device__ constexpr size_t emt_img_bytes(int max_atoms) { return max_atoms <= 512 ? sizeof(double) * 81 : 0; }
+
 template <typename R>
 static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int max_beads, int places) {
     SmemEmt<R> s;
@@ -92,25 +94,27 @@ static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int 
     s.ph = (float4 *)take(nf);
     s.pl = (float4 *)take(nf);
     s.red = (double *)take(sizeof(double) * 64);
-    s.img = (double *)take(sizeof(double) * 81);
+    s.img = (double *)take(emt_img_bytes(max_atoms));
+    if (!emt_img_bytes(max_atoms)) s.img = nullptr;
     s.cjk = (double *)take(sizeof(double) * rp_cells(max_beads));
     s.sig = (R *)take(sizeof(R) * places);
     s.A = (R *)take(sizeof(R) * places);
     s.fx = (R *)take(sizeof(R) * places);
     s.fy = (R *)take(sizeof(R) * places);
     s.fz = (R *)take(sizeof(R) * places);
-    s.en = (double *)take(max_beads > 1 ? sizeof(double) * places : 0);
-    s.cell = (Cell *)take(256);
+    s.en = (double *)take(places > max_atoms ? sizeof(double) * places : 0);
+    unsigned char *const cell = take(256);
+    s.cell = (Cell *)cell;
+    s.seg = (int *)(cell + 224);
     s.perm = (int16_t *)take(sizeof(int16_t) * max_atoms);
-    s.seg = (int *)take(sizeof(int) * 6);
     return s;
 }
 
 inline size_t smem_bytes(int max_atoms, int max_beads, size_t rsize, int places) {
     auto r16 = [](size_t b) { return (b + 15) & ~size_t(15); };
-    return (rsize == 8 ? 3 * r16(8 * places) : 32 * (size_t)places) + r16(8 * 64) + r16(8 * 81) +
-           r16(8 * rp_cells(max_beads)) + 5 * r16(rsize * places) + (max_beads > 1 ? r16(8 * places) : 0) + 256 +
-           r16(2 * max_atoms) + 32;
+    return (rsize == 8 ? 3 * r16(8 * places) : 32 * (size_t)places) + r16(8 * 64) +
+           r16(emt_img_bytes(max_atoms)) + r16(8 * rp_cells(max_beads)) + 5 * r16(rsize * places) +
+           (places > max_atoms ? r16(8 * places) : 0) + 256 + r16(2 * max_atoms);
 }
 
 // Block-wide sum of a double; every thread gets the result.
@@ -150,7 +154,7 @@ struct Cell {
     float hif[9], hf[9];  // FP32 inverse and (FP32 bead forces) FP32 matrix
     unsigned nz;  // bit k set when h[k] != 0
 };
-static_assert(sizeof(Cell) <= 256, "the shared-memory carve reserves 256 bytes for the cell");
+static_assert(sizeof(Cell) <= 224, "the shared-memory carve reserves 224 bytes for the cell, 32 for the groups");
 
 // by the first warp of the CTA, nine lanes an entry each
 static __device__ __forceinline__ void load_cell(const Batch &B, int t, Cell &c) {
@@ -306,7 +310,7 @@ static __device__ __noinline__ double3 min_image_far(const Cell &c, double ex, d
 // first warp, after load_cell
 static __device__ __forceinline__ void image_table(const Cell &c, double *img) {
     const int k = threadIdx.x;
-    if (k >= 27) return;
+    if (k >= 27 || !img) return;
     const double n0 = k / 9 - 1, n1 = k / 3 % 3 - 1, n2 = k % 3 - 1;
     for (int d = 0; d < 3; ++d) img[3 * k + d] = fma(c.h[d], n0, fma(c.h[d + 3], n1, c.h[d + 6] * n2));
 }
@@ -343,7 +347,7 @@ template <> struct PlaceDiff<double> {
         dx = ex;
         dy = ey;
         dz = ez;
-        if (off < 0.4999f && big < 1.5f) {
+        if (off < 0.4999f && big < 1.5f && img) {
             const float kf = 9.f * n[0] + 3.f * n[1] + n[2];
             if (kf != 0.f) {
                 const double *v = img + 3 * ((int)kf + 13);

@@ -1,8 +1,8 @@
 // mdt_emt_plain.cuh -- EMT of one bead with FP64 forces in its short form: one walk over all pairs,
-// both ends added to shared memory.  The thread-per-atom kernel's fallback for a trajectory whose
+// both ends added to shared memory.  The FP32 network kernels' fallback for a trajectory whose
 // descriptors left the training range (a few in a million bead evaluations).  emt_beads
-// (mdt_emt.cuh) is 1.6 times faster, but inlined next to the walks of that kernel, which holds
-// all 128 registers a thread may have, it costs them spills: 79 -> 83 ms for 100 steps of the
+// (mdt_emt.cuh) is 1.6 times faster, but inlined next to the walks of those kernels, which hold
+// all 128 registers a thread may have, it costs spills there: 79 -> 83 ms for 100 steps of the
 // 4096-trajectory surrogate batch (as a call 88 ms), 76-77 ms with this form.
 //
 // Pair layout: pair (i, j = (i+k) mod N), k = 1..N/2, in scratch slot (k-1) N + i (the k = N/2

@@ -44,7 +44,7 @@
 #include <cstdio>
 
 #include "mdt_common.cuh"
-#include "mdt_emt.cuh"
+#include "mdt_emt_plain.cuh"
 #include "mdt_fastmath.cuh"
 #include "mdt_internal.h"
 #include "mdt_nn.cuh"
@@ -1234,7 +1234,7 @@ __device__ void nnf_calc_force(const Batch &B, const NNDev &M, const FastNN &F, 
     for (int b = 0; b < T.nb; ++b) {
         const bool flagged = nnf_bead<NG, ZM, G3ON>(B, M, F, X, S, L, T.t, b, do_forces, L.surrogate != 0);
         if (L.surrogate && flagged) {
-            emt_beads<double>(B, E, SE, T.t, b, 1, do_forces);
+            emt_bead_plain(B, E, SE, T.t, b, do_forces);
             if (threadIdx.x == 0) X.fallback[T.t] += 1;
         }
     }
