@@ -96,7 +96,7 @@ struct Batch {
     int *steps_done;           // per trajectory
     const int *cjk_off;        // per trajectory: offset of its nbeads x nbeads table
     const double *cjk;         // normal-mode tables, column major cjk(j,k)
-    void *pair_scratch;        // per pair slot: dx, dy, dz, Q_ij, Q_ji, F_V (FP64 or FP32)
+    void *pair_scratch;        // six values per pair slot (mdt_emt.cuh), FP64 or FP32
     // trajectory observables of trajectory_info.f90 (projectile = atom 0), updated by the
     // fused MD kernels after every step: turning points of the centroid's z velocity, 1
     // while it moves up, closest approach to any other atom (A, minimum image of the

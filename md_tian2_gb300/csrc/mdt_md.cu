@@ -2,17 +2,13 @@
 //
 // One CTA owns one trajectory (all its beads) at a time and pulls trajectories from a
 // work queue ordered largest-first.  Within a CTA:
-//   * the bead being evaluated is staged in shared memory (positions, accumulators);
-//   * unordered atom pairs are enumerated in a rectangular N x (N/2) layout (pair
-//     (i, (i+k) mod N), k = 1..N/2, the k = N/2 row halved for even N), so every thread
-//     gets the same amount of work without a square-root index decode;
-//   * EMT is evaluated in two pair passes around a per-atom epilogue: pass 1 builds the
-//     neutral-sphere densities and the pair-potential forces and leaves the pair's
-//     density-derivative scalars in a global scratch slot; the epilogue turns each
-//     atom's density into s_i, its energy, its embedded density and the coefficient
-//     A_i = (dE/ds_i) / (beta*eta2*sigma_i); pass 2 scatters (A_i Q_ij + A_j Q_ji) d_ij.
-//     This is the O(N^2)-time, O(N)-memory restatement of the reference's dense
-//     (3,nb,N,N) derivative tensors (src/pes_emt_mod.f90:483-1027).
+//   * the beads being evaluated are staged in shared memory by species (positions, accumulators);
+//   * EMT is evaluated in two pair passes around a per-atom epilogue (mdt_emt.cuh): the first sums
+//     the neutral-sphere densities, the epilogue turns each atom's density into s_i, its energy,
+//     its embedded density and A_i = (dE/ds_i) / (beta*eta2*sigma_i), the second forms the forces
+//     (A_i Q_ij + A_j Q_ji + F_V) d_ij.  This is the O(N^2)-time, O(N)-memory restatement of the
+//     reference's dense (3,nb,N,N) derivative tensors (src/pes_emt_mod.f90:483-1027);
+//   * ring polymers may be shared by the CTAs of a cluster (TrajView's rank and size).
 // The fused kernel runs propagate_1 -> calc_force -> propagate_2 for many steps
 // without leaving the CTA (md_tian2.f90:78-92).
 #include <cooperative_groups.h>
