@@ -177,15 +177,15 @@ static __device__ __noinline__ bool acsf_inside(double xi, double yi, double zi,
 static __device__ int acsf_neighbors_one(const NNDev &M, int i, int N, const double *px, const double *py,
                                          const double *pz, const double *L, int na, int nbi, int nc, int *out) {
     const double cut2 = __dmul_rn(M.maxcut, M.maxcut);
-    const float c2 = f32_of(cut2), cut2f_hi = c2 * 1.0001f, cut2f_lo = c2 * 0.9999f;
+    const float c2 = f32_screen(cut2), cut2f_hi = c2 * 1.0001f, cut2f_lo = c2 * 0.9999f;
     float Lf[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) Lf[k] = f32_of(L[k]);
+    for (int k = 0; k < 9; ++k) Lf[k] = f32_screen(L[k]);
     int cnt = 0;
     const double xi = px[i], yi = py[i], zi = pz[i];
     for (int j = 0; j < N; ++j) {
         const double xj = px[j], yj = py[j], zj = pz[j];
-        const float dx = f32_of(xj - xi), dy = f32_of(yj - yi), dz = f32_of(zj - zi);
+        const float dx = f32_screen(xj - xi), dy = f32_screen(yj - yi), dz = f32_screen(zj - zi);
         for (int n1 = -na; n1 <= na; ++n1)
             for (int n2 = -nbi; n2 <= nbi; ++n2) {
                 const float g1 = (float)n1, g2 = (float)n2;

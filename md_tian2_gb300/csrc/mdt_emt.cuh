@@ -18,7 +18,7 @@ constexpr int kWideBlock = 256;  // the same for batches of at most one trajecto
 //    which cubes the relative error: accurate to ~1 ulp;
 //  * conversions between FP64 and FP32 and FP64 comparisons run on the FP64 pipe too (measured
 //    55 and 64 cycles per warp, an FP64 multiply-add 64, an integer instruction 1-2), so the
-//    pair loops have none: floats are cut out of doubles by shifts (f32_of), ranges are tested
+//    pair loops have none: floats are cut out of doubles by shifts (f32_screen), ranges are tested
 //    on high words, image shifts come from a table of their 27 vectors;
 //  * the minimum-image shift (an integer per cell direction) is found in FP32 and
 //    applied in FP64; when FP32 cannot decide the rounding (fractional part within
@@ -335,7 +335,7 @@ template <> struct PlaceDiff<double> {
     template <typename S_>
     __device__ __forceinline__ void diff(const S_ &S, int j, int, double &dx, double &dy, double &dz) const {
         const double ex = x - S.px[j], ey = y - S.py[j], ez = z - S.pz[j];
-        const float fx = f32_of(ex), fy = f32_of(ey), fz = f32_of(ez);
+        const float fx = f32_screen(ex), fy = f32_screen(ey), fz = f32_screen(ez);
         float n[3], w[3];
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
@@ -728,9 +728,10 @@ static __device__ void emt_beads(const Batch &B, const EmtConst &E, const SmemEm
         const int64_t k = base + g0 + S.perm[p - g0];
         const double x = B.rx[k], y = B.ry[k], z = B.rz[k];
         if constexpr (sizeof(R) == 4) {
-            const float xh = f32_of(x), yh = f32_of(y), zh = f32_of(z);
-            S.ph[p] = make_float4(xh, yh, zh, 0.f);
-            S.pl[p] = make_float4(f32_of(x - f64_of(xh)), f32_of(y - f64_of(yh)), f32_of(z - f64_of(zh)), 0.f);
+            float hi[3], lo[3];
+            split3(x, y, z, hi, lo);
+            S.ph[p] = make_float4(hi[0], hi[1], hi[2], 0.f);
+            S.pl[p] = make_float4(lo[0], lo[1], lo[2], 0.f);
         } else {
             S.px[p] = x;
             S.py[p] = y;

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "mdt_common.cuh"
+#include "mdt_convert.h"
 #include "mdt_exp2tab.cuh"
 
 namespace mdt {
@@ -89,22 +90,15 @@ __device__ __forceinline__ void red_shared(float *p, float v) {
     asm volatile("red.shared.add.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 
-// (float)x by integer instructions, rounded to nearest (halves away from zero): the conversion
-// instruction runs on the FP64 pipe (55 cycles a warp against about 8 here).  |x| < 2^-126 gives
-// 0; |x| >= 2^127, infinities and NaN give NaN.
-static __device__ __forceinline__ float f32_of(double x) {
+// x in FP32 for range decisions (a screen whose undecided values go to FP64): to the nearest, halves
+// away from zero, |x| < 2^-126 as 0, |x| >= 2^127, infinities and NaN as infinity.  f32_of
+// (mdt_convert.h) without its rare branch, which the pair loops would carry three times.
+static __device__ __forceinline__ float f32_screen(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const unsigned e = hi & 0x7ff00000u;
     const unsigned m = ((__funnelshift_l(lo, hi, 3) ^ 0x40000000u) & 0x7fffffffu) + (lo >> 28 & 1u);
-    const unsigned v = e < 0x38100000u ? 0u : e >= 0x47e00000u ? 0x7fffffffu : m;
+    const unsigned v = e < 0x38100000u ? 0u : e >= 0x47e00000u ? 0x7f800000u : m;
     return __uint_as_float(v | (hi & 0x80000000u));
-}
-
-// (double)f of a float by integer instructions; |f| < 2^-126 gives 0, infinities and NaN give NaN.
-static __device__ __forceinline__ double f64_of(float f) {
-    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
-    const unsigned h = m < 0x00800000u ? 0u : m >= 0x7f800000u ? 0x7fffffffu : (m >> 3) + 0x38000000u;
-    return __hiloint2double((int)(h | (u & 0x80000000u)), m < 0x00800000u ? 0 : (int)(u << 29));
 }
 
 // exponent of the largest magnitudes: infinity or NaN (a FP64 comparison runs on the FP64 pipe)

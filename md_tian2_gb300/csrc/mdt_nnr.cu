@@ -1155,12 +1155,14 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                 const int64_t k = A.base + A.i;
                 const double rx = B.rx[k], ry = B.ry[k], rz = B.rz[k];
                 const double x = rx * kAng2BohrD, y = ry * kAng2BohrD, z = rz * kAng2BohrD;
-                A.xhi = f32_of(x);
-                A.yhi = f32_of(y);
-                A.zhi = f32_of(z);
-                A.xli = f32_of(x - f64_of(A.xhi));
-                A.yli = f32_of(y - f64_of(A.yhi));
-                A.zli = f32_of(z - f64_of(A.zhi));
+                float hi[3], lo[3];
+                split3(x, y, z, hi, lo);
+                A.xhi = hi[0];
+                A.yhi = hi[1];
+                A.zhi = hi[2];
+                A.xli = lo[0];
+                A.yli = lo[1];
+                A.zli = lo[2];
                 S.ph[tid] = make_float4(A.xhi, A.yhi, A.zhi, 0.f);
                 S.pl[tid] = make_float4(A.xli, A.yli, A.zli, 0.f);
                 if (mode == 2 && (not_finite(rx) || not_finite(ry) || not_finite(rz) || not_finite(B.vx[k]) ||
@@ -1168,7 +1170,8 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                     S.tr_bad[cur * kRMaxTraj + A.s] = 1;
                 if (R.skin > 0.f) {
                     const double *r0 = X.skref + 3 * k;
-                    const float ddx = f32_of(rx - r0[0]), ddy = f32_of(ry - r0[1]), ddz = f32_of(rz - r0[2]);
+                    // (a displacement that is no finite number counts as infinite: its list is rebuilt)
+                    const float ddx = f32_screen(rx - r0[0]), ddy = f32_screen(ry - r0[1]), ddz = f32_screen(rz - r0[2]);
                     atomicMax(&d2[A.s], __float_as_int(ddx * ddx + ddy * ddy + ddz * ddz));
                 }
             }

@@ -166,7 +166,7 @@ static __device__ double closest_approach_step(const Batch &B, const TrajView &T
         x = y = z = m = 0.f;
         for (int b = 0; b < T.nb; ++b) {
             const int64_t k = T.base + (int64_t)b * T.N + i;
-            const float a = f32_of(B.rx[k]), c = f32_of(B.ry[k]), d = f32_of(B.rz[k]);
+            const float a = f32_screen(B.rx[k]), c = f32_screen(B.ry[k]), d = f32_screen(B.rz[k]);
             x += a;
             y += c;
             z += d;
