@@ -52,8 +52,9 @@ template <typename R> struct SmemEmt {
     float4 *ph, *pl;       // FP32 forces (R = float): their FP32 hi/lo split
     R *sig, *A, *fx, *fy, *fz;
     Cell *cell;
-    double *en;            // per place: the bead's energies (several beads at a time)
+    double *en;            // per place: the bead's energies (several beads at a time; else null)
     int places;            // staged atoms the arrays hold (beads at a time x atoms)
+    size_t bytes;          // all of it
     int16_t *perm;         // atom of each place of a bead (places: species slot 0, slot 1, none)
     int *seg;              // first place of each of the three groups, N, runs per atom of slots 0 and 1
     double *red;           // 64 doubles for block reductions
@@ -67,17 +68,38 @@ __host__ __device__ constexpr size_t rp_cells(int max_beads) {
     return (size_t)max_beads * max_beads + 5 * (size_t)kMaxTypes * max_beads;
 }
 
-// staged atoms of the EMT kernels: the beads of a ring polymer are evaluated several at a time
-// (their per-atom FP64 work fills warps, and the CTA's barriers are shared), up to 512 atoms
-__host__ __device__ constexpr int emt_places(int max_atoms, int max_beads) {
-    return max_atoms * max_beads <= 512 ? max_atoms * max_beads : max_atoms <= 512 ? 512 / max_atoms * max_atoms : max_atoms;
+// Sizes of the EMT code's shared memory: what carve_smem lays out and smem_bytes adds up.
+struct EmtLayout {
+    int max_atoms, max_beads;
+    int places;     // staged atoms
+    bool together;  // beads several at a time: an energy per place
+    bool img;       // the image-shift table
+};
+
+// The EMT kernels evaluate the beads of a ring polymer several at a time (their per-atom FP64 work
+// fills warps, and the CTA's barriers are shared), up to 512 staged atoms: as many as fit, which is
+// more for the small trajectories of a batch than for its largest (emt_group).  Above 512 atoms one
+// at a time, and without the image table: there the positions and sums may reach the shared-memory limit.
+__host__ __device__ constexpr EmtLayout emt_layout(int max_atoms, int max_beads) {
+    return EmtLayout{max_atoms, max_beads,
+                     max_atoms * max_beads <= 512 ? max_atoms * max_beads
+                     : max_atoms <= 512           ? 512 / max_atoms * max_atoms
+                                                  : max_atoms,
+                     max_beads > 1 && max_atoms <= 512, max_atoms <= 512};
 }
 
-// the image-shift table, left out for large trajectories (whose shared memory may reach the limit)
-__host__ __device__ constexpr size_t emt_img_bytes(int max_atoms) { return max_atoms <= 512 ? sizeof(double) * 81 : 0; }
+// one bead at a time: the network kernels' fallback and the allocation-free call
+__host__ __device__ constexpr EmtLayout emt_layout_one(int max_atoms, int max_beads) {
+    return EmtLayout{max_atoms, max_beads, max_atoms, false, max_atoms <= 512};
+}
+
+// beads of an N-atom trajectory evaluated together, at most `per`
+__host__ __device__ constexpr int emt_group(int places, bool together, int N, int per) {
+    return !together ? 1 : per < places / N ? per : places / N;
+}
 
 template <typename R>
-static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int max_beads, int places) {
+static __host__ __device__ SmemEmt<R> carve_smem(unsigned char *base, const EmtLayout &L) {
     SmemEmt<R> s;
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -85,6 +107,7 @@ static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int 
         off += (bytes + 15) & ~size_t(15);
         return p;
     };
+    const int places = L.places;
     const int dp = sizeof(R) == 8 ? places : 0;  // FP64 forces: FP64 positions; FP32: their hi/lo split
     s.places = places;
     s.px = (double *)take(sizeof(double) * dp);
@@ -94,27 +117,27 @@ static __device__ SmemEmt<R> carve_smem(unsigned char *base, int max_atoms, int 
     s.ph = (float4 *)take(nf);
     s.pl = (float4 *)take(nf);
     s.red = (double *)take(sizeof(double) * 64);
-    s.img = (double *)take(emt_img_bytes(max_atoms));
-    if (!emt_img_bytes(max_atoms)) s.img = nullptr;
-    s.cjk = (double *)take(sizeof(double) * rp_cells(max_beads));
+    s.img = (double *)take(L.img ? sizeof(double) * 81 : 0);
+    if (!L.img) s.img = nullptr;
+    s.cjk = (double *)take(sizeof(double) * rp_cells(L.max_beads));
     s.sig = (R *)take(sizeof(R) * places);
     s.A = (R *)take(sizeof(R) * places);
     s.fx = (R *)take(sizeof(R) * places);
     s.fy = (R *)take(sizeof(R) * places);
     s.fz = (R *)take(sizeof(R) * places);
-    s.en = (double *)take(places > max_atoms ? sizeof(double) * places : 0);
+    s.en = (double *)take(L.together ? sizeof(double) * places : 0);
+    if (!L.together) s.en = nullptr;
     unsigned char *const cell = take(256);
     s.cell = (Cell *)cell;
     s.seg = (int *)(cell + 224);
-    s.perm = (int16_t *)take(sizeof(int16_t) * max_atoms);
+    s.perm = (int16_t *)take(sizeof(int16_t) * L.max_atoms);
+    s.bytes = off;
     return s;
 }
 
-inline size_t smem_bytes(int max_atoms, int max_beads, size_t rsize, int places) {
-    auto r16 = [](size_t b) { return (b + 15) & ~size_t(15); };
-    return (rsize == 8 ? 3 * r16(8 * places) : 32 * (size_t)places) + r16(8 * 64) +
-           r16(emt_img_bytes(max_atoms)) + r16(8 * rp_cells(max_beads)) + 5 * r16(rsize * places) +
-           (places > max_atoms ? r16(8 * places) : 0) + 256 + r16(2 * max_atoms);
+// (the layout from an address of no meaning, for its size)
+template <typename R> inline size_t smem_bytes(const EmtLayout &L) {
+    return carve_smem<R>(reinterpret_cast<unsigned char *>(uintptr_t(256)), L).bytes;
 }
 
 // Block-wide sum of a double; every thread gets the result.
@@ -365,7 +388,7 @@ template <> struct PlaceDiff<double> {
 };
 
 // ---------------------------------------------------------------------------
-// EMT for G beads (b0 ..) of one trajectory, G N <= S.places.  Adds forces into B.f* (stores them
+// EMT for G beads (b0 ..) of one trajectory, G <= emt_group.  Adds forces into B.f* (stores them
 // when `store`), sets dens, adds the beads' energies into B.epot.  Must be called by all threads
 // of the CTA.
 //

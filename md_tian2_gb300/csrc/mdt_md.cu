@@ -41,7 +41,7 @@ __device__ void calc_force(const Batch &B, const EmtConst &E, const PropParams &
     if (T.nb > 1) ring_polymer_step(B, P, T, S.cjk);
     // this CTA's beads, several at a time
     const int per = (T.nb + T.size - 1) / T.size, b0 = min(T.rank * per, T.nb), b1 = min(b0 + per, T.nb);
-    const int G = min(per, S.places / T.N);
+    const int G = emt_group(S.places, S.en != nullptr, T.N, per);
     for (int b = b0; b < b1; b += G) emt_beads<R>(B, E, S, T.t, b, min(G, b1 - b), do_forces, single);
     if (do_forces) set_acceleration(B, T, b0, b1);
     team_sync(T);
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) phase_kernel(Batch B, EmtConst E
                                                     int *counter, int phase) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
-    SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads, emt_places(B.max_atoms, B.max_beads));
+    SmemEmt<R> S = carve_smem<R>(smem_raw, emt_layout(B.max_atoms, B.max_beads));
     const int rank = cluster_rank(), size = cluster_size();
     for (;;) {
         const int w = next_work(counter, &work_slot, rank, size);
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) md_steps_kernel(Batch B, EmtCons
                                                        int *counter, int nsteps) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
-    SmemEmt<R> S = carve_smem<R>(smem_raw, B.max_atoms, B.max_beads, emt_places(B.max_atoms, B.max_beads));
+    SmemEmt<R> S = carve_smem<R>(smem_raw, emt_layout(B.max_atoms, B.max_beads));
     const int rank = cluster_rank(), size = cluster_size();
     for (;;) {
         const int w = next_work(counter, &work_slot, rank, size);
@@ -452,7 +452,7 @@ template <typename K> static cudaError_t prepare(const LaunchCfg &c, K kernel, s
 template <typename R, int NT>
 static cudaError_t launch_phase_t(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P,
                                   int phase) {
-    const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R), emt_places(B.max_atoms, B.max_beads));
+    const size_t sm = smem_bytes<R>(emt_layout(B.max_atoms, B.max_beads));
     const cudaError_t e = prepare(c, phase_kernel<R, NT>, sm);
     if (e != cudaSuccess) return e;
     return launch_team(c, phase_kernel<R, NT>, sm, B, E, P, c.order, c.counter, phase);
@@ -470,7 +470,7 @@ cudaError_t launch_phase(const LaunchCfg &c, const Batch &B, const EmtConst &E, 
 template <typename R, int NT>
 static cudaError_t launch_md_t(const LaunchCfg &c, const Batch &B, const EmtConst &E, const PropParams &P,
                                int nsteps) {
-    const size_t sm = smem_bytes(B.max_atoms, B.max_beads, sizeof(R), emt_places(B.max_atoms, B.max_beads));
+    const size_t sm = smem_bytes<R>(emt_layout(B.max_atoms, B.max_beads));
     const cudaError_t e = prepare(c, md_steps_kernel<R, NT>, sm);
     if (e != cudaSuccess) return e;
     return launch_team(c, md_steps_kernel<R, NT>, sm, B, E, P, c.order, c.counter, nsteps);
@@ -507,7 +507,8 @@ cudaError_t launch_pack_state(cudaStream_t s, const Batch &B, double *dr, double
 }
 
 int max_resident_ctas(int max_atoms, int max_beads, int precision) {
-    const size_t sm = smem_bytes(max_atoms, max_beads, precision == 1 ? 4 : 8, emt_places(max_atoms, max_beads));
+    const EmtLayout L = emt_layout(max_atoms, max_beads);
+    const size_t sm = precision == 1 ? smem_bytes<float>(L) : smem_bytes<double>(L);
     int n = 0;
     auto ask = [&](auto kernel) {
         if (sm > 47 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kNNBlock) nn_force_kernel(Batch B, NNDev M, Em
     SmemNN<R> S = carve_nn<R>(smem_raw, M, LN.max_atoms, LN.ngeta);
     SmemEmt<double> SE = carve_smem<double>(smem_raw + nn_smem_bytes(LN.max_atoms, M.maxnb, LN.ngeta, M.nelem,
                                                                      M.maxweights, sizeof(R)),
-                                            B.max_atoms, B.max_beads, B.max_atoms);
+                                            emt_layout_one(B.max_atoms, B.max_beads));
     load_weights_nn(M, S.w);
     for (;;) {
         if (threadIdx.x == 0) work_slot = atomicAdd(counter, 1);
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kNNBlock) nn_md_steps_kernel(Batch B, NNDev M,
     SmemNN<R> S = carve_nn<R>(smem_raw, M, LN.max_atoms, LN.ngeta);
     SmemEmt<double> SE = carve_smem<double>(smem_raw + nn_smem_bytes(LN.max_atoms, M.maxnb, LN.ngeta, M.nelem,
                                                                      M.maxweights, sizeof(R)),
-                                            B.max_atoms, B.max_beads, B.max_atoms);
+                                            emt_layout_one(B.max_atoms, B.max_beads));
     load_weights_nn(M, S.w);
     for (;;) {
         if (threadIdx.x == 0) work_slot = atomicAdd(counter, 1);
@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(kNNBlock) nn_md_steps_kernel(Batch B, NNDev M,
 
 size_t nn_total_smem(const NNDev &M, int max_atoms, int max_beads, int ngeta, int precision) {
     const size_t rs = precision == 1 ? 4 : 8;
-    return nn_smem_bytes(max_atoms, M.maxnb, ngeta, M.nelem, M.maxweights, rs) + smem_bytes(max_atoms, max_beads, 8, max_atoms);
+    return nn_smem_bytes(max_atoms, M.maxnb, ngeta, M.nelem, M.maxweights, rs) +
+           smem_bytes<double>(emt_layout_one(max_atoms, max_beads));
 }
 
 template <typename R, bool SURR>

@@ -173,7 +173,7 @@ FLaunch flaunch(const Batch &B, const NNDev &M, int surrogate) {
 size_t nnf_smem_total(const Batch &B, const NNDev &M, const FastNN &F) {
     const FLaunch L = flaunch(B, M, 0);
     const size_t wb = kFW * warp_bytes_f(L.maxnb, L.mw, M.nlayers, L.ls, L.sgs);
-    const size_t emt = smem_bytes(B.max_atoms, B.max_beads, 8, B.max_atoms);
+    const size_t emt = smem_bytes<double>(emt_layout_one(B.max_atoms, B.max_beads));
     return shared_bytes_f(B.max_atoms, B.max_beads, F.wtotal, M.nelem) + (wb > emt ? wb : emt);
 }
 
@@ -1280,7 +1280,7 @@ __global__ void __launch_bounds__(kFBlock, G3ON ? 2 : 3)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int work_slot;
     const SmemF S = carve_f(smem_raw, L, B.max_beads, F.wtotal, M.nelem, M.nlayers);
-    SmemEmt<double> SE = carve_smem<double>(S.warp_base, B.max_atoms, B.max_beads, B.max_atoms);
+    SmemEmt<double> SE = carve_smem<double>(S.warp_base, emt_layout_one(B.max_atoms, B.max_beads));
     SE.red = S.red;
     SE.cjk = S.cjk;
     load_model_smem(M, F, S);

@@ -1036,7 +1036,7 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
     constexpr int KT = KA + KB, bs = kRS;
     const int tid = threadIdx.x;
     const SmemR S = carve_r<KT, NH, TC>(smem_raw);
-    SmemEmt<double> SE = carve_smem<double>(S.emt, B.max_atoms, B.max_beads, B.max_atoms);
+    SmemEmt<double> SE = carve_smem<double>(S.emt, emt_layout_one(B.max_atoms, B.max_beads));
     SE.red = S.red;
     SE.cjk = S.red;  // single-bead trajectories only: the ring-polymer table is never read
     TcCtx C{0u, S.tcbar, X.tcerr};
@@ -1422,7 +1422,7 @@ size_t nnr_smem(const RadialNN &R) { return smem_r(R.nin, R.nh, R.tc); }
 
 size_t nnr_hb_bytes(const RadialNN &R) { return hb_bytes(R.nin, R.nh, R.tc); }
 
-size_t nnr_emt_smem(int max_atoms) { return smem_bytes(max_atoms, 1, 8, max_atoms); }
+size_t nnr_emt_smem(int max_atoms) { return smem_bytes<double>(emt_layout_one(max_atoms, 1)); }
 
 int nnr_resident_ctas(const RadialNN &R) {
     const size_t sm = nnr_smem(R);

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(kNoAllocBlock) emt_noalloc_kernel(int N, int n
     B.pair_scratch = scratch;
     B.max_atoms = N;
     B.max_beads = 1;
-    SmemEmt<double> S = carve_smem<double>(emt_base, N, 1, N);
+    SmemEmt<double> S = carve_smem<double>(emt_base, emt_layout_one(N, 1));
     emt_beads<double>(B, E, S, 0, 0, 1, true);
     if (threadIdx.x == 0 && s_bad) *energy = NAN;
 }
@@ -258,7 +258,7 @@ extern "C" int32_t mdt_emt_force_noalloc(int32_t natoms, const int32_t *idx, con
         }
         scratch = g_scratch_addr[dev];
     }
-    const size_t sm = ((natoms + 15) & ~15) + ((8 * (size_t)natoms + 15) & ~size_t(15)) + smem_bytes(natoms, 1, 8, natoms);
+    const size_t sm = ((natoms + 15) & ~15) + ((8 * (size_t)natoms + 15) & ~size_t(15)) + smem_bytes<double>(emt_layout_one(natoms, 1));
     emt_noalloc_kernel<<<1, kNoAllocBlock, sm, (cudaStream_t)stream>>>(natoms, ntypes, cell, E, x, y, z, idx, fx, fy, fz,
                                                                        energy, dens, scratch);
     return cudaGetLastError() == cudaSuccess ? MDT_OK : MDT_ERR_CUDA;
