@@ -103,7 +103,8 @@ struct mdt_ctx {
     float *g_dg = nullptr, *g_xdot = nullptr;
     double *g_eat = nullptr, *g_arow = nullptr;
     double lc_key[4] = {0, 0, 0, 0};  // (gamma, step, Tsurf, Tproj) they were formed for
-    bool lc_valid = false;
+    bool lc_valid = false;      // lcoef holds those of lc_key, written on this stream
+    bool lc_captured = false;   // a call of this batch was captured: a graph may rewrite lcoef
     int rmaxblock = kRBlockMax; // largest block the pack plan may use
     int *tcerr = nullptr;       // device word: a tensor-core GEMM of the network timed out
 
@@ -158,7 +159,7 @@ void free_batch(mdt_ctx *c) {
     c->rptraj = nullptr;
     c->rnpack = c->rblock = 0;
     c->lcoef = nullptr;
-    c->lc_valid = false;
+    c->lc_valid = c->lc_captured = false;
     c->tc_G = c->tc_eat = nullptr;
     c->tc_dg = nullptr;
     c->g_slot = nullptr;
@@ -238,18 +239,24 @@ PropParams to_dev(const mdt_ctx *c, const mdt_prop_params *p) {
 }
 
 // Constant-friction Langevin coefficients for the parameters of a propagation: they depend on
-// (gamma, dt, T) and the batch's masses, bead counts and propagators (fixed by mdt_batch_define),
-// so they are formed once per parameter set.
+// (gamma, dt, T) and the batch's masses, bead counts and propagators (fixed by mdt_batch_define).
+// The kernel that forms them is launched before the propagation that reads them, on its stream, and
+// left out only when the buffer certainly holds them: written by the last call on this stream for the
+// same parameters.  A call under stream capture records it (a replay forms its own coefficients, and
+// nothing ran yet), and from then on a replay may rewrite the buffer at any time, so every later
+// call of this batch launches it.
 int ensure_lcoef(mdt_ctx *c, const mdt_prop_params *p) {
-    bool need = false;
-    for (int t = 0; t < c->ntypes; ++t) need |= c->B.algo[t] == kPropLangevinConst;
+    if (!c->lcoef) return MDT_OK;  // no type with this propagator
     const double key[4] = {p->gamma_const, p->step, p->Tsurf, p->Tproj};
-    if (!need || (c->lcoef && c->lc_valid && std::memcmp(key, c->lc_key, sizeof(key)) == 0)) return MDT_OK;
-    cudaError_t e = cudaSuccess;
-    if (!c->lcoef) c->lcoef = dalloc<double>(c, 8 * (size_t)c->total_atoms, e);
-    if (!c->lcoef) return fail(c, MDT_ERR_NOMEM, "Langevin coefficient buffer");
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) {
+        cudaGetLastError();
+        st = cudaStreamCaptureStatusActive;  // not told: as if
+    }
+    if (st != cudaStreamCaptureStatusNone) c->lc_captured = true;
+    if (!c->lc_captured && c->lc_valid && std::memcmp(key, c->lc_key, sizeof(key)) == 0) return MDT_OK;
     c->lc_valid = false;
-    e = launch_lcoef(c->stream, c->B, to_dev(c, p), c->ba_traj, c->total_ba, c->lcoef);
+    const cudaError_t e = launch_lcoef(c->stream, c->B, to_dev(c, p), c->ba_traj, c->total_ba, c->lcoef);
     c->launches++;
     if (e != cudaSuccess) return cuda_fail(c, e, "Langevin coefficients");
     std::memcpy(c->lc_key, key, sizeof(key));
@@ -981,6 +988,7 @@ int32_t mdt_set_stream(mdt_ctx *c, void *s) {
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
         c->own_stream = true;
     }
+    c->lc_valid = false;
     return MDT_OK;
 }
 
@@ -1229,6 +1237,8 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
         if (e == cudaSuccess) e = cudaMemsetAsync(c->gen, 0, sizeof(int) * ((size_t)ntraj + 1), c->stream);
         c->refill_count = c->gen ? c->gen + ntraj : nullptr;
         if (e == cudaSuccess) c->draws = dalloc<double>(c, 5 * (size_t)ntraj, e);
+        const bool lc = std::find(algo, algo + ntypes, (int32_t)kPropLangevinConst) != algo + ntypes;
+        if (e == cudaSuccess && lc) c->lcoef = dalloc<double>(c, 8 * (size_t)at, e);
     }
     if (e != cudaSuccess) {
         free_batch(c);
