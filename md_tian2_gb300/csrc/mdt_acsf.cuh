@@ -228,8 +228,8 @@ __device__ void acsf_cache(const NNDev &M, const WarpCache<R> &C, int i, int ei,
         const double dx = px[j] + n1 * L[0] + n2 * L[3] + n3 * L[6] - px[i];
         const double dy = py[j] + n1 * L[1] + n2 * L[4] + n3 * L[7] - py[i];
         const double dz = pz[j] + n1 * L[2] + n2 * L[5] + n3 * L[8] - pz[i];
-        const double r2 = dx * dx + dy * dy + dz * dz;
-        const R r = narrow<R>(r2 * rsqrt_nr(r2));
+        double ir;
+        const R r = narrow<R>(dist_of(dx * dx + dy * dy + dz * dz, ir));
         R *e = C.nb + q * C.st;
         e[0] = narrow<R>(dx);
         e[1] = narrow<R>(dy);
@@ -562,8 +562,7 @@ __device__ __forceinline__ bool triplet_geom(const NNDev &M, const WarpCache<R> 
     T.rjk2 = T.jx * T.jx + T.jy * T.jy + T.jz * T.jz;
     if (!(T.rjk2 <= rc * rc)) return false;
     if constexpr (sizeof(R) == 8) {
-        T.ijk = rsqrt_nr(T.rjk2);
-        T.rjk = T.rjk2 * T.ijk;
+        T.rjk = dist_of(T.rjk2, T.ijk);
     } else {
         T.rjk = NM<R>::sq(T.rjk2);
     }

@@ -121,6 +121,22 @@ static __device__ __forceinline__ double rsqrt_nr(double x) {
     return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
+// Distance r of r2 = r^2, and 1/r.  Two atoms on one site (r2 = 0, or too small for the approximation) have r = 0 and
+// 1/r infinite as by sqrt and division, so that the forces between them are not finite numbers.
+static __device__ __noinline__ double2 dist_rare(double r2) {
+    const double r = sqrt(r2);
+    return make_double2(r, 1.0 / r);
+}
+static __device__ __forceinline__ double dist_of(double r2, double &inv) {
+    if ((unsigned)__double2hiint(r2) < 0x00100000u) {
+        const double2 d = dist_rare(r2);
+        inv = d.y;
+        return d.x;
+    }
+    inv = rsqrt_nr(r2);
+    return r2 * inv;
+}
+
 // n/d from the reciprocal id of d (within an ulp or two): the residual's correction makes the
 // quotient round as a division does, in 3 FP64 instructions instead of about 10
 static __device__ __forceinline__ double div_by(double n, double d, double id) {
