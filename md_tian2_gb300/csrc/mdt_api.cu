@@ -341,7 +341,8 @@ int ensure_nn_scratch(mdt_ctx *c) {
     int *img = dalloc<int>(c, 3 * (size_t)c->T, e);
     int *fb = dalloc<int>(c, (size_t)c->T, e);
     int *st = dalloc<int>(c, (size_t)c->T, e);
-    if (!nbw || !nbcnt || !img || !fb || !st) return fail(c, MDT_ERR_NOMEM, "neighbour-list scratch allocation failed");
+    double *epart = dalloc<double>(c, (size_t)c->T + 64 * (size_t)c->num_sms, e);  // T x parts of nn_cfg
+    if (!nbw || !nbcnt || !img || !fb || !st || !epart) return fail(c, MDT_ERR_NOMEM, "neighbour-list scratch allocation failed");
     std::vector<int> h(3 * (size_t)c->T);
     std::vector<double> box(9 * (size_t)c->T);
     e = cudaMemcpy(box.data(), c->B.box, sizeof(double) * box.size(), cudaMemcpyDeviceToHost);
@@ -359,6 +360,7 @@ int ensure_nn_scratch(mdt_ctx *c) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "neighbour-list scratch set-up");
     c->X = NNScratch{nbw, nbcnt, img, fb, st};
+    c->X.epart = epart;
     c->nn_maxnb_alloc = c->M.maxnb;
     return MDT_OK;
 }
@@ -375,6 +377,7 @@ LaunchCfg nn_cfg(mdt_ctx *c, int precision, bool split = false) {
         g.parts = std::max(1, std::min((2 * slots + c->T - 1) / c->T, (c->max_atoms + kNNWarps - 1) / kNNWarps));
         g.grid = std::max(1, std::min(c->T * g.parts, slots));
         g.total_ba = c->total_ba;
+        g.launches = &c->launches;
     }
     return g;
 }

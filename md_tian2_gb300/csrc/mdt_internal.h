@@ -16,6 +16,7 @@ struct LaunchCfg {
     int *counter;      // device work-queue counter (reset by the launcher)
     int parts = 1;     // CTAs per trajectory (EMT ring polymers: a cluster; generic HDNNP force calls, single beads)
     int64_t total_ba = 0;
+    int64_t *launches = nullptr;  // (parts > 1: counts the kernels around a split HDNNP force call)
     int threads = 128; // EMT kernels: threads per CTA (kBlock or kWideBlock)
 };
 

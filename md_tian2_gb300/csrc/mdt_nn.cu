@@ -81,7 +81,8 @@ __device__ SmemNN<R> carve_nn(unsigned char *base, const NNDev &M, int max_atoms
 // One bead: wrapped positions, neighbour lists, descriptors, network, forces.
 // Adds eV and eV/A into B.epot / B.f*.  Returns (in S.flag) whether a descriptor left
 // the scaling range widened by M.margin.  `part` of `parts`: the CTA's share of the bead's central
-// atoms, groups of kNNWarps dealt in turn; with several parts the sums meet in global memory.
+// atoms, groups of kNNWarps dealt in turn; with several parts the forces meet in global memory and
+// each part's energy goes to X.epart (nn_join_kernel adds them in order: an energy has the same bits in every call).
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ bool nn_bead(const Batch &B, const NNDev &M, const NNScratch &X, const SmemNN<R> &S, int t, int b,
@@ -237,7 +238,7 @@ __device__ bool nn_bead(const Batch &B, const NNDev &M, const NNScratch &X, cons
     }
     const double c = kHa2eV * kAng2BohrD;
     if (parts > 1) {
-        if (tid == 0) atomicAdd(&B.epot[B.bead_off[t] + b], etot * kHa2eV);
+        if (tid == 0) X.epart[(int64_t)t * parts + part] = etot;
         for (int i = tid; do_forces && i < N; i += nt) {
             if (S.fx[i] != R(0)) atomicAdd(&B.fx[base + i], (double)S.fx[i] * c);
             if (S.fy[i] != R(0)) atomicAdd(&B.fy[base + i], (double)S.fy[i] * c);
@@ -302,12 +303,18 @@ __global__ void nn_zero_kernel(Batch B, int64_t total) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
         B.fx[k] = 0.0; B.fy[k] = 0.0; B.fz[k] = 0.0;
         B.ax[k] = 0.0; B.ay[k] = 0.0; B.az[k] = 0.0;
-        if (k < B.ntraj) B.epot[B.bead_off[k]] = 0.0;
     }
 }
 
-__global__ void nn_accel_kernel(Batch B) {
-    for (int t = blockIdx.x; t < B.ntraj; t += gridDim.x) set_acceleration(B, traj_view(B, t), 0, 1);
+__global__ void nn_join_kernel(Batch B, const double *epart, int parts, int do_forces) {
+    for (int t = blockIdx.x; t < B.ntraj; t += gridDim.x) {
+        if (threadIdx.x == 0) {
+            double e = 0.0;
+            for (int p = 0; p < parts; ++p) e += epart[(int64_t)t * parts + p];
+            B.epot[B.bead_off[t]] = e * kHa2eV;
+        }
+        if (do_forces) set_acceleration(B, traj_view(B, t), 0, 1);
+    }
 }
 
 template <typename R, bool SURR>
@@ -387,16 +394,22 @@ static cudaError_t nn_launch_t(const LaunchCfg &c, const Batch &B, const NNDev &
     NNLaunch LN{B.max_atoms, ngeta, SURR || mode == 2 ? 1 : c.parts};
     cudaError_t e = cudaMemsetAsync(c.counter, 0, sizeof(int), c.stream);
     if (e != cudaSuccess) return e;
-    if (LN.parts > 1) {
+    const bool split = LN.parts > 1 && !X.gout;  // (a pass that leaves descriptors: its results are those alone)
+    if (split) {
         const int64_t total = c.total_ba;
         nn_zero_kernel<<<(int)std::min<int64_t>((total + 255) / 256, 4096), 256, 0, c.stream>>>(B, total);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (mode == 0 || mode == 1) {
         e = cudaFuncSetAttribute(nn_force_kernel<R, SURR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
         nn_force_kernel<R, SURR><<<c.grid, kNNBlock, sm, c.stream>>>(B, M, E, X, P, LN, c.order, c.counter,
                                                                      mode == 0 ? 1 : 0);
-        if (LN.parts > 1 && mode == 0) nn_accel_kernel<<<std::min(B.ntraj, 4096), 128, 0, c.stream>>>(B);
+        if (split) {
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            nn_join_kernel<<<std::min(B.ntraj, 4096), 128, 0, c.stream>>>(B, X.epart, LN.parts, mode == 0 ? 1 : 0);
+            *c.launches += 2;
+        }
     } else {
         e = cudaFuncSetAttribute(nn_md_steps_kernel<R, SURR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;

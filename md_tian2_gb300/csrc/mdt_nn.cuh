@@ -195,6 +195,7 @@ struct NNScratch {
     int *skok;
     int skcap;
     int *tcerr;        // set when a tensor-core GEMM did not complete within its wait limit
+    double *epart;     // generic force calls split over CTAs: the energy of each share (Ha)
     // generic kernels: dE/dG [ba][maxsf] and the atomic energies (Ha, output node) of a prior
     // tensor-core network pass; when set, the kernels skip descriptors and network and run the
     // forces (descriptor VJP) from them
