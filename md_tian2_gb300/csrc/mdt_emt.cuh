@@ -338,7 +338,24 @@ static __device__ __forceinline__ void image_table(const Cell &c, double *img) {
     for (int d = 0; d < 3; ++d) img[3 * k + d] = fma(c.h[d], n0, fma(c.h[d + 3], n1, c.h[d + 6] * n2));
 }
 
-// FP64 forces: min_image with its shift from the table: no FP64 conversion, comparison or product.
+// e minus the shift of |n| <= 1 per direction, without the table (large trajectories)
+static __device__ __noinline__ double3 image_near(const Cell &c, float n0, float n1, float n2, double ex, double ey,
+                                                  double ez) {
+    const float n[3] = {n0, n1, n2};
+    double d[3] = {ex, ey, ez};
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+        if (n[v] == 0.f) continue;
+        const double m = n[v] < 0.f ? 1.0 : -1.0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            if (c.nz >> (3 * v + q) & 1u) d[q] = fma(c.h[3 * v + q], m, d[q]);
+    }
+    return make_double3(d[0], d[1], d[2]);
+}
+
+// FP64 forces: min_image with its shift from the table: no FP64 conversion, comparison or product, and
+// nothing at all for a pair whose nearest image is its own.
 // A fractional coordinate near a tie, or an image further away, takes min_image itself.
 template <> struct PlaceDiff<double> {
     double x, y, z;
@@ -370,14 +387,20 @@ template <> struct PlaceDiff<double> {
         dx = ex;
         dy = ey;
         dz = ez;
-        if (off < 0.4999f && big < 1.5f && img) {
+        if (off < 0.4999f && big < 1.5f) {
             const float kf = 9.f * n[0] + 3.f * n[1] + n[2];
-            if (kf != 0.f) {
-                const double *v = img + 3 * ((int)kf + 13);
-                dx -= v[0];
-                dy -= v[1];
-                dz -= v[2];
+            if (kf == 0.f) return;
+            if (!img) {
+                const double3 d = image_near(*cell, n[0], n[1], n[2], ex, ey, ez);
+                dx = d.x;
+                dy = d.y;
+                dz = d.z;
+                return;
             }
+            const double *v = img + 3 * ((int)kf + 13);
+            dx -= v[0];
+            dy -= v[1];
+            dz -= v[2];
         } else {
             const double3 d = min_image_far(*cell, ex, ey, ez);
             dx = d.x;
