@@ -1782,6 +1782,9 @@ int32_t mdt_nn_set_model(mdt_ctx *c, const mdt_nn_model *m, int32_t ntypes, cons
     M.pnorm = (const double *)up(pnorm.data(), 8 * nk);
     M.smin = (const double *)up(m->smin, 8 * nk);
     M.smax = (const double *)up(m->smax, 8 * nk);
+    std::vector<double> sk(nk);
+    for (size_t k = 0; k < nk; ++k) sk[k] = (m->scmax - m->scmin) / (m->smax[k] - m->smin[k]);
+    M.sk = (const double *)up(sk.data(), 8 * nk);
     M.savg = (const double *)up(m->savg, 8 * nk);
     M.act = (const uint8_t *)up(act.data(), act.size());
     M.wd = (const double *)up(m->weights, 8 * (size_t)ne * m->maxweights);

@@ -88,9 +88,10 @@ __host__ __device__ constexpr EmtLayout emt_layout(int max_atoms, int max_beads)
                      max_beads > 1 && max_atoms <= 512, max_atoms <= 512};
 }
 
-// one bead at a time: the network kernels' fallback and the allocation-free call
+// One bead at a time, without the image table: the network kernels' fallback, whose shared memory bounds the
+// models and sizes that fit, and the allocation-free call.
 __host__ __device__ constexpr EmtLayout emt_layout_one(int max_atoms, int max_beads) {
-    return EmtLayout{max_atoms, max_beads, max_atoms, false, max_atoms <= 512};
+    return EmtLayout{max_atoms, max_beads, max_atoms, false, false};
 }
 
 // beads of an N-atom trajectory evaluated together, at most `per`
@@ -338,7 +339,8 @@ static __device__ __forceinline__ void image_table(const Cell &c, double *img) {
     for (int d = 0; d < 3; ++d) img[3 * k + d] = fma(c.h[d], n0, fma(c.h[d + 3], n1, c.h[d + 6] * n2));
 }
 
-// e minus the shift of |n| <= 1 per direction, without the table (large trajectories)
+// e minus the shift of |n| <= 1 per direction, without the table (large trajectories, the network
+// kernels' fallback)
 static __device__ __noinline__ double3 image_near(const Cell &c, float n0, float n1, float n2, double ex, double ey,
                                                   double ez) {
     const float n[3] = {n0, n1, n2};

@@ -51,6 +51,7 @@ struct NNDev {
     // per element e and symmetry function s at [e*maxsf + s]
     const int *sftype, *e1, *e2, *izeta, *etaslot;
     const double *eta, *rs, *lam, *zeta, *pnorm, *smin, *smax, *savg;
+    const double *sk;             // (scmax - scmin)/(smax - smin)
     const uint8_t *act;           // [e][layer][node]
     const double *wd;             // weights, FP64
     const float *wf;              // weights, FP32 copy

@@ -60,7 +60,6 @@ template <typename R> struct SmemTrain {
     int8_t *nbelem;
     R *buf;   // per warp: G, c/v, then 6 x (L+1) x kMaxNodes network buffers
     double *scal;  // 0: a (dL/dE in Ha^-1 units)
-    double *smn, *sk;  // scaling per element and function: scaled = (G - smn) sk + scmin
     int stride;
 };
 
@@ -71,7 +70,7 @@ __host__ __device__ inline size_t train_smem_bytes(int max_atoms, int maxnb, int
     s += r16(rs * (size_t)nelem * maxweights) * (1 + warps);
     s += r16(rs * warps * maxnb * (6 + ngeta)) + r16(rs * warps * maxnb * 3) + r16(4 * warps * maxnb) +
          r16(warps * maxnb);
-    s += r16(rs * warps * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes)) + r16(8 * 4) + 2 * r16(8 * nelem * kMaxSF);
+    s += r16(rs * warps * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes)) + r16(8 * 4);
     return s;
 }
 
@@ -107,8 +106,6 @@ __device__ SmemTrain<R> carve_train(unsigned char *base, const NNDev &M, int max
     s.nbelem = (int8_t *)take(W * M.maxnb);
     s.buf = (R *)take(sizeof(R) * W * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes));
     s.scal = (double *)take(8 * 4);
-    s.smn = (double *)take(8 * M.nelem * kMaxSF);
-    s.sk = (double *)take(8 * M.nelem * kMaxSF);
     return s;
 }
 
@@ -151,15 +148,6 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
     const size_t nw = (size_t)M.nelem * M.maxweights;
     for (size_t k = tid; k < nw; k += nt) S.w[k] = (R)D.theta[k];
     for (size_t k = tid; k < nw * W; k += nt) S.gradw[k] = R(0);
-    // the scaling's FP64 divisions once per CTA, not per atom and pass
-    for (int k = tid; k < M.nelem * kMaxSF; k += nt) {
-        const int e = k / kMaxSF, f = k - e * kMaxSF;
-        if (f >= M.nsf[e]) continue;
-        const double mn = M.smin[e * M.maxsf + f];
-        S.smn[k] = mn;
-        S.sk[k] = (M.scmax - M.scmin) / (M.smax[e * M.maxsf + f] - mn);
-    }
-    __syncthreads();
     WarpCache<R> C{S.nb + (size_t)warp * M.maxnb * S.stride, S.slotf + (size_t)warp * M.maxnb * 3,
                    S.nbatom + warp * M.maxnb, S.nbelem + warp * M.maxnb, S.stride};
     R *wb = S.buf + (size_t)warp * (2 * kMaxSF + 6 * (kMaxLayers + 1) * kMaxNodes);
@@ -194,7 +182,7 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
             const int ei = S.elem[i];
             if (ei < 0) continue;
             const int cnt = X.nbcnt[base + i];
-            const int nsf = M.nsf[ei], sfb = ei * kMaxSF;
+            const int nsf = M.nsf[ei], sfb = ei * M.maxsf;
             const R *we = S.w + (size_t)ei * M.maxweights;
             acsf_cache<R>(M, C, i, ei, cnt, X.nbw + (base + i) * (int64_t)M.maxnb, S.px, S.py, S.pz, S.elem, S.lat);
             if (D.dgin) {  // the network ran outside: its output and dE/dG
@@ -204,7 +192,7 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
                 __syncwarp();
             } else {
                 for (int s = lane; s < nsf; s += 32)
-                    h[s] = (R)((D.G[(base + i) * M.maxsf + s] - S.smn[sfb + s]) * S.sk[sfb + s] + M.scmin);
+                    h[s] = (R)((D.G[(base + i) * M.maxsf + s] - M.smin[sfb + s]) * M.sk[sfb + s] + M.scmin);
                 __syncwarp();
                 net_forward<R>(M, we, ei, z, h, zd, hd, false);
                 if (lane == 0) e_warp += (double)h[M.nlayers * kMaxNodes] + (M.remove_atom_energies ? M.atom_energy[ei] : 0.0);
@@ -233,7 +221,7 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
                         // (each lane starts at its own column: rows of 32 weights share their banks)
                         for (int q = 0, n = s % n1; q < n1; ++q, n = n + 1 == n1 ? 0 : n + 1)
                             v += wl[s * n1 + n] * dl[1 * kMaxNodes + n];
-                        cv[s] = v * (R)S.sk[sfb + s];
+                        cv[s] = v * (R)M.sk[sfb + s];
                     }
                 }
                 __syncwarp();
@@ -282,21 +270,21 @@ __global__ void __launch_bounds__(32 * TrainCfg<R>::warps) train_kernel(Batch B,
             const int ei = S.elem[i];
             if (ei < 0) continue;
             const int cnt = X.nbcnt[base + i];
-            const int nsf = M.nsf[ei], sfb = ei * kMaxSF;
+            const int nsf = M.nsf[ei], sfb = ei * M.maxsf;
             const R *we = S.w + (size_t)ei * M.maxweights;
             R *gwe = gw + (size_t)ei * M.maxweights;
             acsf_cache<R>(M, C, i, ei, cnt, X.nbw + (base + i) * (int64_t)M.maxnb, S.px, S.py, S.pz, S.elem, S.lat);
             acsf_jvp<R>(M, C, ei, cnt, i, S.ux, S.uy, S.uz, cv);
             if (D.xdot) {  // the network's sweep runs outside: its inputs
                 for (int s = lane; s < nsf; s += 32)
-                    D.xdot[(base + i) * M.maxsf + s] = (float)(cv[s] * (R)S.sk[sfb + s]);
+                    D.xdot[(base + i) * M.maxsf + s] = (float)(cv[s] * (R)M.sk[sfb + s]);
                 if (lane == 0) D.arow[base + i] = (double)a;
                 __syncwarp();
                 continue;
             }
             for (int s = lane; s < nsf; s += 32) {
-                h[s] = (R)((D.G[(base + i) * M.maxsf + s] - S.smn[sfb + s]) * S.sk[sfb + s] + M.scmin);
-                hd[s] = cv[s] * (R)S.sk[sfb + s];
+                h[s] = (R)((D.G[(base + i) * M.maxsf + s] - M.smin[sfb + s]) * M.sk[sfb + s] + M.scmin);
+                hd[s] = cv[s] * (R)M.sk[sfb + s];
             }
             __syncwarp();
             net_forward<R>(M, we, ei, z, h, zd, hd, true);

@@ -65,3 +65,32 @@ def test_emt_layout(tmp_path):
     bad, seen = map(int, subprocess.run([str(tmp_path / "layout")], check=True, capture_output=True,
                                         text=True).stdout.split())
     assert seen > 1000 and bad == 0
+
+
+# what the network kernels laid out beside their own buffers before the image table
+SIZES = r"""
+#include <cstdio>
+#include "mdt_emt.cuh"
+using namespace mdt;
+int main() {
+    auto r16 = [](size_t b) { return (b + 15) & ~size_t(15); };
+    long larger = 0;
+    for (int n = 1; n <= 4096; ++n)
+        for (int nb : {1, 2, 8, 32}) {
+            const size_t was = 8 * r16(8 * n) + 2 * r16(8 * 64) + r16(8 * rp_cells(nb)) + 256 + 2 * r16(n);
+            larger += smem_bytes<double>(emt_layout_one(n, nb)) > was;
+        }
+    std::printf("%ld\n", larger);
+    return 0;
+}
+"""
+
+
+def test_fallback_layout_no_larger(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not Path(nvcc).exists():
+        pytest.skip("no nvcc")
+    (tmp_path / "sizes.cu").write_text(SIZES)
+    subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-O1", "-std=c++17", "-I", str(CSRC),
+                    str(tmp_path / "sizes.cu"), "-o", str(tmp_path / "sizes")], check=True, capture_output=True)
+    assert int(subprocess.run([str(tmp_path / "sizes")], check=True, capture_output=True, text=True).stdout) == 0
