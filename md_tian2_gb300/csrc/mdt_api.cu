@@ -55,6 +55,7 @@ struct mdt_ctx {
     double *rnd[4] = {nullptr, nullptr, nullptr, nullptr};
     double *summary = nullptr;
     size_t scratch_prec_bytes = 0;
+    TeamWork team_work{};
     int emt_per_sm[2] = {0, 0};  // resident CTAs of the EMT kernels (FP64, FP32 forces); 0: not asked yet
 
     // HDNNP / surrogate
@@ -273,11 +274,7 @@ int check_ready(mdt_ctx *c, bool need_emt) {
     return MDT_OK;
 }
 
-// Ring polymers: a cluster of CTAs shares each trajectory's beads and transforms, the largest of
-// 8, 4, 2 that leaves at most four waves of resident CTAs.  With one CTA per trajectory a batch
-// waits for its longest ring polymer (32 beads, one after the other): 96 FP64 trajectories 31.3 ms
-// with one, 13.1 with 8; 1024 with FP32 forces 26.3 ms with one, 22.4 with 2, 33 with 4 (fewer beads at a
-// time fill fewer warps, and every CTA repeats the tables and sums of a step).
+// Ring polymers: a cluster of CTAs shares each trajectory's beads and transforms (team_log2).
 LaunchCfg cfg(mdt_ctx *c, int precision) {
     int &per_sm = c->emt_per_sm[precision == MDT_PREC_FP32 ? 1 : 0];
     if (!per_sm) per_sm = max_resident_ctas(c->max_atoms, c->max_beads, precision);
@@ -286,9 +283,7 @@ LaunchCfg cfg(mdt_ctx *c, int precision) {
     // at most one trajectory per SM: twice the warps shorten its chain of phases
     if (c->max_beads == 1 && c->T <= c->num_sms) g.threads = kWideBlock;
     if (c->max_beads > 1) {
-        g.parts = 1;
-        while (g.parts < 8 && 2 * g.parts <= c->max_beads && (int64_t)c->T * 2 * g.parts <= 4 * (int64_t)slots)
-            g.parts *= 2;
+        g.parts = 1 << team_log2(c->team_work, c->T, c->max_beads, slots);
         const int teams = std::max(1, std::min(c->T, slots / g.parts));
         g.grid = teams * g.parts;
     }
@@ -1038,6 +1033,7 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
     int at = 0, bd = 0;
     c->max_atoms = 0;
     c->max_beads = 0;
+    c->team_work = TeamWork{};
     for (int t = 0; t < ntraj; ++t) {
         const int N = natoms[t], nb = nbeads[t];
         if (N < 1 || nb < 1 || nb > 32)
@@ -1052,6 +1048,7 @@ int32_t mdt_batch_define(mdt_ctx *c, int32_t ntraj, const int32_t *natoms, const
         pairs += (int64_t)nb * N * (N / 2);
         c->max_atoms = std::max(c->max_atoms, N);
         c->max_beads = std::max(c->max_beads, nb);
+        c->team_work.add(N, nb);
         auto it = std::find(nb_tables.begin(), nb_tables.end(), nb);
         if (it == nb_tables.end()) {
             nb_tables.push_back(nb);

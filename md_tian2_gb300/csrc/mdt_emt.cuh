@@ -94,6 +94,34 @@ __host__ __device__ constexpr EmtLayout emt_layout_one(int max_atoms, int max_be
     return EmtLayout{max_atoms, max_beads, max_atoms, false, false};
 }
 
+// Work of a batch with teams of 1, 2, 4, 8 CTAs per trajectory, in pairs of atoms: CTA time it takes up
+// (a CTA of a team waits where the trajectory has fewer beads) and its longest trajectory's.
+struct TeamWork {
+    double all[4], longest[4];
+    void add(int natoms, int nbeads) {
+        for (int k = 0; k < 4; ++k) {
+            const int rounds = (nbeads + (1 << k) - 1) >> k;
+            const double w = (double)rounds * natoms * natoms;
+            all[k] += w * (1 << k);
+            longest[k] = longest[k] > w ? longest[k] : w;
+        }
+    }
+};
+
+// CTAs per trajectory of a ring-polymer batch (log2), `slots` of them resident: doubled while it brings the batch's
+// end nearer (its longest trajectory and an even share of all work), has beads to share and leaves at most
+// four waves.  With one CTA per trajectory a batch waits for its longest ring polymer (32 beads, one after the
+// other): 96 FP64 trajectories 31.3 ms with one, 13.1 with 8; 1024 with FP32 forces 26.3 ms with one, 22.4
+// with 2, 33 with 4 (fewer beads at a time fill fewer warps, and every CTA repeats the tables and sums of a
+// step).  1199 single beads beside one 2-bead ring polymer: 1.9 ms with one, 2.6 with 2 (half the CTAs wait).
+inline int team_log2(const TeamWork &w, int64_t ntraj, int max_beads, int64_t slots) {
+    int k = 0;
+    while (k < 3 && (2 << k) <= max_beads && ntraj * (2 << k) <= 4 * slots &&
+           w.longest[k + 1] + w.all[k + 1] / slots < w.longest[k] + w.all[k] / slots)
+        ++k;
+    return k;
+}
+
 // beads of an N-atom trajectory evaluated together, at most `per`
 __host__ __device__ constexpr int emt_group(int places, bool together, int N, int per) {
     return !together ? 1 : per < places / N ? per : places / N;
