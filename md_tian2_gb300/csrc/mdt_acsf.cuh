@@ -17,6 +17,8 @@
 // where A1 = sum u_s zeta_s lambda_s, A2 = sum u_s eta_s (1+lambda_s cos), A3 = sum u_s (1+lambda_s cos):
 // three multiply-adds per function and triplet instead of three full derivative factors.
 #pragma once
+#include <type_traits>
+
 #include "mdt_common.cuh"
 #include "mdt_nn.cuh"
 
@@ -540,8 +542,16 @@ __device__ void acsf_jvp(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
 // Grid form of the G3 functions (NNDev::g3fast): cells (eta slot m, (lambda, zeta)
 // slot q) share one neighbour pair; per triplet the ng exponentials and nlz angular
 // powers meet in an outer product accumulated in registers.
+//
+// Each walk in three forms, by the set's structure (g3_form).  Most sets are a product of at most two lambdas and
+// four zetas (each zeta with lambda -1 and +1): the product walk takes the powers of both p = 1 + lambda cos by one
+// decoding of an exponent, in registers; compiled for 3 etas x 3 zetas and for 4 x 4, whose sums take
+// registers most networks do not need (compiled for 4 x 4 alone 18.3 instead of 15.7 ms below).  Any other set of
+// up to 8 cells walks its cells one by one.  512 H/graphene configurations, FP32, zeta 1, 2, 4: 4.9 ms with
+// the product walk, 6.8 cell by cell; 2048 with the tensor-core network 15.7 against 20.0 ms (zeta 1, 4, 16
+// fixed at compile time: 13.9); 64 in FP64 8.4 against 9.0.
 // ---------------------------------------------------------------------------
-constexpr int kGM = 4, kGQ = 8;
+constexpr int kGM = 4, kGQ = 8;  // largest grid
 
 __device__ __forceinline__ bool fast_pair(const NNDev &M, int ei, int ej, int ek) {
     const int p1 = M.g3pair[ei][0], p2 = M.g3pair[ei][1];
@@ -573,78 +583,118 @@ __device__ __forceinline__ bool triplet_geom(const NNDev &M, const WarpCache<R> 
     return true;
 }
 
-template <typename R> struct GridConst {
-    R lam[kGQ], zl[kGQ], pn[kGQ], eta[kGM];
-    int zm1[kGQ];
-    int lidx[kGQ];   // which distinct lambda (0/1) the cell uses
-    R lams[2];
-    int ng, nq, nl;
+// p = 1 + lambda cos with its squares p^2 .. p^16 (as far as `bits`, all exponents' bits, go), from which every
+// integer power up to 31 is a product
+template <typename R> struct Powers {
+    R w[5];
+    bool on;  // p > 0: the cells of this lambda count
+    __device__ __forceinline__ Powers(R lam, R cost, int bits) {
+        w[0] = R(1) + lam * cost;
+        on = w[0] > R(0);
+#pragma unroll
+        for (int b = 1; b < 5; ++b) {
+            w[b] = R(0);
+            if (bits >> b) w[b] = w[b - 1] * w[b - 1];
+        }
+    }
 };
 
-// (1 + lambda cos) for the (at most two) distinct lambdas and its squaring ladder
-// p, p^2, p^4, p^8, p^16, from which every integer power up to 31 is a product.
-template <typename R> struct Ladder {
-    R pw[2][5];
-    bool pos[2];
+// Any cells.  each(cos, f) calls f(q, p^(zeta-1), p^zeta) for every cell q, with zeros where p <= 0.
+template <typename R> struct AnyCells {
+    static constexpr int NQ = kGQ;
+    R zl[NQ], lams[2];
+    int zm1[NQ], bits;
+    unsigned of[2];  // the cells of each of the two lambdas
+    static __device__ __forceinline__ int sf(const NNDev &M, int ei, int m, int q) {
+        return q < M.nlz[ei] ? M.sf_of[ei][m][q] : -1;
+    }
+    static __device__ __forceinline__ R pn(const NNDev &M, int ei, int q) {
+        return q < M.nlz[ei] ? widen<R>(M.lz_pnorm[ei][q]) : R(0);
+    }
+    __device__ __forceinline__ AnyCells(const NNDev &M, int ei) {
+        bits = 0;
+        lams[0] = widen<R>(M.lz_lam[ei][0]);
+        lams[1] = R(0);
+        of[0] = of[1] = 0u;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            zl[q] = R(0);
+            zm1[q] = 0;
+            if (q >= M.nlz[ei]) continue;
+            zl[q] = widen<R>(M.lz_zl[ei][q]);
+            zm1[q] = M.lz_zm1[ei][q];
+            bits |= zm1[q];
+            if (M.lz_lam[ei][q] == M.lz_lam[ei][0]) {
+                of[0] |= 1u << q;
+            } else {
+                lams[1] = widen<R>(M.lz_lam[ei][q]);
+                of[1] |= 1u << q;
+            }
+        }
+    }
+    template <typename F> __device__ __forceinline__ void each(R cost, F f) const {
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            if (!of[l]) continue;
+            const Powers<R> L(lams[l], cost, bits);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                if (!(of[l] >> q & 1u)) continue;
+                R r = zm1[q] & 1 ? L.w[0] : R(1);
+#pragma unroll
+                for (int b = 1; b < 5; ++b)
+                    if ((zm1[q] >> b) & 1) r *= L.w[b];
+                f(q, L.on ? r : R(0), L.on ? r * L.w[0] : R(0));
+            }
+        }
+    }
 };
 
-template <typename R>
-__device__ __forceinline__ void ladder_make(const GridConst<R> &g, R cost, Ladder<R> &L) {
+// the product of two lambdas and NZ zetas, cell 2 z + l (cells that are not in the set have no function)
+template <typename R, int NZ> struct ProductCells {
+    static constexpr int NQ = 2 * NZ;
+    R zl[NQ], lams[2];
+    int ex[NZ], bits;
+    static __device__ __forceinline__ int sf(const NNDev &M, int ei, int m, int q) { return M.gsf[ei][m][q]; }
+    static __device__ __forceinline__ R pn(const NNDev &M, int ei, int q) { return widen<R>(M.gpn[ei][q >> 1]); }
+    __device__ __forceinline__ ProductCells(const NNDev &M, int ei) {
+        bits = 0;
 #pragma unroll
-    for (int l = 0; l < 2; ++l) {
-        const R p = R(1) + g.lams[l] * cost;
-        L.pos[l] = (l < g.nl) && (p > R(0));
-        L.pw[l][0] = p;
+        for (int l = 0; l < 2; ++l) lams[l] = widen<R>(M.glam[ei][l]);
 #pragma unroll
-        for (int b = 1; b < 5; ++b) L.pw[l][b] = L.pw[l][b - 1] * L.pw[l][b - 1];
+        for (int z = 0; z < NZ; ++z) {
+            ex[z] = M.gex[ei][z];
+            bits |= ex[z];
+#pragma unroll
+            for (int l = 0; l < 2; ++l) zl[2 * z + l] = widen<R>((float)(ex[z] + 1) * M.glam[ei][l]);
+        }
     }
-}
-
-template <typename R> __device__ __forceinline__ R ladder_pow(const Ladder<R> &L, int l, int e) {
-    R r = R(1);
-    if constexpr (sizeof(R) == 8) {
-        // the exponent is the same for the whole warp: only the powers it holds are multiplied
+    template <typename F> __device__ __forceinline__ void each(R cost, F f) const {
+        const Powers<R> L0(lams[0], cost, bits), L1(lams[1], cost, bits);
 #pragma unroll
-        for (int b = 0; b < 5; ++b)
-            if ((e >> b) & 1) r *= L.pw[l][b];
-    } else {
+        for (int z = 0; z < NZ; ++z) {
+            R r0 = R(1), r1 = R(1);
+            if (ex[z] & 1) {
+                r0 = L0.w[0];
+                r1 = L1.w[0];
+            }
 #pragma unroll
-        for (int b = 0; b < 5; ++b) r *= ((e >> b) & 1) ? L.pw[l][b] : R(1);
+            for (int b = 1; b < 5; ++b)
+                if ((ex[z] >> b) & 1) {
+                    r0 *= L0.w[b];
+                    r1 *= L1.w[b];
+                }
+            f(2 * z, L0.on ? r0 : R(0), L0.on ? r0 * L0.w[0] : R(0));
+            f(2 * z + 1, L1.on ? r1 : R(0), L1.on ? r1 * L1.w[0] : R(0));
+        }
     }
-    return r;
-}
-
-template <typename R> __device__ __forceinline__ GridConst<R> grid_const(const NNDev &M, int ei) {
-    GridConst<R> g;
-    g.ng = M.ng3eta[ei];
-    g.nq = M.nlz[ei];
-#pragma unroll
-    for (int q = 0; q < kGQ; ++q) {
-        g.lam[q] = widen<R>(M.lz_lam[ei][q]);
-        g.zl[q] = widen<R>(M.lz_zl[ei][q]);
-        g.pn[q] = widen<R>(M.lz_pnorm[ei][q]);
-        g.zm1[q] = M.lz_zm1[ei][q];
-    }
-#pragma unroll
-    for (int m = 0; m < kGM; ++m) g.eta[m] = m < g.ng ? g3_eta<R>(M, ei, m) : R(0);
-    g.nl = 0;
-    g.lams[0] = g.lams[1] = R(0);
-#pragma unroll
-    for (int q = 0; q < kGQ; ++q) {
-        g.lidx[q] = 0;
-        if (q >= g.nq) continue;
-        if (g.nl > 0 && g.lams[0] == g.lam[q]) g.lidx[q] = 0;
-        else if (g.nl > 1 && g.lams[1] == g.lam[q]) g.lidx[q] = 1;
-        else if (g.nl < 2) { g.lams[g.nl] = g.lam[q]; g.lidx[q] = g.nl; ++g.nl; }
-    }
-    return g;
-}
+};
 
 // exp(-eta_m (r_ij^2 + r_ik^2 + r_jk^2)) for every eta slot
-template <typename R>
-__device__ __forceinline__ void grid_pexp(const GridConst<R> &g, const Triplet<R> &T, R *E) {
+template <typename R, int GM>
+__device__ __forceinline__ void grid_pexp(const R *eta, int ng, const Triplet<R> &T, R *E) {
 #pragma unroll
-    for (int m = 0; m < kGM; ++m) E[m] = (m < g.ng) ? T.a[6 + m] * T.c[6 + m] * NM<R>::ex(-g.eta[m] * T.rjk2) : R(0);
+    for (int m = 0; m < GM; ++m) E[m] = m < ng ? T.a[6 + m] * T.c[6 + m] * NM<R>::ex(-eta[m] * T.rjk2) : R(0);
 }
 
 // forces of one triplet from its A1, A2, A3 (head of this file): on the centre, the row's neighbour
@@ -678,189 +728,66 @@ __device__ __forceinline__ void vjp_pairs(const Triplet<R> &T, R A1, R A2, R A3,
     atomicAdd(&C.slotf[3 * q4 + 2], -T.c[2] * P2 - T.jz * P3);
 }
 
-// The set of the benchmark networks (NNDev::g3std): three etas, zeta 1, 4 and 16, lambda -1 and +1.
-// The same walks with the cells fixed at compile time: (1 + lambda cos)^(zeta-1) is a product of
-// the squares p, p^2, p^4, p^8 taken once per lambda (the general walk multiplies five factors per
-// cell), nothing is indexed at run time (the general walk keeps its ladder in local memory), and the
-// sums run in the general walk's order.
-template <typename R> struct StdCells {
-    R p[2], pp[2][3];  // 1 + lambda cos; its powers zeta - 1 (all zero where 1 + lambda cos <= 0)
-    __device__ __forceinline__ StdCells(R cost) {
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-            p[l] = R(1) + R(l ? 1 : -1) * cost;
-            const bool on = p[l] > R(0);
-            const R p2 = p[l] * p[l], p4 = p2 * p2, p8 = p4 * p4, a = p[l] * p2;
-            pp[l][0] = on ? R(1) : R(0);
-            pp[l][1] = on ? a : R(0);
-            pp[l][2] = on ? a * p4 * p8 : R(0);
-        }
-    }
-};
-
-template <typename R> __device__ __forceinline__ void std_pexp(const R *eta, const Triplet<R> &T, R *E) {
-#pragma unroll
-    for (int m = 0; m < 3; ++m) E[m] = T.a[6 + m] * T.c[6 + m] * NM<R>::ex(-eta[m] * T.rjk2);
-}
-
-template <typename R>
-__device__ void acsf_g3_forward_std(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, R *G) {
-    const int lane = threadIdx.x & 31;
+template <typename R, int GM, typename CELLS>
+__device__ __forceinline__ void g3_forward_walk(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, R *G) {
+    const int lane = threadIdx.x & 31, ng = M.ng3eta[ei];
+    constexpr int GQ = CELLS::NQ;
     const CutK<R> ck = cut_k<R>(M, ei);
-    const R eta[3] = {g3_eta<R>(M, ei, 0), g3_eta<R>(M, ei, 1), g3_eta<R>(M, ei, 2)};
-    R acc[3][6];
+    const CELLS g(M, ei);
+    R eta[GM];
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
+    for (int m = 0; m < GM; ++m) eta[m] = m < ng ? g3_eta<R>(M, ei, m) : R(0);
+    R acc[GM][GQ];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) acc[m][q] = R(0);
+    for (int m = 0; m < GM; ++m)
+#pragma unroll
+        for (int q = 0; q < GQ; ++q) acc[m][q] = R(0);
     RowWalk tw;
     tw.init(cnt, lane);
     while (tw.valid) {
         Triplet<R> T;
         if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
-            R E[3];
-            std_pexp<R>(eta, T, E);
-            const StdCells<R> L(T.cost0);
+            R E[GM];
+            grid_pexp<R, GM>(eta, ng, T, E);
 #pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                const R pw = L.pp[q & 1][q >> 1] * L.p[q & 1];
+            for (int m = 0; m < GM; ++m) E[m] *= T.pfc;
+            g.each(T.cost0, [&](int q, R, R pw) {
 #pragma unroll
-                for (int m = 0; m < 3; ++m) acc[m][q] += E[m] * T.pfc * pw;
-            }
+                for (int m = 0; m < GM; ++m) acc[m][q] += E[m] * pw;
+            });
         }
         tw.next();
     }
 #pragma unroll
-    for (int m = 0; m < 3; ++m)
+    for (int m = 0; m < GM; ++m)
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
+        for (int q = 0; q < GQ; ++q) {
+            const int s = m < ng ? CELLS::sf(M, ei, m, q) : -1;
+            if (s < 0) continue;
             const R v = warp_sum(acc[m][q]);
-            const int s = M.sf_of[ei][m][q];
-            if (lane == 0 && s >= 0) G[s] = v * (q < 2 ? R(1) : q < 4 ? R(0.125) : R(1.0 / 32768.0));
-        }
-    __syncwarp();
-}
-
-template <typename R>
-__device__ void acsf_g3_vjp_std(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix, R &fiy,
-                                R &fiz) {
-    const int lane = threadIdx.x & 31;
-    const CutK<R> ck = cut_k<R>(M, ei);
-    const R eta[3] = {g3_eta<R>(M, ei, 0), g3_eta<R>(M, ei, 1), g3_eta<R>(M, ei, 2)};
-    R Wc[3][6];
-#pragma unroll
-    for (int m = 0; m < 3; ++m)
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const int s = M.sf_of[ei][m][q];
-            Wc[m][q] = s >= 0 ? c[s] * (q < 2 ? R(1) : q < 4 ? R(0.125) : R(1.0 / 32768.0)) : R(0);
-        }
-    R sjx = R(0), sjy = R(0), sjz = R(0);  // force on the current row's neighbour q3
-    RowWalk tw;
-    tw.init(cnt, lane);
-    while (tw.valid) {
-        Triplet<R> T;
-        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
-            R E[3];
-            std_pexp<R>(eta, T, E);
-            const StdCells<R> L(T.cost0);
-            R A1 = R(0), A2 = R(0), A3 = R(0);
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                const R plam = L.p[q & 1], pp = L.pp[q & 1][q >> 1];
-                const R zl = R((q & 1 ? 1 : -1) * (q < 2 ? 1 : q < 4 ? 4 : 16));
-                R S = R(0), Tq = R(0);
-#pragma unroll
-                for (int m = 0; m < 3; ++m) {
-                    const R w = Wc[m][q] * E[m];
-                    S += w;
-                    Tq += eta[m] * w;
-                }
-                A1 += zl * pp * S;
-                A2 += plam * pp * Tq;
-                A3 += plam * pp * S;
-            }
-            vjp_pairs<R>(T, A1, A2, A3, C, tw.q4, fix, fiy, fiz, sjx, sjy, sjz);
-        }
-        if (tw.row_end) {
-            atomicAdd(&C.slotf[3 * tw.q3], sjx);
-            atomicAdd(&C.slotf[3 * tw.q3 + 1], sjy);
-            atomicAdd(&C.slotf[3 * tw.q3 + 2], sjz);
-            sjx = sjy = sjz = R(0);
-        }
-        tw.next();
-    }
-}
-
-template <typename R> __device__ void acsf_g3_forward_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
-                                                           R *G) {
-    if (M.g3std[ei]) {
-        acsf_g3_forward_std<R>(M, C, ei, cnt, G);
-        return;
-    }
-    const int lane = threadIdx.x & 31;
-    const CutK<R> ck = cut_k<R>(M, ei);
-    const R rc = ck.rc;
-    const GridConst<R> g = grid_const<R>(M, ei);
-    R acc[kGM][kGQ];
-#pragma unroll
-    for (int m = 0; m < kGM; ++m)
-#pragma unroll
-        for (int q = 0; q < kGQ; ++q) acc[m][q] = R(0);
-    RowWalk tw;
-    tw.init(cnt, lane);
-    while (tw.valid) {
-        Triplet<R> T;
-        if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
-            R E[kGM];
-            grid_pexp<R>(g, T, E);
-#pragma unroll
-            for (int m = 0; m < kGM; ++m) E[m] *= T.pfc;
-            Ladder<R> L;
-            ladder_make<R>(g, T.cost0, L);
-#pragma unroll
-            for (int q = 0; q < kGQ; ++q) {
-                if (q >= g.nq) break;
-                const int l = g.lidx[q];
-                if (!L.pos[l]) continue;
-                const R pw = ladder_pow<R>(L, l, g.zm1[q]) * L.pw[l][0];
-#pragma unroll
-                for (int m = 0; m < kGM; ++m) acc[m][q] += E[m] * pw;
-            }
-        }
-        tw.next();
-    }
-#pragma unroll
-    for (int m = 0; m < kGM; ++m)
-#pragma unroll
-        for (int q = 0; q < kGQ; ++q) {
-            if (m >= g.ng || q >= g.nq) continue;
-            const R v = warp_sum(acc[m][q]);
-            const int s = M.sf_of[ei][m][q];
-            if (lane == 0 && s >= 0) G[s] = v * g.pn[q];
+            if (lane == 0) G[s] = v * CELLS::pn(M, ei, q);
         }
     __syncwarp();
 }
 
 // G3 part of the VJP in grid form; adds into fix/fiy/fiz and the slot forces
-template <typename R>
-__device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix, R &fiy,
-                                 R &fiz) {
-    if (M.g3std[ei]) {
-        acsf_g3_vjp_std<R>(M, C, ei, cnt, c, fix, fiy, fiz);
-        return;
-    }
-    const int lane = threadIdx.x & 31;
+template <typename R, int GM, typename CELLS>
+__device__ __forceinline__ void g3_vjp_walk(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix,
+                                            R &fiy, R &fiz) {
+    const int lane = threadIdx.x & 31, ng = M.ng3eta[ei];
+    constexpr int GQ = CELLS::NQ;
     const CutK<R> ck = cut_k<R>(M, ei);
-    const R rc = ck.rc;
-    const GridConst<R> g = grid_const<R>(M, ei);
-    R Wc[kGM][kGQ];
+    const CELLS g(M, ei);
+    R eta[GM];
 #pragma unroll
-    for (int m = 0; m < kGM; ++m)
+    for (int m = 0; m < GM; ++m) eta[m] = m < ng ? g3_eta<R>(M, ei, m) : R(0);
+    R Wc[GM][GQ];
 #pragma unroll
-        for (int q = 0; q < kGQ; ++q) {
-            const int s = (m < g.ng && q < g.nq) ? M.sf_of[ei][m][q] : -1;
-            Wc[m][q] = s >= 0 ? c[s] * g.pn[q] : R(0);
+    for (int m = 0; m < GM; ++m)
+#pragma unroll
+        for (int q = 0; q < GQ; ++q) {
+            const int s = m < ng ? CELLS::sf(M, ei, m, q) : -1;
+            Wc[m][q] = s >= 0 ? c[s] * CELLS::pn(M, ei, q) : R(0);
         }
     R sjx = R(0), sjy = R(0), sjz = R(0);  // force on the current row's neighbour q3
     RowWalk tw;
@@ -868,29 +795,21 @@ __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
     while (tw.valid) {
         Triplet<R> T;
         if (fast_pair(M, ei, C.nbelem[tw.q3], C.nbelem[tw.q4]) && triplet_geom<R>(M, C, tw.q3, tw.q4, ck, T)) {
-            R E[kGM];
-            grid_pexp<R>(g, T, E);
-            Ladder<R> L;
-            ladder_make<R>(g, T.cost0, L);
+            R E[GM];
+            grid_pexp<R, GM>(eta, ng, T, E);
             R A1 = R(0), A2 = R(0), A3 = R(0);
-#pragma unroll
-            for (int q = 0; q < kGQ; ++q) {
-                if (q >= g.nq) break;
-                const int l = g.lidx[q];
-                if (!L.pos[l]) continue;
-                const R plam = L.pw[l][0];
-                const R pp = ladder_pow<R>(L, l, g.zm1[q]);
+            g.each(T.cost0, [&](int q, R pp, R pl) {
                 R S = R(0), Tq = R(0);
 #pragma unroll
-                for (int m = 0; m < kGM; ++m) {
+                for (int m = 0; m < GM; ++m) {
                     const R w = Wc[m][q] * E[m];
                     S += w;
-                    Tq += g.eta[m] * w;
+                    Tq += eta[m] * w;
                 }
                 A1 += g.zl[q] * pp * S;
-                A2 += plam * pp * Tq;
-                A3 += plam * pp * S;
-            }
+                A2 += pl * Tq;
+                A3 += pl * S;
+            });
             vjp_pairs<R>(T, A1, A2, A3, C, tw.q4, fix, fiy, fiz, sjx, sjy, sjz);
         }
         if (tw.row_end) {
@@ -904,19 +823,22 @@ __device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
 }
 
 // G3 part of the JVP in grid form; lane 0 writes v[s]
-template <typename R>
-__device__ void acsf_g3_jvp_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, int i, const R *ux,
-                                 const R *uy, const R *uz, R *v) {
-    const int lane = threadIdx.x & 31;
+template <typename R, int GM, typename CELLS>
+__device__ __forceinline__ void g3_jvp_walk(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, int i, const R *ux,
+                                            const R *uy, const R *uz, R *v) {
+    const int lane = threadIdx.x & 31, ng = M.ng3eta[ei];
+    constexpr int GQ = CELLS::NQ;
     const CutK<R> ck = cut_k<R>(M, ei);
-    const R rc = ck.rc;
-    const GridConst<R> g = grid_const<R>(M, ei);
+    const CELLS g(M, ei);
+    R eta[GM];
+#pragma unroll
+    for (int m = 0; m < GM; ++m) eta[m] = m < ng ? g3_eta<R>(M, ei, m) : R(0);
     const R uix = ux[i], uiy = uy[i], uiz = uz[i];
-    R acc[kGM][kGQ];
+    R acc[GM][GQ];
 #pragma unroll
-    for (int m = 0; m < kGM; ++m)
+    for (int m = 0; m < GM; ++m)
 #pragma unroll
-        for (int q = 0; q < kGQ; ++q) acc[m][q] = R(0);
+        for (int q = 0; q < GQ; ++q) acc[m][q] = R(0);
     RowWalk tw;
     tw.init(cnt, lane);
     while (tw.valid) {
@@ -932,34 +854,57 @@ __device__ void acsf_g3_jvp_fast(const NNDev &M, const WarpCache<R> &C, int ei, 
             const R d3 = T.a[4] * T.c[4] * T.dfcjk / T.rjk;
             const R X1 = b1 * q1 + b2 * q2 + T.pfc * T.rinv0 * q3, X2 = T.pfc * (q1 + q2 - q3),
                     X3 = d1 * q1 + d2 * q2 - d3 * q3;
-            R E[kGM];
-            grid_pexp<R>(g, T, E);
-            Ladder<R> L;
-            ladder_make<R>(g, T.cost0, L);
+            R E[GM];
+            grid_pexp<R, GM>(eta, ng, T, E);
+            g.each(T.cost0, [&](int q, R pp, R pl) {
+                const R t1 = g.zl[q] * X1, t2 = R(2) * X2;
 #pragma unroll
-            for (int q = 0; q < kGQ; ++q) {
-                if (q >= g.nq) break;
-                const int l = g.lidx[q];
-                if (!L.pos[l]) continue;
-                const R plam = L.pw[l][0];
-                const R base = ladder_pow<R>(L, l, g.zm1[q]) * g.pn[q];
-                const R t1 = g.zl[q] * X1 + plam * X3, t2 = R(2) * plam * X2;
-#pragma unroll
-                for (int m = 0; m < kGM; ++m) acc[m][q] -= base * E[m] * (t1 - g.eta[m] * t2);
-            }
+                for (int m = 0; m < GM; ++m) acc[m][q] -= E[m] * (pp * t1 + pl * (X3 - eta[m] * t2));
+            });
         }
         tw.next();
     }
 #pragma unroll
-    for (int m = 0; m < kGM; ++m)
+    for (int m = 0; m < GM; ++m)
 #pragma unroll
-        for (int q = 0; q < kGQ; ++q) {
-            if (m >= g.ng || q >= g.nq) continue;
+        for (int q = 0; q < GQ; ++q) {
+            const int s = m < ng ? CELLS::sf(M, ei, m, q) : -1;
+            if (s < 0) continue;
             const R val = warp_sum(acc[m][q]);
-            const int s = M.sf_of[ei][m][q];
-            if (lane == 0 && s >= 0) v[s] = val;
+            if (lane == 0) v[s] = val * CELLS::pn(M, ei, q);
         }
     __syncwarp();
+}
+
+// calls f(GM, cells) of the form of element ei's walk
+template <typename R, typename F> __device__ __forceinline__ void g3_form(const NNDev &M, int ei, F f) {
+    const int nz = M.gz[ei];
+    if (nz == 0) f(std::integral_constant<int, kGM>(), (AnyCells<R> *)nullptr);
+    else if (nz <= 3 && M.ng3eta[ei] <= 3) f(std::integral_constant<int, 3>(), (ProductCells<R, 3> *)nullptr);
+    else f(std::integral_constant<int, 4>(), (ProductCells<R, 4> *)nullptr);
+}
+
+template <typename R> __device__ void acsf_g3_forward_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt,
+                                                           R *G) {
+    g3_form<R>(M, ei, [&](auto gm, auto *cells) {
+        g3_forward_walk<R, decltype(gm)::value, std::remove_reference_t<decltype(*cells)>>(M, C, ei, cnt, G);
+    });
+}
+
+template <typename R>
+__device__ void acsf_g3_vjp_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, const R *c, R &fix, R &fiy,
+                                 R &fiz) {
+    g3_form<R>(M, ei, [&](auto gm, auto *cells) {
+        g3_vjp_walk<R, decltype(gm)::value, std::remove_reference_t<decltype(*cells)>>(M, C, ei, cnt, c, fix, fiy, fiz);
+    });
+}
+
+template <typename R>
+__device__ void acsf_g3_jvp_fast(const NNDev &M, const WarpCache<R> &C, int ei, int cnt, int i, const R *ux,
+                                 const R *uy, const R *uz, R *v) {
+    g3_form<R>(M, ei, [&](auto gm, auto *cells) {
+        g3_jvp_walk<R, decltype(gm)::value, std::remove_reference_t<decltype(*cells)>>(M, C, ei, cnt, i, ux, uy, uz, v);
+    });
 }
 
 }  // namespace mdt

@@ -1734,10 +1734,26 @@ int32_t mdt_nn_set_model(mdt_ctx *c, const mdt_nn_model *m, int32_t ntypes, cons
             M.nlz[e] = nq;
             M.g3pair[e][0] = pe1;
             M.g3pair[e][1] = pe2;
-            const int zm1[3] = {0, 3, 15};
-            M.g3std[e] = nq == 6 && M.ng3eta[e] == 3;
-            for (int q = 0; q < nq && M.g3std[e]; ++q)
-                M.g3std[e] = M.lz_zm1[e][q] == zm1[q >> 1] && M.lz_lam[e][q] == (q & 1 ? 1.f : -1.f);
+            // as a product of lambdas and zetas, both ascending
+            std::vector<float> lam(M.lz_lam[e], M.lz_lam[e] + nq);
+            std::vector<int> ex(M.lz_zm1[e], M.lz_zm1[e] + nq);
+            std::sort(lam.begin(), lam.end());
+            lam.erase(std::unique(lam.begin(), lam.end()), lam.end());
+            std::sort(ex.begin(), ex.end());
+            ex.erase(std::unique(ex.begin(), ex.end()), ex.end());
+            M.gz[e] = lam.size() <= 2 && ex.size() <= 4 ? (int)ex.size() : 0;
+            for (int l = 0; l < 2; ++l) M.glam[e][l] = l < (int)lam.size() ? lam[l] : 0.f;
+            for (int z = 0; z < 4; ++z) {
+                M.gex[e][z] = z < (int)ex.size() ? ex[z] : 0;
+                M.gpn[e][z] = std::ldexp(1.f, -M.gex[e][z]);
+            }
+            for (int g = 0; g < 4; ++g)
+                for (int q = 0; q < 8; ++q) M.gsf[e][g][q] = -1;
+            for (int q = 0; M.gz[e] && q < nq; ++q) {
+                const int z = (int)(std::find(ex.begin(), ex.end(), M.lz_zm1[e][q]) - ex.begin());
+                const int l = (int)(std::find(lam.begin(), lam.end(), M.lz_lam[e][q]) - lam.begin());
+                for (int g = 0; g < 4; ++g) M.gsf[e][g][2 * z + l] = M.sf_of[e][g][q];
+            }
         }
     }
     std::vector<uint8_t> act((size_t)ne * kMaxLayers * kMaxNodes, 'l');

@@ -66,7 +66,11 @@ struct NNDev {
     int lz_zm1[kMaxElem][8];             // zeta - 1 (integer)
     int8_t sf_of[kMaxElem][4][8];        // symmetry-function index of cell (m, q), -1 if none
     int g3pair[kMaxElem][2];             // the shared neighbour-element pair
-    int g3std[kMaxElem];                 // 1: three etas, cells (zeta 1, 4, 16) x (lambda -1, +1) in this order
+    // the same cells as a product of two lambdas and gz zetas (exponents gex = zeta - 1, norms gpn), function of
+    // cell 2 z + l at eta slot m in gsf, -1 if none; gz = 0: no such product
+    int gz[kMaxElem], gex[kMaxElem][4];
+    float glam[kMaxElem][2], gpn[kMaxElem][4];
+    int8_t gsf[kMaxElem][4][8];
 };
 
 // ---------------------------------------------------------------------------
