@@ -1,5 +1,5 @@
 // mdt_acsf.cuh -- atom-centred symmetry functions as CTA/warp device functions, shared by
-// the HDNNP/surrogate force kernels (mdt_nn.cu) and the training kernels (mdt_train.cu).
+// the HDNNP/surrogate force kernels (mdt_nn_kernels.cuh) and the training kernels (mdt_train.cu).
 //
 // One warp owns one central atom i.  Its neighbour cache (per neighbour q: the vector
 // d_q = x_q - x_i, r_q, fc(r_q), dfc/dr(r_q) and exp(-eta r_q^2) for every distinct G3 eta

@@ -40,6 +40,10 @@ int max_resident_ctas(int max_atoms, int max_beads, int precision);
 cudaError_t launch_nn(const LaunchCfg &c, const Batch &B, const NNDev &M, const EmtConst &E, const NNScratch &X,
                       const PropParams &P, int ngeta, int nsteps, int mode, int precision, bool surrogate);
 int nn_resident_ctas(const NNDev &M, int max_atoms, int max_beads, int ngeta, int precision, bool surrogate);
+// the same in FP64 (called by these two)
+cudaError_t launch_nn_fp64(const LaunchCfg &c, const Batch &B, const NNDev &M, const EmtConst &E, const NNScratch &X,
+                           const PropParams &P, int ngeta, int nsteps, int mode, bool surrogate);
+int nn_resident_fp64(size_t smem, bool surrogate);
 
 // FP32 fast path (mdt_nnf.cu)
 int nnf_zm_supported(int zm);

@@ -1,6 +1,6 @@
 // mdt_nnf.cu -- FP32 fast path of the HDNNP / EMT-surrogate force evaluation and MD step.
 //
-// Same results as the generic kernels of mdt_nn.cu (RuNNer's short-range prediction,
+// Same results as the generic kernels of mdt_nn_kernels.cuh (RuNNer's short-range prediction,
 // src/pes_nene_mod.f90:7145-7368, with the symmetry functions of
 // RuNNer_src/atomsymfunction2.f90 and atomsymfunction3Andi.f90) for the models that
 // FastNN::ok admits, organised for throughput:
