@@ -1741,7 +1741,8 @@ int32_t mdt_nn_set_model(mdt_ctx *c, const mdt_nn_model *m, int32_t ntypes, cons
             lam.erase(std::unique(lam.begin(), lam.end()), lam.end());
             std::sort(ex.begin(), ex.end());
             ex.erase(std::unique(ex.begin(), ex.end()), ex.end());
-            M.gz[e] = lam.size() <= 2 && ex.size() <= 4 ? (int)ex.size() : 0;
+            if (lam.size() > 2) M.g3fast[e] = 0;  // (the grid forms hold the powers of two)
+            M.gz[e] = M.g3fast[e] && ex.size() <= 4 ? (int)ex.size() : 0;
             for (int l = 0; l < 2; ++l) M.glam[e][l] = l < (int)lam.size() ? lam[l] : 0.f;
             for (int z = 0; z < 4; ++z) {
                 M.gex[e][z] = z < (int)ex.size() ? ex[z] : 0;

@@ -1,5 +1,6 @@
 """The three forms of the G3 walks by the structure of a function set: products of two lambdas and three or
-four zetas, up to four etas, with functions missing and with one lambda; sets that are no such product.
+four zetas, up to four etas, with functions missing and with one lambda; sets that are no such product, and one of three
+lambdas, which takes the walk over a list.
 FP64 energies and forces against the oracle (parity bar 1e-10, scaled by the largest force above
 1 eV/A), and the training gradient, which takes the tangent walk, against central differences of the
 oracle's loss (its second-order error and rounding: 1e-5)."""
@@ -27,6 +28,7 @@ SETS = {
     "missing": ((0.001, 0.01, 0.1), ((1.0, (1.0,)), (4.0, BOTH), (16.0, (-1.0,)))),
     "one lambda": ((0.01, 0.1), ((1.0, (1.0,)), (2.0, (1.0,)), (8.0, (1.0,)))),
     "other lambda": ((0.01, 0.1), ((1.0, (0.5, 1.0)), (4.0, (0.5, 1.0)))),
+    "3 lambdas": ((0.01, 0.1), ((1.0, (-1.0, 0.5, 1.0)), (4.0, (-1.0, 0.5, 1.0)))),
     "5 zetas": ((0.01, 0.1), ((1.0, (1.0,)), (2.0, BOTH), (3.0, (-1.0,)), (4.0, BOTH), (6.0, (1.0,)))),
     "7 zetas": ((0.001, 0.01, 0.1), tuple((float(z), (1.0,)) for z in (1, 2, 3, 5, 8, 16, 31))),
 }
