@@ -1036,9 +1036,6 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
     constexpr int KT = KA + KB, bs = kRS;
     const int tid = threadIdx.x;
     const SmemR S = carve_r<KT, NH, TC>(smem_raw);
-    SmemEmt<double> SE = carve_smem<double>(S.emt, emt_layout_one(B.max_atoms, B.max_beads));
-    SE.red = S.red;
-    SE.cjk = S.red;  // single-bead trajectories only: the ring-polymer table is never read
     TcCtx C{0u, S.tcbar, X.tcerr};
     uint32_t phase = 0;  // parity of this thread's tile mbarrier
     if constexpr (TC) {
@@ -1298,6 +1295,9 @@ __global__ void __launch_bounds__(kRBlockMax, 1)
                 bool anyfb = false;
                 for (int s = 0; s < pd.y; ++s) anyfb |= stat[s] && flag[s];
                 if (anyfb) {  // uniform over the CTA
+                    SmemEmt<double> SE = carve_smem<double>(S.emt, emt_layout_one(B.max_atoms, 1));
+                    SE.red = S.red;
+                    SE.cjk = S.red;  // single-bead trajectories only: the ring-polymer table is never read
                     __syncthreads();
                     for (int s = 0; s < pd.y; ++s) {
                         if (!stat[s] || !flag[s]) continue;
