@@ -8,7 +8,8 @@ namespace mdt {
 
 
 // ---------------------------------------------------------------------------
-// Propagators (src/md_algo.f90).  Thread per atom, all beads of the atom.
+// Propagators (src/md_algo.f90).  Work items (dimension, atom), all beads of the atom, over the
+// threads of the trajectory's CTA or of the cluster that shares it.
 // ---------------------------------------------------------------------------
 // A trajectory as its team of CTAs sees it: one CTA, or the CTAs of a cluster that share a ring
 // polymer (their work items interleave, their state meets in global memory, team_sync orders it).
