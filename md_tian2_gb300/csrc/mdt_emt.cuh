@@ -113,7 +113,8 @@ struct TeamWork {
 // four waves.  With one CTA per trajectory a batch waits for its longest ring polymer (32 beads, one after the
 // other): 96 FP64 trajectories 31.3 ms with one, 13.1 with 8; 1024 with FP32 forces 26.3 ms with one, 22.4
 // with 2, 33 with 4 (fewer beads at a time fill fewer warps, and every CTA repeats the tables and sums of a
-// step).  1199 single beads beside one 2-bead ring polymer: 1.9 ms with one, 2.6 with 2 (half the CTAs wait).
+// step).  1199 single beads beside one 2-bead ring polymer, five FP64 steps: 1.2 ms with one, 2.5 with 2 (half the
+// CTAs wait).
 inline int team_log2(const TeamWork &w, int64_t ntraj, int max_beads, int64_t slots) {
     int k = 0;
     while (k < 3 && (2 << k) <= max_beads && ntraj * (2 << k) <= 4 * slots &&
